@@ -53,8 +53,9 @@ class Decoder:
         self.logits = torch.zeros(vocab, dtype=torch.float32, device=self.dev)
         self.pos = torch.zeros(1, dtype=torch.int32, device=self.dev)
         self.token = torch.zeros(1, dtype=torch.int64, device=self.dev)
-        self.host_token = torch.zeros(1, dtype=torch.int64).pin_memory()   # generate() feeds every step from the host, as the reference does
-        self.graph_layers = self.graph_head = None
+        self.host_token = torch.zeros(1, dtype=torch.int64).pin_memory()   # a caller's callback sees a token before the host feeds it to the next step
+        self.picks = [(torch.zeros(1, dtype=torch.int64).pin_memory(), torch.cuda.Event()) for _ in range(2)]   # read-outs in flight, with what to wait for
+        self.graph_layers = self.graph_step = None
         self.fed = 0            # tokens feed() has taken since the last reset
 
     # ---- what a model supplies ----
@@ -86,7 +87,9 @@ class Decoder:
 
     # ---- steps ----
     def capture(self) -> None:
-        """Runs one throw-away step (kernel attributes are set on first launch), then captures the two graphs."""
+        """Runs one throw-away step (kernel attributes are set on first launch), then captures two graphs: the layers alone, for
+        prompt tokens whose logits nobody asks for, and a whole step.  The step is one graph so that the head's product starts
+        reading its weights while the last layer's product ends, as the layers' do among each other."""
         torch = self.torch
         self.sync_ranks()
         with torch.cuda.stream(self.stream):
@@ -94,13 +97,14 @@ class Decoder:
             self._enqueue_layers()
             self._enqueue_head()
             self.stream.synchronize()
-            self.graph_layers, self.graph_head = torch.cuda.CUDAGraph(), torch.cuda.CUDAGraph()
+            self.graph_layers, self.graph_step = torch.cuda.CUDAGraph(), torch.cuda.CUDAGraph()
             # with collectives in the graph, other threads of the process (the collective library's watchdog) may call
             # the runtime during the capture: only this thread's calls belong to it
             mode = dict(capture_error_mode="thread_local") if self.world > 1 else {}
             with torch.cuda.graph(self.graph_layers, stream=self.stream, **mode):
                 self._enqueue_layers()
-            with torch.cuda.graph(self.graph_head, stream=self.stream, **mode):
+            with torch.cuda.graph(self.graph_step, stream=self.stream, **mode):
+                self._enqueue_layers()
                 self._enqueue_head()
             self.stream.synchronize()
         self.reset()
@@ -118,9 +122,7 @@ class Decoder:
         """Consumes the token in self.token at position self.pos; with want_token the pick replaces self.token."""
         with self.torch.cuda.stream(self.stream):
             if self.graph_layers is not None:
-                self.graph_layers.replay()
-                if want_token:
-                    self.graph_head.replay()
+                (self.graph_step if want_token else self.graph_layers).replay()
             else:
                 self._enqueue_layers()
                 if want_token:
@@ -196,6 +198,10 @@ class Decoder:
         token from a host generator seeded with `seed` (the generator stays on the host, as the reference's does).  The
         prompt goes through prefill() in blocks (in the prompt's activation mode) on one GPU and on a column-cut sharded
         decoder with an NCCL group, token by token otherwise; batched_prefill overrides the choice.
+        With a callback, and on several GPUs, the host has each token before the next step begins and feeds it back from its
+        side, as the reference's loop does.  Otherwise nothing a step needs passes through the host (its token is where the
+        pick or the draw left it), so a step is launched before the token of the one before is read: the round trip to the
+        host runs beside the next step (B200, four layers of width 1024: 139 us a token, 160 with it between the steps).
         Raises when the context would overflow."""
         torch = self.torch
         if not prompt or len(prompt) + max_new > self.max_positions:
@@ -206,17 +212,32 @@ class Decoder:
         rng = np.random.default_rng(seed) if temperature > 0.0 else None
         with torch.cuda.stream(self.stream):
             self.feed_prompt(prompt, batched_prefill)
-            for n in range(max_new):
+            ahead = on_token is None and self.world == 1
+
+            def draw_and_send(n: int) -> None:
                 if rng is not None:               # the step left the greedy pick in self.token: draw instead
                     self._sample(temperature, top_k, top_p, float(rng.random()))
-                tok = int(self.token.item())      # device -> host read of the step's result
+                host, sent = self.picks[n % 2]
+                host.copy_(self.token, non_blocking=True)
+                sent.record(self.stream)
+
+            if max_new > 0:
+                draw_and_send(0)
+            for n in range(max_new):
+                if ahead and n + 1 < max_new:
+                    self.step(want_token=True)
+                    draw_and_send(n + 1)
+                host, sent = self.picks[n % 2]
+                sent.synchronize()                # device -> host read of the step's result
+                tok = int(host[0])
                 out.append(tok)
                 if on_token:
                     on_token(tok)
-                if n + 1 < max_new:
+                if not ahead and n + 1 < max_new:
                     self.host_token[0] = tok      # host -> device: the next step's input comes from the caller's side
                     self.token.copy_(self.host_token, non_blocking=True)
                     self.step(want_token=True)
+                    draw_and_send(n + 1)
         self.be.dev_check(self.stream.cuda_stream)
         return out
 
@@ -226,4 +247,4 @@ class Decoder:
 
     def close(self) -> None:
         self.stream.synchronize()
-        self.graph_layers = self.graph_head = None
+        self.graph_layers = self.graph_step = None

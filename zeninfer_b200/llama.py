@@ -8,7 +8,7 @@ through the quantised product kernels (zen_cuda_dev_gemv); the operators between
 points of include/zen_cuda.h.  Nothing here computes on the host: Python only orders launches and builds the RoPE
 cos/sin tables (the reference's table contract, rope_table :264-276).
 
-A step is captured once into two CUDA graphs (layers; lm_head + pick), because the position and the token are read
+A step is captured once into a CUDA graph (and the layers alone into another, for prompt tokens), because the position and the token are read
 from device memory.  The prompt goes through prefill() in blocks (tensor-core products) or token by token.
 
 Several GPUs (one process per GPU, `rank` of `world`): every matrix but the embedding table is cut by output rows, a
@@ -416,7 +416,7 @@ class LlamaDecoder(Decoder):
 
     def close(self) -> None:
         self.stream.synchronize()
-        self.graph_layers = self.graph_head = None     # captured collectives hold on to the communicator: release them before the group goes
+        self.graph_layers = self.graph_step = None     # captured collectives hold on to the communicator: release them before the group goes
         if self.peer is not None:
             self.peer.close()                          # collective: every rank closes its decoder
             self.peer = None
