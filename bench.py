@@ -921,8 +921,8 @@ def run_decode(args, brief: bool = False) -> dict | None:
     """Config: 32 layers, d 4096, 32 query / 8 KV heads of 128, SwiGLU 14336, vocab 128256, eps 1e-5, theta 500000,
     weights N(0, 0.02) seed 6, a prompt of 512 uniform-random ids, then greedy decode steps.  The prompt is consumed as
     blocks of tensor-core products and timed separately (prefill_ms); sharded, the block's partial products are summed by
-    two NCCL all-reduces per layer.  A step is one decoded token: the launches of 32 layers, the lm_head and the pick, replayed from two CUDA
-    graphs (RMSNorm and the residual adds are folded into the projection launches)."""
+    two NCCL all-reduces per layer.  A step is one decoded token: the launches of 32 layers, the lm_head and the pick, replayed from a CUDA
+    graph (RMSNorm and the residual adds are folded into the projection launches)."""
     import torch
     from zeninfer_b200 import Backend
     from zeninfer_b200.backend import ACT_INT8
@@ -1058,7 +1058,7 @@ def run_decode(args, brief: bool = False) -> dict | None:
 
     fn, fs, fr, fp = ("n" in dec.fuse), ("s" in dec.fuse), ("r" in dec.fuse), ("p" in dec.fuse)
     per_layer = 5 + (0 if (fn and fr) else 2) + (0 if (fs or fp) else 1)   # q|k|v, attention block, o, gate|up, down + norm / residual / SwiGLU launches
-    launches_per_step = 1 + (0 if fn else 1) + per_layer * cfg.layers + 1 + 1 + 2   # embed, layers, advance, lm_head, pick (2): per rank
+    launches_per_step = 1 + (0 if fn else 1) + per_layer * cfg.layers + 1 + 1 + 1   # embed, layers, advance, lm_head, pick: per rank
     gathers = ((2 if dec.col_cut else 4) * cfg.layers + 1) if world > 1 else 0
     line = ({
         "metric": "decode_tokens_per_s", "value": tok_s, "unit": "tokens/s", "n_gpus": world, "steps": steps, "warmup": warm, "ms_per_step": ms / steps,
@@ -1066,7 +1066,7 @@ def run_decode(args, brief: bool = False) -> dict | None:
         "config": {"workload": "greedy decode, random-init Llama-3-8B shape in Q8_0 (config 4): 32 layers, d 4096, 32/8 heads of 128, ffn 14336, "
                                f"vocab 128256; prompt of {prompt_len} random ids (untimed here, see prefill_ms), then {warm} + {steps} decode steps",
                    "activations": "int8 (bit-exact reference codes)", "l2": "inputs larger than L2: 8.5 GB of weights stream per token",
-                   "launch": f"two CUDA graphs per token, {launches_per_step} kernel launches (folded into the projections: '{dec.fuse}')", "weights": "torch.randn on the device, seed 6, N(0, 0.02)",
+                   "launch": f"one CUDA graph per token, {launches_per_step} kernel launches (folded into the projections: '{dec.fuse}')", "weights": "torch.randn on the device, seed 6, N(0, 0.02)",
                    "sharding": ("none (one GPU)" if world == 1 else f"output rows of every matrix over {world} GPUs, rank-local heads and KV cache, "
                                 f"{gathers} exchanges per token inside the step graphs "
                                 + ("(o and down cut by columns, their partial products all-reduced into the residual stream; logits gathered), "
