@@ -94,6 +94,22 @@ def test_gemv_fp32_mode_vs_oracle(be, zo, rows, cols):
     be.set_q8_act_mode(ACT_INT8)
 
 
+# Rows that share a stage of the ring (up to 2048 columns, a multiple of 256): one and several groups of a CTA's slice, an even and
+# an odd number of them, groups of fewer rows than a stage holds, 24 to 64 blocks per row.
+@pytest.mark.parametrize("rows,cols", [(1, 256), (7, 1024), (149, 1024), (1184, 1024), (1185, 768), (4443, 1280), (9473, 1024), (2500, 1792), (5000, 2048), (4737, 512)])
+@pytest.mark.parametrize("mode,int8", [(ACT_INT8, True), (ACT_FP32, False)])
+def test_gemv_of_short_rows(be, zo, mode, int8, rows, cols):
+    w = seeded_weights(Q8_0, rows, cols, 50 + rows)
+    x = seeded_acts(1, cols, 60 + cols)[0]
+    be.set_q8_act_mode(mode)
+    y = be.gemv("Q8_0", w, x, rows, cols)
+    be.release_weights(w)
+    be.set_q8_act_mode(ACT_INT8)
+    ref = ref_int8_f64(w, *zo.quantise_acts(x[None]), rows, cols) if int8 else ref_fp32_f64(Q8_0, w, x, rows, cols)
+    rel = assert_parity(y, ref[0], what=f"short rows {rows}x{cols}")
+    assert rel < (1e-5 if int8 else 1e-4)       # 32-bit sums of at most 64 scaled blocks; two int8 digits per activation
+
+
 def test_gemv_against_reference_golden(be, golden):
     be.set_q8_act_mode(ACT_INT8)
     w = np.ascontiguousarray(golden["i8_gemv_w"])

@@ -158,11 +158,11 @@ struct RowGroup {
     uint32_t task, row0, nrows;  // nrows == 0: no group (the odd tail of a pair)
 };
 
-// Walks a row slice in groups of at most kTeamWarps rows that never straddle two tasks.
+// Walks a row slice in groups of at most `most` rows that never straddle two tasks.
 struct GroupWalk {
-    uint32_t r, r_end, ti;
+    uint32_t r, r_end, ti, most;
     bool paired;   // kGemvFlagPairSwiglu: every group goes out twice in a row, for task 0 and then for task 1
-    __device__ GroupWalk(uint32_t first, uint32_t last, bool paired_ = false) : r(first), r_end(last), ti(0), paired(paired_) {}
+    __device__ GroupWalk(uint32_t first, uint32_t last, bool paired_ = false, uint32_t most_ = kTeamWarps) : r(first), r_end(last), ti(0), most(most_), paired(paired_) {}
     __device__ bool done() const { return r >= r_end; }
     __device__ RowGroup next(const GemvParams& p) {
         RowGroup g{0, 0, 0};
@@ -170,7 +170,7 @@ struct GroupWalk {
         if (paired) {
             g.task = ti;
             g.row0 = r;
-            g.nrows = min(static_cast<uint32_t>(kTeamWarps), r_end - r);
+            g.nrows = min(most, r_end - r);
             if (ti) r += g.nrows;
             ti ^= 1u;
             return g;
@@ -178,7 +178,7 @@ struct GroupWalk {
         while (r >= p.task[ti].first_row + p.task[ti].rows) ++ti;
         g.task = ti;
         g.row0 = r - p.task[ti].first_row;
-        g.nrows = min(min(static_cast<uint32_t>(kTeamWarps), p.task[ti].rows - g.row0), r_end - r);
+        g.nrows = min(min(most, p.task[ti].rows - g.row0), r_end - r);
         r += g.nrows;
         return g;
     }
@@ -203,11 +203,28 @@ __device__ __forceinline__ int dot32(const uint4& wa, const uint4& wb, const uin
 #ifndef ZK_GEMV_MIN_CTAS
 #define ZK_GEMV_MIN_CTAS 1
 #endif
+// kPack: rows per warp and group.  A stage holds eight rows of 4096 columns; with rows of 2048 columns or fewer the ring would hold
+// only eight short ones per stage, and since a stage comes round once per copy latency (about 2 us), a launch took 0.65 us per eight
+// rows and CTA however short they were.  So up to four rows per warp go in one stage (batch 1, rows contiguous in both planes); the
+// slice is cut into groups of equal size, an even number of them where it takes more than one, for the two teams.
+// B200, us before -> now, int8 / two-digit activations: 32000 x 1024 19.2 -> 8.5 / 19.2 -> 10.0, 8192 x 1024 5.9 -> 3.7 / 5.9 -> 4.0,
+// 32000 x 2048 18.8 -> 13.8 / 19.1 -> 16.0.
+constexpr int kGemvPackRows = 4;
+constexpr uint32_t kGemvPackMaxK = kGemvSegBlocks / 2 * 32;      // two rows to the eight-row stage's row
+__host__ __device__ inline bool gemv_packs(uint32_t K, int batch) { return batch == 1 && K <= kGemvPackMaxK && K % 256 == 0; }
+__device__ __forceinline__ uint32_t gemv_group_rows(uint32_t slice, uint32_t nb, bool paired) {
+    const uint32_t most = kTeamWarps * min(kGemvSegBlocks / nb, static_cast<uint32_t>(kGemvPackRows));
+    uint32_t groups = max(1u, (slice + most - 1) / most);
+    if (!paired && (groups & 1) && slice > kTeamWarps) ++groups;
+    return min(most, ((slice + groups - 1) / groups + kTeamWarps - 1) / kTeamWarps * kTeamWarps);
+}
+
 // kFuse: the launch may carry kGemvFlag* work (fused RMSNorm / SwiGLU input, accumulating store).  It is a template
 // parameter because even untaken flag tests in the prologue and the store cost the plain 4096 x 4096 product 5 %.
-template <int kBatch, int kDigits, bool kFuse = false>
+template <int kBatch, int kDigits, bool kFuse = false, int kPack = 1>
 __global__ void __launch_bounds__(kGemvThreads, (kBatch * kDigits == 1 ? ZK_GEMV_MIN_CTAS : 1))
     gemv_q8_0_kernel(const __grid_constant__ GemvParams p) {
+    static_assert(kPack == 1 || kBatch == 1, "several rows per warp only for one token");
     const uint32_t flags = kFuse ? p.flags : 0u;
     extern __shared__ __align__(128) uint8_t smem[];
     const uint32_t nb = p.K >> 5, nbp = (nb + 7) & ~7u, nseg = (nb + kGemvSegBlocks - 1) / kGemvSegBlocks;
@@ -233,7 +250,8 @@ __global__ void __launch_bounds__(kGemvThreads, (kBatch * kDigits == 1 ? ZK_GEMV
     cta_row_slice(p.total_rows, blockIdx.x, gridDim.x, r_first, r_last);
     const uint32_t n_mine = r_last - r_first;
     // A group of whole single-segment rows is contiguous in both planes: one copy each.
-    const bool contiguous = nseg == 1 && nb == nbp;
+    const bool contiguous = kPack > 1 || (nseg == 1 && nb == nbp);
+    const uint32_t group_rows = kPack > 1 ? gemv_group_rows(n_mine, nb, kFuse && (p.flags & kGemvFlagPairSwiglu)) : static_cast<uint32_t>(kTeamWarps);
     const uint32_t cstride = contiguous ? nb * 32 : kGemvSegBlocks * 32;  // stage row pitch of the codes, bytes
     const uint32_t sstride = contiguous ? nb : kGemvSegBlocks;             // stage row pitch of the scales, halves
 
@@ -256,7 +274,7 @@ __global__ void __launch_bounds__(kGemvThreads, (kBatch * kDigits == 1 ? ZK_GEMV
         bool announce = p.gather.world != 0 && blockIdx.x == 0;
         uint32_t unit = 0;
         bool ok = true;
-        GroupWalk walk(r_first, r_last, kFuse && (p.flags & kGemvFlagPairSwiglu));
+        GroupWalk walk(r_first, r_last, kFuse && (p.flags & kGemvFlagPairSwiglu), group_rows);
         while (!walk.done() && ok) {
             RowGroup pair[kTeams];
 #pragma unroll
@@ -275,7 +293,7 @@ __global__ void __launch_bounds__(kGemvThreads, (kBatch * kDigits == 1 ? ZK_GEMV
                         if (lane == 0) {
                             // Pull what the ring cannot hold yet into L2, so later refills do not pay DRAM latency.
                             uint32_t budget = kL2PrefetchCap;
-                            GroupWalk pre(r_first + min(static_cast<uint32_t>(kGemvStages * kTeamWarps) / nseg, n_mine), r_last);
+                            GroupWalk pre(r_first + min(kGemvStages * group_rows / nseg, n_mine), r_last, false, group_rows);
                             while (!pre.done() && budget) {
                                 const RowGroup g = pre.next(p);
                                 const GemvTask& t = p.task[g.task];
@@ -511,7 +529,7 @@ __global__ void __launch_bounds__(kGemvThreads, (kBatch * kDigits == 1 ? ZK_GEMV
     const bool pair_swiglu = kFuse && (flags & kGemvFlagPairSwiglu);
     float* pair_buf = reinterpret_cast<float*>(norm_part);   // [2 parities][batch][row of the group]: the prologue is done with norm_part
     uint32_t pair_parity = 0;
-    GroupWalk walk(r_first, r_last, pair_swiglu);
+    GroupWalk walk(r_first, r_last, pair_swiglu, group_rows);
     while (!walk.done() && ok) {
         RowGroup pair[kTeams];
 #pragma unroll
@@ -519,16 +537,18 @@ __global__ void __launch_bounds__(kGemvThreads, (kBatch * kDigits == 1 ? ZK_GEMV
         RowGroup g = pair[0];
         if constexpr (kTeams > 1) { if (team == 1) g = pair[kTeams - 1]; }  // no runtime-indexed local array
         const GemvTask& t = p.task[g.task];
-        const uint32_t row = g.row0 + twarp;
-        const bool valid = static_cast<uint32_t>(twarp) < g.nrows;
-        float acc[kBatch];
+        // a sum per token, or (kPack > 1) per row: the warp's rows of the group are kTeamWarps apart
+        constexpr int kSums = kBatch * kPack, kRowBlocks = kPack > 1 ? kGemvPackMaxK / 1024 : kLaneBlocks;      // blocks of a row per lane
+        auto valid_row = [&](int i) { return static_cast<uint32_t>(twarp + kTeamWarps * i) < g.nrows; };
+        auto y_at = [&](int i) { return kPack > 1 ? t.y + g.row0 + twarp + kTeamWarps * i : t.y + static_cast<size_t>(i) * t.rows + g.row0 + twarp; };
+        auto valid_sum = [&](int i) { return valid_row(kPack > 1 ? i : 0); };
+        float acc[kSums];
 #pragma unroll
-        for (int b = 0; b < kBatch; ++b) acc[b] = 0.0f;
+        for (int b = 0; b < kSums; ++b) acc[b] = 0.0f;
         // y += W x: fetch the old outputs now, so that their latency hides behind the row's dot products
-        float y_old[kBatch];
+        float y_old[kSums];
 #pragma unroll
-        for (int b = 0; b < kBatch; ++b)
-            y_old[b] = (kFuse && (flags & kGemvFlagAccumulate) && valid && lane == 0 && t.y) ? __ldcg(t.y + static_cast<size_t>(b) * t.rows + row) : 0.0f;
+        for (int b = 0; b < kSums; ++b) y_old[b] = (kFuse && (flags & kGemvFlagAccumulate) && valid_sum(b) && lane == 0 && t.y) ? __ldcg(y_at(b)) : 0.0f;
 
         for (uint32_t s = 0; s < nseg; ++s) {
             const uint32_t unit = pair_base + s * kTeams + team;
@@ -541,13 +561,16 @@ __global__ void __launch_bounds__(kGemvThreads, (kBatch * kDigits == 1 ? ZK_GEMV
 #ifdef ZK_TRACE
             if (team == 0 && unit < 4) ZK_STAMP(5 + 3 * (unit >> 1));
 #endif
-            if (valid) {
+#pragma unroll
+            for (int pr = 0; pr < kPack; ++pr) {
+                if (!valid_row(pr)) break;
                 const uint8_t* st = ring + stage * kQ8StageBytes;
-                const uint4* wq = reinterpret_cast<const uint4*>(st + twarp * cstride);
-                const __half* ws = reinterpret_cast<const __half*>(st + kQ8StageCodeBytes) + twarp * sstride;
+                const uint4* wq = reinterpret_cast<const uint4*>(st + (twarp + kTeamWarps * pr) * cstride);
+                const __half* ws = reinterpret_cast<const __half*>(st + kQ8StageCodeBytes) + (twarp + kTeamWarps * pr) * sstride;
                 if (x_in_regs) {
 #pragma unroll
-                    for (int i = 0; i < kLaneBlocks; ++i) {
+                    for (int i = 0; i < kRowBlocks; ++i) {
+                        if (kPack > 1 && i * 32 >= static_cast<int>(nb)) break;
                         const uint32_t bl = i * 32 + lane;
                         // A lane whose block index is past the row holds zero codes; the bytes it reads are
                         // stale but inside the stage, and its term is dropped by selection (stale scale bits
@@ -556,11 +579,11 @@ __global__ void __launch_bounds__(kGemvThreads, (kBatch * kDigits == 1 ? ZK_GEMV
                         const float dw = __half2float(ws[bl]);
                         const int isum = dot32(wa, wb, xra[i], xrb[i]);
                         const float term = (dw * xrs[i]) * static_cast<float>(isum);
-                        acc[0] += bl < nb ? term : 0.0f;
+                        acc[pr] += bl < nb ? term : 0.0f;
                     }
                 } else {
 #pragma unroll
-                    for (int i = 0; i < kLaneBlocks; ++i) {
+                    for (int i = 0; i < kRowBlocks; ++i) {
                         const uint32_t bl = i * 32 + lane;           // block within the segment
                         const uint32_t b = s * kGemvSegBlocks + bl;  // block within the row
                         if (b < nb) {
@@ -573,7 +596,7 @@ __global__ void __launch_bounds__(kGemvThreads, (kBatch * kDigits == 1 ? ZK_GEMV
                                 int isum = dot32(wa, wb, xc[0], xc[32]);
                                 if (kDigits == 2) isum = isum * 256 + dot32(wa, wb, xc[kpad_blocks * 2], xc[kpad_blocks * 2 + 32]);
                                 const float dx = xscale[static_cast<size_t>(tk) * kpad_blocks + b];
-                                acc[tk] = fmaf(dw * dx, static_cast<float>(isum), acc[tk]);
+                                acc[tk + pr] = fmaf(dw * dx, static_cast<float>(isum), acc[tk + pr]);
                             }
                         }
                     }
@@ -588,28 +611,29 @@ __global__ void __launch_bounds__(kGemvThreads, (kBatch * kDigits == 1 ? ZK_GEMV
         if (kFuse && pair_swiglu) {
             // team 1 (up) hands its row sums to team 0 (gate) through shared memory; the barrier also agrees on failure,
             // so that no warp waits at it for one that gave up
-            float v[kBatch];
+            float v[kSums];
 #pragma unroll
-            for (int tk = 0; tk < kBatch; ++tk) {
-                v[tk] = acc[tk];
+            for (int i = 0; i < kSums; ++i) v[i] = acc[i];
 #pragma unroll
-                for (int o = 16; o > 0; o >>= 1) v[tk] += __shfl_xor_sync(0xffffffffu, v[tk], o);
+            for (int o = 16; o > 0; o >>= 1) {
+#pragma unroll
+                for (int i = 0; i < kSums; ++i) v[i] += __shfl_xor_sync(0xffffffffu, v[i], o);
             }
-            float* slot = pair_buf + pair_parity * (kBatch * kTeamWarps);
+            float* slot = pair_buf + pair_parity * (kSums * kTeamWarps);
             if (team == 1 && lane == 0) {
 #pragma unroll
-                for (int tk = 0; tk < kBatch; ++tk) slot[tk * kTeamWarps + twarp] = v[tk];
+                for (int i = 0; i < kSums; ++i) slot[i * kTeamWarps + twarp] = v[i];
             }
             uint32_t any_failed;
             asm volatile(
                 "{ .reg .pred p, q; setp.ne.u32 q, %2, 0; barrier.red.or.pred p, 2, %1, q; selp.u32 %0, 1, 0, p; }"
                 : "=r"(any_failed) : "r"(kGemvWarps * 32), "r"(static_cast<uint32_t>(!ok)) : "memory");
             if (any_failed) { ok = false; break; }
-            if (team == 0 && lane == 0 && valid && t.y) {
+            if (team == 0 && lane == 0 && t.y) {
 #pragma unroll
-                for (int tk = 0; tk < kBatch; ++tk) {
-                    const float z = v[tk];
-                    t.y[static_cast<size_t>(tk) * t.rows + row] = (z / (1.0f + expf(-z))) * slot[tk * kTeamWarps + twarp];
+                for (int i = 0; i < kSums; ++i) {
+                    const float z = v[i];
+                    if (valid_sum(i)) *y_at(i) = (z / (1.0f + expf(-z))) * slot[i * kTeamWarps + twarp];
                 }
             }
             pair_parity ^= 1u;
@@ -621,14 +645,20 @@ __global__ void __launch_bounds__(kGemvThreads, (kBatch * kDigits == 1 ? ZK_GEMV
         const uint32_t traced_unit = pair_base;
 #endif
         pair_base += kTeams * nseg;
-        if (valid) {
+        if (valid_row(0)) {
 #pragma unroll
-            for (int tk = 0; tk < kBatch; ++tk) {
-                float v = acc[tk];
+            for (int o = 16; o > 0; o >>= 1) {
 #pragma unroll
-                for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-                if (lane == 0 && t.y) t.y[static_cast<size_t>(tk) * t.rows + row] = kFuse ? y_old[tk] + v : v;   // y_old is zero unless accumulating
-                if (lane == 0 && p.gather.world) stash[static_cast<size_t>(tk) * n_mine + (t.first_row + row - r_first)] = v;
+                for (int i = 0; i < kSums; ++i) acc[i] += __shfl_xor_sync(0xffffffffu, acc[i], o);
+            }
+#pragma unroll
+            for (int i = 0; i < kSums; ++i) {
+                if (!valid_sum(i) || lane) continue;
+                if (t.y) *y_at(i) = kFuse ? y_old[i] + acc[i] : acc[i];   // y_old is zero unless accumulating
+                if (p.gather.world) {
+                    const uint32_t token = kPack > 1 ? 0 : i, row = g.row0 + twarp + (kPack > 1 ? kTeamWarps * i : 0);
+                    stash[static_cast<size_t>(token) * n_mine + (t.first_row + row - r_first)] = acc[i];
+                }
             }
         }
 #ifdef ZK_TRACE

@@ -453,9 +453,9 @@ unsigned long long* g_trace = nullptr;  // profiling builds: device buffer [laun
 size_t g_trace_launch = 0;
 #endif
 
-template <int kBatch, int kDigits, bool kFuse>
+template <int kBatch, int kDigits, bool kFuse, int kPack = 1>
 cudaError_t launch_gemv_q8_0(const zk::GemvParams& p, unsigned grid, size_t smem, cudaStream_t st, bool pdl) {
-    auto* fn = &zk::gemv_q8_0_kernel<kBatch, kDigits, kFuse>;
+    auto* fn = &zk::gemv_q8_0_kernel<kBatch, kDigits, kFuse, kPack>;
     static size_t configured = 0;  // per instantiation; one device per process, calls serialised by the backend mutex
     if (smem > configured) {       // raised outside any stream capture by the first (uncaptured) launch of a shape
         cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
@@ -480,6 +480,7 @@ cudaError_t launch_gemv_q8_0(const zk::GemvParams& p, unsigned grid, size_t smem
 
 template <int kDigits, bool kFuse>
 cudaError_t dispatch_batch_fuse(int batch, const zk::GemvParams& p, unsigned grid, size_t smem, cudaStream_t st, bool pdl) {
+    if (zk::gemv_packs(p.K, batch)) return launch_gemv_q8_0<1, kDigits, kFuse, zk::kGemvPackRows>(p, grid, smem, st, pdl);
     switch (batch) {
     case 1: return launch_gemv_q8_0<1, kDigits, kFuse>(p, grid, smem, st, pdl);
     case 2: return launch_gemv_q8_0<2, kDigits, kFuse>(p, grid, smem, st, pdl);
