@@ -242,3 +242,30 @@ def test_group_scale_kernel_equals_its_restatement(zo, tokens, rows, cols, int8)
     # equal up to the last bit of a step here and there: the restatement rounds a fused multiply-add through float64
     assert np.abs(got.astype(np.float64) - want).max() <= 2e-6 * np.abs(want).max()
     assert np.mean(got == want) > 0.9
+
+
+# A launch of many row tiles takes the narrowest of the four tile widths that holds its tokens: each width, full and one token into
+# the next.
+@pytest.mark.parametrize("tokens", [20, 32, 33, 64, 65, 96, 97])
+def test_group_scale_tiles_of_every_width(zo, tokens):
+    test_group_scale_kernel_equals_its_restatement(zo, tokens, 18944, 512, False)
+
+
+@pytest.mark.parametrize("tokens", [8, 60, 77, 128])
+def test_group_scale_tiles_split_between_two_ctas(tokens):
+    # 149 row tiles: most are split, so a result is the sum of two partial sums and may differ from the restatement's by their roundings
+    import torch
+    from helpers import group_product
+    from zeninfer_b200 import Backend
+    be, rows, cols = Backend(), 19072, 512
+    w, x = seeded_weights(Q8_0, rows, cols, 721), seeded_acts(tokens, cols, 722)
+    h = be.dev_upload("Q8_0", w, rows, cols)
+    ws_bytes = be.gemm_workspace_bytes(tokens, cols, ACT_FP32)
+    ws, y, d_x = torch.zeros(ws_bytes, dtype=torch.uint8, device="cuda"), torch.full((tokens, rows), float("nan"), device="cuda"), torch.from_numpy(x).cuda()
+    torch.cuda.synchronize()
+    be.dev_gemm_q8_0([h], [y.data_ptr()], d_x.data_ptr(), tokens, ws.data_ptr(), ws_bytes, act_mode=ACT_FP32)
+    be.dev_check()
+    got = y.cpu().numpy()
+    be.dev_free(h)
+    want = group_product(blocks.dequantize(Q8_0, w, rows, cols), x)
+    assert np.abs(got.astype(np.float64) - want).max() <= 2e-6 * np.abs(want).max()

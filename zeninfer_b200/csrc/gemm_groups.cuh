@@ -27,13 +27,21 @@
 // tensor (group_digits_q8_0_kernel, group_digits_kq_kernel) and kept beside the decode planes: 2 bytes per weight of extra
 // device memory.
 //
-// Shape: one persistent CTA per SM, 18 warps.  Warp 0: TMA producer, per 128-wide K tile four tiles (wh, wl, xh, xl; 128
-// rows x 128 B, K-major, 128-byte swizzle) into a 3-stage ring.  Warp 1: MMA issuer, tcgen05.mma kind::i8, M = 128 weight
-// rows, N = 128 tokens, K = 32; accumulator sets alternate between the two halves of TMEM.  Warps 2..17: epilogue, thread =
-// weight row = TMEM lane, 32 token columns per warp.
+// Shape: one persistent CTA per SM.  Warp 0: TMA producer, per 128-wide K tile four tiles (wh, wl: 128 rows x 128 B; xh, xl:
+// kN rows; K-major, 128-byte swizzle) into a ring of three to five stages.  Warp 1: MMA issuer, tcgen05.mma kind::i8, M = 128
+// weight rows, N = kN tokens, K = 32; accumulator sets alternate between the two halves of TMEM.  Then 4 kN / 32 epilogue warps,
+// thread = weight row = TMEM lane, 32 token columns per warp.
+//
+// What bounds the kernel are the operand bytes that pass through an SM's shared memory, 256 (128 + kN) per 128 columns of K and
+// tile; a tile of few tokens brings its 32 KB of weights and little else.  So the tile's width (32, 64, 96 or 128 tokens) is the one
+// with the fewest bytes through the busiest SM (gg_tile_columns); with tiles of 128 only, eight tokens cost what 128 do.
+// B200, with the two launches in front merged into one and overlapped: 128256 x 4096 times 8 tokens 271 -> 176 us, 11008 x 4096
+// times 77 40.3 -> 37.1, 14336 x 4096 times 512 116.8 -> 114.8.
 #pragma once
 #include <cuda.h>
 #include <cuda_fp16.h>
+
+#include <algorithm>
 
 #include "gemm_q8_0_i8.cuh"
 
@@ -41,29 +49,44 @@ namespace zk {
 
 constexpr int kGgGroup = 256;                       // weights per common scale
 constexpr int kGgKTilesPerGroup = kGgGroup / kGemmKTile;
-constexpr int kGgStages = 3;
-constexpr int kGgNTile = 128;
+constexpr int kGgNTile = 128;                                   // the widest tile; unit planes are padded to whole ones
 constexpr uint32_t kGgTileBytes = kGemmM * kGemmKTile;          // 16 KB: 128 rows x 128 B
-constexpr uint32_t kGgStageBytes = 4 * kGgTileBytes;            // wh | wl | xh | xl
-constexpr int kGgEpiWarps = 16;
-constexpr int kGgThreads = (2 + kGgEpiWarps) * 32;
+template <int kN> __host__ __device__ constexpr uint32_t gg_x_bytes() { return kN * kGemmKTile; }
+template <int kN> __host__ __device__ constexpr uint32_t gg_stage_bytes() { return 2 * kGgTileBytes + 2 * gg_x_bytes<kN>(); }    // wh | wl | xh | xl
+template <int kN> __host__ __device__ constexpr int gg_stages() { return kN == 32 ? 5 : kN == 64 ? 4 : 3; }
+template <int kN> __host__ __device__ constexpr int gg_epilogue_warps() { return kN / 8; }
+template <int kN> __host__ __device__ constexpr int gg_threads() { return (2 + gg_epilogue_warps<kN>()) * 32; }
 constexpr float kGgFullScale = 32639.0f;                        // 256 * 127 + 127
 
 struct GroupGemmParams {
     CUtensorMap map_wh[kGemmMaxTensors], map_wl[kGemmMaxTensors];   // [rows][K] int8, box 128 B x 128 rows, SWIZZLE_128B
-    CUtensorMap map_xh, map_xl;                                     // [tokens][K] int8, same box
+    CUtensorMap map_xh, map_xl;                                     // [tokens][K] int8, box 128 B x kN rows
     const float* w_unit[kGemmMaxTensors];   // [rows][groups]
     const float* x_unit;                    // [groups][t_ld]
     float* out[kGemmMaxTensors];            // [tokens][rows]
     uint32_t rows[kGemmMaxTensors];
     uint32_t m_start[kGemmMaxTensors];      // first row tile of each tensor in the launch's numbering (0xffffffff: unused)
     uint32_t tensors, tokens, groups, t_ld;
-    uint32_t m_tiles, n_tiles;
+    uint32_t m_tiles, n_tiles, n_columns;   // n_columns: tokens per tile
     uint32_t stream_k;                      // 1: CTAs share the (tile, group) units evenly; a tile is split between at most two CTAs
     int* error_word;
 };
 
-__host__ __device__ inline size_t gemm_groups_smem_bytes() { return 1024 + static_cast<size_t>(kGgStages) * kGgStageBytes + 256; }
+template <int kN> __host__ __device__ constexpr size_t gemm_groups_smem_bytes() { return 1024 + static_cast<size_t>(gg_stages<kN>()) * gg_stage_bytes<kN>() + 256; }
+
+// The tile's columns: fewest operand bytes through the busiest SM.  Tiles beyond the SMs are shared out evenly (stream-K), fewer
+// run side by side.
+inline uint32_t gg_tile_columns(uint32_t m_tiles, uint32_t tokens, uint32_t sms) {
+    uint32_t best = kGgNTile;
+    double best_cost = 0.0;
+    for (uint32_t n : {128u, 96u, 64u, 32u}) {
+        const uint32_t n_tiles = (tokens + n - 1) / n;
+        if (n_tiles * n > (tokens + kGgNTile - 1) / kGgNTile * kGgNTile) continue;      // the unit plane ends there
+        const double cost = std::max(1.0, static_cast<double>(m_tiles) * n_tiles / sms) * (kGemmM + n);
+        if (best_cost == 0.0 || cost < best_cost) { best_cost = cost; best = n; }
+    }
+    return best;
+}
 
 __device__ __forceinline__ void gg_locate(const GroupGemmParams& p, uint32_t mt_all, uint32_t& ti, uint32_t& mt) {
     ti = (mt_all >= p.m_start[1] ? 1u : 0u) + (mt_all >= p.m_start[2] ? 1u : 0u);
@@ -94,21 +117,26 @@ struct GroupWork {
     }
 };
 
-// Clears the output tiles two CTAs of a stream-K launch share (launched right before it, same grid).
-__global__ void gg_zero_split_tiles_kernel(const __grid_constant__ GroupGemmParams p) {
-    if (blockIdx.x == 0) return;
+// Clears the output tile that CTAs `cta` - 1 and `cta` of a stream-K launch of `ctas` share; all threads of a block.
+__device__ __forceinline__ void gg_zero_split_tile(const GroupGemmParams& p, uint32_t cta, uint32_t ctas) {
     const uint64_t total = static_cast<uint64_t>(p.m_tiles) * p.n_tiles * p.groups;
-    const uint32_t cut = static_cast<uint32_t>(total * blockIdx.x / gridDim.x);
+    const uint32_t cut = static_cast<uint32_t>(total * cta / ctas);
     if (cut % p.groups == 0) return;
     const uint32_t tile = cut / p.groups, nt = tile / p.m_tiles;
     uint32_t ti, mt;
     gg_locate(p, tile % p.m_tiles, ti, mt);
     float* out = p.out[ti];
     const uint32_t rows = p.rows[ti];
-    for (uint32_t i = threadIdx.x; i < kGgNTile * kGemmM; i += blockDim.x) {
-        const uint32_t t = nt * kGgNTile + i / kGemmM, r = mt * kGemmM + i % kGemmM;
+    for (uint32_t i = threadIdx.x; i < p.n_columns * kGemmM; i += blockDim.x) {
+        const uint32_t t = nt * p.n_columns + i / kGemmM, r = mt * kGemmM + i % kGemmM;
         if (t < p.tokens && r < rows) out[static_cast<size_t>(t) * rows + r] = 0.0f;
     }
+}
+// For the launches behind the first of one call (the first one's tiles are cleared beside the activations' digits).
+__global__ void gg_zero_split_tiles_kernel(const __grid_constant__ GroupGemmParams p) {
+    pdl_launch_dependents();
+    pdl_wait();
+    if (blockIdx.x) gg_zero_split_tile(p, blockIdx.x, gridDim.x);
 }
 
 // acc[c / 2] += (uw256 * ux[c]) * float(256 * a[c] + b[c]) for sixteen token columns; ux: their activation units.  The
@@ -125,8 +153,11 @@ __device__ __forceinline__ void gg_fold16(const uint32_t (&a)[16], const uint32_
     }
 }
 
-__global__ void __launch_bounds__(kGgThreads, 1) gemm_groups_kernel(const __grid_constant__ GroupGemmParams p) {
-    constexpr uint32_t kTmemCols = 512;             // two accumulator sets of (A, B) x 128 columns
+template <int kN>
+__global__ void __launch_bounds__(gg_threads<kN>(), 1) gemm_groups_kernel(const __grid_constant__ GroupGemmParams p) {
+    constexpr int kGgStages = gg_stages<kN>(), kGgEpiWarps = gg_epilogue_warps<kN>();
+    constexpr uint32_t kGgStageBytes = gg_stage_bytes<kN>(), kXBytes = gg_x_bytes<kN>();
+    constexpr uint32_t kTmemCols = kN > 64 ? 512 : 4 * kN;          // two accumulator sets of (A, B) x kN columns, a power of two
     extern __shared__ uint8_t smem_raw[];
     uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~static_cast<uintptr_t>(1023));
     uint64_t* full = reinterpret_cast<uint64_t*>(smem + kGgStages * kGgStageBytes);
@@ -157,12 +188,28 @@ __global__ void __launch_bounds__(kGgThreads, 1) gemm_groups_kernel(const __grid
     __syncthreads();
     tc_fence_after_sync();
     const uint32_t tmem_base = *tmem_base_slot;
+    pdl_launch_dependents();
 
     if (warp == 0) {
         // ---------------- TMA producer ----------------
         if (lane == 0) {
+            // The weights are constants: the ring's first stages are asked for before the previous launch (the activations'
+            // digits) has finished, their activations behind the wait.
             uint32_t it = 0, tile, g0, g1;
-            bool ok = true;
+            int late_k[kGgStages], late_n[kGgStages];
+            bool ok = true, waited = false;
+            auto load_x = [&](uint32_t stage, int kx, int n) {
+                uint8_t* st = smem + stage * kGgStageBytes + 2 * kGgTileBytes;
+                tma_load_2d(st, &p.map_xh, kx, n, &full[stage]);
+                tma_load_2d(st + kXBytes, &p.map_xl, kx, n, &full[stage]);
+            };
+            auto settle = [&](uint32_t stages) {
+                pdl_wait();
+                waited = true;
+#pragma unroll
+                for (int s = 0; s < kGgStages; ++s)
+                    if (s < static_cast<int>(stages)) load_x(s, late_k[s], late_n[s]);
+            };
             GroupWork work(p);
             while (ok && work.next(tile, g0, g1)) {
                 const uint32_t nt = tile / p.m_tiles;
@@ -170,6 +217,7 @@ __global__ void __launch_bounds__(kGgThreads, 1) gemm_groups_kernel(const __grid
                 gg_locate(p, tile % p.m_tiles, ti, mt);
                 for (uint32_t kt = g0 * kGgKTilesPerGroup; kt < g1 * kGgKTilesPerGroup; ++kt, ++it) {
                     const uint32_t stage = it % kGgStages;
+                    if (it == kGgStages && !waited) settle(kGgStages);
                     if (it >= kGgStages && !mbar_wait(&empty[stage], ((it / kGgStages) - 1) & 1)) {
                         *abort_word = 1; atomicExch(p.error_word, kErrEmptyWaitTimeout); ok = false;
                     }
@@ -180,15 +228,21 @@ __global__ void __launch_bounds__(kGgThreads, 1) gemm_groups_kernel(const __grid
                     mbar_arrive_expect_tx(&full[stage], kGgStageBytes);
                     tma_load_2d(st, &p.map_wh[ti], kx, static_cast<int>(mt * kGemmM), &full[stage]);
                     tma_load_2d(st + kGgTileBytes, &p.map_wl[ti], kx, static_cast<int>(mt * kGemmM), &full[stage]);
-                    tma_load_2d(st + 2 * kGgTileBytes, &p.map_xh, kx, static_cast<int>(nt * kGgNTile), &full[stage]);
-                    tma_load_2d(st + 3 * kGgTileBytes, &p.map_xl, kx, static_cast<int>(nt * kGgNTile), &full[stage]);
+                    if (waited) {
+                        load_x(stage, kx, static_cast<int>(nt * kN));
+                    } else {
+#pragma unroll
+                        for (int s = 0; s < kGgStages; ++s)
+                            if (s == static_cast<int>(stage)) { late_k[s] = kx; late_n[s] = static_cast<int>(nt * kN); }
+                    }
                 }
             }
+            if (!waited) settle(min(it, static_cast<uint32_t>(kGgStages)));
         }
     } else if (warp == 1) {
         // ---------------- MMA issuer ----------------
         if (lane == 0) {
-            constexpr uint32_t idesc = umma_idesc_i8(kGemmM, kGgNTile);
+            constexpr uint32_t idesc = umma_idesc_i8(kGemmM, kN);
             uint32_t it = 0, gcount = 0, tile, g0, g1;
             bool ok = true;
             GroupWork work(p);
@@ -202,7 +256,7 @@ __global__ void __launch_bounds__(kGgThreads, 1) gemm_groups_kernel(const __grid
                         }
                         tc_fence_after_sync();
                     }
-                    const uint32_t acc_a = tmem_base + set * 256, acc_b = acc_a + 128;
+                    const uint32_t acc_a = tmem_base + set * 2 * kN, acc_b = acc_a + kN;
                     for (uint32_t h = 0; h < static_cast<uint32_t>(kGgKTilesPerGroup) && ok; ++h, ++it) {
                         const uint32_t stage = it % kGgStages;
                         if (*abort_word || !mbar_wait(&full[stage], (it / kGgStages) & 1)) {
@@ -213,7 +267,7 @@ __global__ void __launch_bounds__(kGgThreads, 1) gemm_groups_kernel(const __grid
                         tc_fence_after_sync();
                         const uint32_t base = smem_u32(smem + stage * kGgStageBytes);
                         const uint64_t wh = umma_desc_k_sw128(base), wl = umma_desc_k_sw128(base + kGgTileBytes);
-                        const uint64_t xh = umma_desc_k_sw128(base + 2 * kGgTileBytes), xl = umma_desc_k_sw128(base + 3 * kGgTileBytes);
+                        const uint64_t xh = umma_desc_k_sw128(base + 2 * kGgTileBytes), xl = umma_desc_k_sw128(base + 2 * kGgTileBytes + kXBytes);
 #pragma unroll
                         for (uint32_t j = 0; j < static_cast<uint32_t>(kGemmBlocksPerTile); ++j) {
                             // 32 bytes of K = two 16-byte units further into the swizzle atom
@@ -236,6 +290,7 @@ __global__ void __launch_bounds__(kGgThreads, 1) gemm_groups_kernel(const __grid
         const uint32_t lane_addr = tmem_base + ((quad * 32) << 16) + part * 32;
         uint32_t gcount = 0, tile, g0, g1;
         bool ok = true;
+        pdl_wait();                                               // the units, the outputs and what they overwrite
         GroupWork work(p);
         while (ok && work.next(tile, g0, g1)) {
             const uint32_t nt = tile / p.m_tiles;
@@ -247,7 +302,7 @@ __global__ void __launch_bounds__(kGgThreads, 1) gemm_groups_kernel(const __grid
 #pragma unroll
             for (int c = 0; c < 16; ++c) acc[c] = 0ull;
             const float* uw_row = p.w_unit[ti] + static_cast<size_t>(row_ok ? r : 0) * p.groups;
-            const uint32_t col0 = nt * kGgNTile + part * 32;    // below t_ld: the unit plane is padded to whole tiles
+            const uint32_t col0 = nt * kN + part * 32;    // below t_ld: the unit plane is padded to whole tiles
             float uw_next = __ldg(uw_row + g0);
             for (uint32_t g = g0; g < g1 && ok; ++g, ++gcount) {
                 const uint32_t set = gcount & 1;
@@ -261,12 +316,12 @@ __global__ void __launch_bounds__(kGgThreads, 1) gemm_groups_kernel(const __grid
                 tc_fence_after_sync();
                 const float* ux = p.x_unit + static_cast<size_t>(g) * p.t_ld + col0;
                 uint32_t va[16], vb[16];
-                tmem_ld_32x16(lane_addr + set * 256, va);
-                tmem_ld_32x16(lane_addr + set * 256 + 128, vb);
+                tmem_ld_32x16(lane_addr + set * 2 * kN, va);
+                tmem_ld_32x16(lane_addr + set * 2 * kN + kN, vb);
                 tmem_ld_wait();
                 gg_fold16(va, vb, uw256, ux, acc);
-                tmem_ld_32x16(lane_addr + set * 256 + 16, va);
-                tmem_ld_32x16(lane_addr + set * 256 + 128 + 16, vb);
+                tmem_ld_32x16(lane_addr + set * 2 * kN + 16, va);
+                tmem_ld_32x16(lane_addr + set * 2 * kN + kN + 16, vb);
                 tmem_ld_wait();
                 tc_fence_before_sync();
                 __syncwarp();
@@ -411,11 +466,22 @@ __global__ void __launch_bounds__(256) group_digits_kq_kernel(const uint8_t* __r
 // Activations x [tokens][K] fp32 -> xh, xl [tokens][K] int8 and units [K / 256][t_ld] (group-major).  int8_mode: the values
 // are first quantised per 32-block exactly as the reference's int8 route does (round(x * 127 / amax), fp32 scale), and it is
 // d_x * q_x that gets the two digits; otherwise x itself (the reference's fp32-activation prefill).
+// The first `zero_ctas` blocks clear the output tiles that two CTAs of the product behind this launch will share (p; zero_ctas is
+// its grid, or 0); the columns past the last token get a zero unit.
 __global__ void __launch_bounds__(256) group_digits_acts_kernel(const float* __restrict__ x, int8_t* __restrict__ xh, int8_t* __restrict__ xl,
-                                                                float* __restrict__ unit_t, uint32_t tokens, uint32_t K, uint32_t t_ld, int int8_mode) {
-    const size_t wid = (static_cast<size_t>(blockIdx.x) * blockDim.x + threadIdx.x) >> 5;
+                                                                float* __restrict__ unit_t, uint32_t tokens, uint32_t K, uint32_t t_ld, int int8_mode,
+                                                                uint32_t zero_ctas, const __grid_constant__ GroupGemmParams p) {
+    pdl_launch_dependents();
+    pdl_wait();
+    if (blockIdx.x < zero_ctas) {
+        if (blockIdx.x) gg_zero_split_tile(p, blockIdx.x, zero_ctas);
+        return;
+    }
+    const size_t wid = (static_cast<size_t>(blockIdx.x - zero_ctas) * blockDim.x + threadIdx.x) >> 5;
     const int lane = threadIdx.x & 31;
     const uint32_t groups = K / kGgGroup;
+    if (wid < groups)
+        for (uint32_t c = tokens + lane; c < t_ld; c += 32) unit_t[wid * t_ld + c] = 0.0f;
     if (wid >= static_cast<size_t>(tokens) * groups) return;
     const uint32_t t = static_cast<uint32_t>(wid / groups), g = static_cast<uint32_t>(wid % groups);
     const size_t e0 = static_cast<size_t>(t) * K + static_cast<size_t>(g) * kGgGroup + lane * 8;

@@ -992,12 +992,15 @@ bool ensure_group_digits(State& s, const zen_cuda_weights* w, cudaStream_t st) {
     return true;
 }
 
-cudaError_t configure_gemm_groups() {
+template <int kN>
+cudaError_t launch_gemm_groups(State& s, const zk::GroupGemmParams& p, unsigned grid, cudaStream_t st) {
     static bool configured = false;
-    if (configured) return cudaSuccess;
-    const cudaError_t e = cudaFuncSetAttribute(&zk::gemm_groups_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(zk::gemm_groups_smem_bytes()));
-    if (e == cudaSuccess) configured = true;
-    return e;
+    if (!configured) {
+        const cudaError_t e = cudaFuncSetAttribute(&zk::gemm_groups_kernel<kN>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(zk::gemm_groups_smem_bytes<kN>()));
+        if (e != cudaSuccess) return e;
+        configured = true;
+    }
+    return launch_pdl(s, zk::gemm_groups_kernel<kN>, dim3(grid), dim3(zk::gg_threads<kN>()), zk::gemm_groups_smem_bytes<kN>(), st, p);
 }
 
 // All tensors have their two-digit planes (ensure_group_digits) and share the columns; `ws` holds gemm_groups_ws_bytes.
@@ -1005,19 +1008,12 @@ bool enqueue_gemm_groups(State& s, const zen_cuda_weights* const* w, float* cons
                          cudaStream_t st, int act_mode) {
     const size_t cols = w[0]->cols;
     const uint32_t groups = static_cast<uint32_t>(cols / zk::kGgGroup);
-    const uint32_t n_tiles = static_cast<uint32_t>((tokens + zk::kGgNTile - 1) / zk::kGgNTile), t_ld = n_tiles * zk::kGgNTile;
+    const uint32_t t_ld = static_cast<uint32_t>((tokens + zk::kGgNTile - 1) / zk::kGgNTile) * zk::kGgNTile;
     const size_t plane = (tokens * cols + 255) & ~size_t(255);
     int8_t* xh = reinterpret_cast<int8_t*>(ws);
     int8_t* xl = reinterpret_cast<int8_t*>(ws + plane);
     float* x_unit = reinterpret_cast<float*>(ws + 2 * plane);
-    if (tokens % zk::kGgNTile)      // the columns past the last token carry a zero unit
-        if (cudaMemsetAsync(x_unit, 0, static_cast<size_t>(groups) * t_ld * sizeof(float), st) != cudaSuccess) return set_error(s, "gemm: clearing the activation units failed");
-    const size_t warps = tokens * groups;
-    zk::group_digits_acts_kernel<<<static_cast<unsigned>((warps + 7) / 8), 256, 0, st>>>(d_x, xh, xl, x_unit, static_cast<uint32_t>(tokens), static_cast<uint32_t>(cols),
-                                                                                        t_ld, act_mode == ZEN_CUDA_ACT_INT8 ? 1 : 0);
-    if (cudaGetLastError() != cudaSuccess) return set_error(s, "gemm: activation digits launch failed");
-    ++s.stats.dispatches;
-    if (configure_gemm_groups() != cudaSuccess) return set_error(s, "gemm: shared-memory opt-in failed");
+    const unsigned digit_ctas = static_cast<unsigned>((tokens * groups + 7) / 8);
     for (size_t i0 = 0; i0 < count; i0 += zk::kGemmMaxTensors) {
         const size_t n = std::min<size_t>(zk::kGemmMaxTensors, count - i0);
         zk::GroupGemmParams p{};
@@ -1033,25 +1029,36 @@ bool enqueue_gemm_groups(State& s, const zen_cuda_weights* const* w, float* cons
             p.m_start[j] = m_tiles;
             m_tiles += (p.rows[j] + zk::kGemmM - 1) / zk::kGemmM;
         }
-        if (!make_map_2d(s, &p.map_xh, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, xh, cols, tokens, cols, zk::kGemmKTile, zk::kGgNTile, CU_TENSOR_MAP_SWIZZLE_128B)) return false;
-        if (!make_map_2d(s, &p.map_xl, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, xl, cols, tokens, cols, zk::kGemmKTile, zk::kGgNTile, CU_TENSOR_MAP_SWIZZLE_128B)) return false;
+        const uint32_t columns = zk::gg_tile_columns(m_tiles, static_cast<uint32_t>(tokens), static_cast<uint32_t>(s.sm_count));
+        if (!make_map_2d(s, &p.map_xh, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, xh, cols, tokens, cols, zk::kGemmKTile, columns, CU_TENSOR_MAP_SWIZZLE_128B)) return false;
+        if (!make_map_2d(s, &p.map_xl, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, xl, cols, tokens, cols, zk::kGemmKTile, columns, CU_TENSOR_MAP_SWIZZLE_128B)) return false;
         p.x_unit = x_unit;
         p.tensors = static_cast<uint32_t>(n);
         p.tokens = static_cast<uint32_t>(tokens);
         p.groups = groups;
         p.t_ld = t_ld;
         p.m_tiles = m_tiles;
-        p.n_tiles = n_tiles;
+        p.n_columns = columns;
+        p.n_tiles = static_cast<uint32_t>((tokens + columns - 1) / columns);
         p.error_word = s.d_error;
         const unsigned tiles = p.m_tiles * p.n_tiles;
         const unsigned grid = std::min<unsigned>(tiles, static_cast<unsigned>(s.sm_count));
         p.stream_k = (s.gemm_stream_k && tiles % grid != 0 && static_cast<uint64_t>(tiles) * groups / grid >= groups) ? 1u : 0u;
-        if (p.stream_k) {
-            zk::gg_zero_split_tiles_kernel<<<grid, 256, 0, st>>>(p);
+        if (i0 == 0) {
+            const uint32_t zero_ctas = p.stream_k ? grid : 0u;
+            if (launch_pdl(s, zk::group_digits_acts_kernel, dim3(digit_ctas + zero_ctas), dim3(256), 0, st, d_x, xh, xl, x_unit, static_cast<uint32_t>(tokens),
+                           static_cast<uint32_t>(cols), t_ld, act_mode == ZEN_CUDA_ACT_INT8 ? 1 : 0, zero_ctas, p) != cudaSuccess)
+                return set_error(s, "gemm: activation digits launch failed");
+            ++s.stats.dispatches;
+        } else if (p.stream_k) {
+            if (launch_pdl(s, zk::gg_zero_split_tiles_kernel, dim3(grid), dim3(256), 0, st, p) != cudaSuccess) return set_error(s, "gemm: clearing the split tiles failed");
             ++s.stats.dispatches;
         }
-        zk::gemm_groups_kernel<<<grid, zk::kGgThreads, zk::gemm_groups_smem_bytes(), st>>>(p);
-        if (cudaGetLastError() != cudaSuccess) return set_error(s, std::string("gemm launch: ") + cudaGetErrorString(cudaGetLastError()));
+        const cudaError_t e = columns == 128  ? launch_gemm_groups<128>(s, p, grid, st)
+                              : columns == 96 ? launch_gemm_groups<96>(s, p, grid, st)
+                              : columns == 64 ? launch_gemm_groups<64>(s, p, grid, st)
+                                              : launch_gemm_groups<32>(s, p, grid, st);
+        if (e != cudaSuccess) return set_error(s, std::string("gemm launch: ") + cudaGetErrorString(e));
         ++s.stats.dispatches;
     }
     return true;
