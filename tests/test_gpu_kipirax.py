@@ -207,6 +207,13 @@ def test_window_attention(be, heads, kv, dim, vdim, window, keep):
         close(got[prompt:], (want * ref.sigmoid(gates.astype(np.float64))[:, :, None])[prompt:], 1e-4)
 
 
+# The same on the tensor cores (heads padded to 128): windows and kept tokens around the borders of their blocks of 64 keys.
+@pytest.mark.parametrize("heads,kv,dim,vdim,window,keep", [(4, 2, 128, 128, 64, 4), (8, 2, 120, 100, 17, 70), (2, 2, 128, 112, 63, 65), (4, 1, 100, 128, 1, 2), (8, 1, 128, 128, 700, 0),
+                                                           (16, 2, 97, 128, 65, 64)])
+def test_window_attention_tiles(be, heads, kv, dim, vdim, window, keep):
+    test_window_attention(be, heads, kv, dim, vdim, window, keep)
+
+
 def test_attention_reports_a_position_past_the_cache(be):
     heads, kv, dim, vdim, T = 2, 1, 8, 8, 4
     kc, vc, out, w = zeros(T, kv, 32), zeros(T, kv, 32), zeros(8, heads, 32), dev(np.ones(dim))

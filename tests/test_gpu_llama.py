@@ -371,6 +371,37 @@ def test_attention_prefill_block(be, H, KH, D, T, pos0, window):
     assert_parity(out.cpu().numpy(), ref, 1e-5, "prefill attention")
 
 
+# Heads of 128 values on the tensor cores: a tile of 128 / (query heads per KV head) tokens and one more or fewer, blocks of 64 keys
+# full, begun and one key long, windows that begin inside a block, one token alone, a group that does not divide 128 beside them.
+@pytest.mark.parametrize("H,KH,T,pos0,window", [(4, 1, 31, 0, 0), (4, 1, 32, 1, 0), (4, 1, 33, 64, 0), (8, 8, 127, 1, 0), (8, 8, 129, 63, 0), (2, 1, 65, 190, 64), (4, 2, 64, 100, 63),
+                                                (16, 1, 9, 240, 0), (128, 1, 3, 5, 0), (32, 8, 17, 2, 9), (32, 8, 1, 0, 0), (3, 1, 40, 30, 0)])
+def test_attention_prefill_tiles(be, H, KH, T, pos0, window):
+    test_attention_prefill_block(be, H, KH, 128, T, pos0, window)
+
+
+def test_attention_prefill_precision_and_infinite_keys(be):
+    # scores of widely different sizes, values up to 1e6 beside small ones; a key whose score is minus infinity has no weight
+    import torch
+    H, KH, D, T, pos0, P = 4, 1, 128, 40, 150, 256
+    rng = np.random.default_rng(3)
+    q, kc = rng.standard_normal((T, H, D)).astype(np.float32) * 3, rng.standard_normal((P, D)).astype(np.float32)
+    vc = (rng.standard_normal((P, D)) * 10.0 ** rng.integers(-3, 7, (1, D))).astype(np.float32)
+    q[:, :, 5] = 1.0 + np.abs(q[:, :, 5])
+    kc[77, 5] = -np.inf
+    dq, dkc, dvc, dpos, out = dev(q), dev(kc), dev(vc), dev(np.array([pos0], np.int32)), torch.zeros((T, H, D), device="cuda")
+    torch.cuda.synchronize()
+    be.dev_attention_prefill(dq.data_ptr(), dkc.data_ptr(), dvc.data_ptr(), dpos.data_ptr(), out.data_ptr(), T, H, KH, D, P, 0.0, 0, 0)
+    torch.cuda.synchronize()
+    be.dev_check(0)
+    sc = np.einsum("thd,nd->htn", q.astype(np.float64), kc.astype(np.float64)) / np.sqrt(D)
+    sc = np.where(np.arange(P)[None, None, :] <= pos0 + np.arange(T)[None, :, None], sc, -np.inf)
+    a = np.exp(sc - sc.max(-1, keepdims=True))
+    ref = np.einsum("htn,nd->thd", a / a.sum(-1, keepdims=True), vc.astype(np.float64))
+    # per column, against the column's size: a score of up to 40 in fp32 (2^-24 of it, four roundings) moves a weight by 1e-5 at most
+    err = np.abs(out.cpu().numpy() - ref).max(axis=(0, 1)) / np.abs(ref).max(axis=(0, 1))
+    assert err.max() < 1e-5, err.max()
+
+
 def test_embed_and_rope_rows(be):
     import torch
     rows, cols, T = 300, 256, 19
@@ -474,6 +505,12 @@ def test_gate_up_launch_with_the_swiglu_store(be, mode, rows, cols, tokens, norm
         be.dev_gemv_fused(hs, [hid.data_ptr(), None], x.data_ptr(), tokens, mode, 0, swiglu_pair=True, accumulate=True)
     for h in hs:
         be.dev_free(h)
+
+
+@pytest.mark.parametrize("mode", [ACT_INT8, ACT_FP32])
+@pytest.mark.parametrize("rows,cols", [(8, 256), (149, 1024), (4096, 1024), (9500, 1024), (8192, 2048)])
+def test_gate_up_launch_of_short_rows(be, mode, rows, cols):
+    test_gate_up_launch_with_the_swiglu_store(be, mode, rows, cols, 1, True)
 
 
 @pytest.mark.parametrize("mode", [ACT_FP32, ACT_INT8])

@@ -25,6 +25,7 @@
 #include <unordered_map>
 #include <vector>
 
+#include "attention_tc.cuh"
 #include "decode_ops.cuh"
 #include "gemm_q8_0_i8.cuh"
 #include "gemm_groups.cuh"
@@ -2556,6 +2557,18 @@ int zen_cuda_dev_attention_prefill(const float* d_q, const float* d_k_cache, con
         (head_dim != 64 && head_dim != 128 && head_dim != 256))
         return set_error(s, "dev_attention_prefill: bad arguments (head_dim 64, 128 or 256)") ? 1 : 0;
     if (scale == 0.0f) scale = 1.0f / std::sqrt(static_cast<float>(head_dim));
+    if (const size_t ctas = zk::attention_tc_ctas(head_dim, tokens, heads, kv_heads)) {
+        if (ctas > 0x7fffffffu) return set_error(s, "dev_attention_prefill: too many tiles") ? 1 : 0;
+        auto* kernel = zk::attention_prefill_tc_kernel<false>;
+        static bool opted_in = false;                       // under the lock
+        if (!opted_in) {
+            ZC_CUDA(s, cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(zk::kTcSmem)));
+            opted_in = true;
+        }
+        ZC_DEV_LEAVE(launch_pdl(s, kernel, dim3(static_cast<unsigned>(ctas)), dim3(zk::kTcThreads), zk::kTcSmem, st, d_q, d_k_cache, d_v_cache, d_pos, d_out,
+                                static_cast<uint32_t>(tokens), static_cast<uint32_t>(heads), static_cast<uint32_t>(kv_heads), scale, static_cast<uint32_t>(window),
+                                static_cast<uint32_t>(max_positions), s.d_error, zk::AttnWindow{}));
+    }
     // query heads per thread: the largest of 4, 2, 1 that divides the group and keeps 2 * R * head_dim / 8 row values in registers
     const size_t group = heads / kv_heads;
     const int cap = head_dim == 256 ? 2 : 4;

@@ -9,6 +9,7 @@
 #include <type_traits>
 
 #include "attention.cuh"
+#include "attention_tc.cuh"
 #include "gemm_bf16.cuh"
 #include "gemv_bf16.cuh"
 #include "host_state.h"
@@ -299,6 +300,13 @@ int zen_cuda_dev_window_attention_rows(const zen_cuda_window_attention* a, const
         r = launch(e, zk::qk_norm_append_rows_kernel, dim3(u32(tokens)), dim3(256), 0, d_proj_q, d_proj_k, d_proj_v, u32(ld), win, a->heads, a->kv_heads, a->pitch,
                    d_pos, d_q, a->k_cache, a->v_cache, a->max_positions, e.d_error);
         if (!e.leave(r, "window_attention_rows: append")) return 0;
+    }
+    if (const size_t tiles = zk::attention_tc_ctas(a->pitch, tokens, a->heads, a->kv_heads)) {
+        if (tiles > 0x7fffffffu) return e.fail("window_attention_rows: too many tiles");
+        r = launch(e, zk::attention_prefill_tc_kernel<true>, dim3(u32(tiles)), dim3(zk::kTcThreads), zk::kTcSmem, static_cast<const float*>(d_q),
+                   static_cast<const float*>(a->k_cache), static_cast<const float*>(a->v_cache), d_pos, d_out, u32(tokens), a->heads, a->kv_heads, a->scale, a->window,
+                   a->max_positions, e.d_error, win);
+        return e.leave(r, "window_attention_rows");
     }
     const uint32_t group = a->heads / a->kv_heads;
     const int cap = a->pitch > 128 ? 2 : 4, r_heads = (cap >= 4 && group % 4 == 0) ? 4 : group % 2 == 0 ? 2 : 1;
