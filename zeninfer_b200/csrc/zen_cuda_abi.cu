@@ -1775,7 +1775,7 @@ bool host_rms_norm(State& s, const float* x, const float* weight, float* y, size
     const auto t0 = clock_type::now();
     for (size_t r0 = 0; r0 < rows; r0 += 65535) {
         const size_t nr = std::min<size_t>(65535, rows - r0);
-        const cudaError_t e = launch_pdl(s, zk::residual_rms_norm_kernel, dim3(static_cast<unsigned>(nr)), dim3(zk::kNormThreads), 0, s.stream,
+        const cudaError_t e = launch_pdl(s, zk::residual_rms_norm_kernel, dim3(static_cast<unsigned>(nr)), dim3(zk::norm_threads(nr, cols, s.sm_count)), 0, s.stream,
                                          s.d_x + off[0] + r0 * cols, static_cast<const float*>(nullptr), static_cast<const float*>(s.d_x + off[1]),
                                          s.d_y + r0 * cols, static_cast<uint32_t>(cols), eps);
         if (e != cudaSuccess) return set_error(s, std::string("rms_norm launch: ") + cudaGetErrorString(e));
@@ -2466,7 +2466,7 @@ int zen_cuda_dev_embed_q8_0(const zen_cuda_weights* w, const int64_t* d_token, f
 int zen_cuda_dev_rms_norm(float* d_x, const float* d_delta, const float* d_weight, float* d_y, size_t n, size_t rows, float eps, void* stream) {
     ZC_DEV_ENTER("dev_rms_norm");
     if (!d_x || !n || !rows || rows > 65535 || (d_weight && !d_y) || (!d_weight && !d_delta)) return set_error(s, "dev_rms_norm: bad arguments") ? 1 : 0;
-    const cudaError_t e = launch_pdl(s, zk::residual_rms_norm_kernel, dim3(static_cast<unsigned>(rows)), dim3(zk::kNormThreads), 0, st, d_x, d_delta, d_weight, d_y,
+    const cudaError_t e = launch_pdl(s, zk::residual_rms_norm_kernel, dim3(static_cast<unsigned>(rows)), dim3(zk::norm_threads(rows, n, s.sm_count)), 0, st, d_x, d_delta, d_weight, d_y,
                                      static_cast<uint32_t>(n), eps);
     ZC_DEV_LEAVE(e);
 }
@@ -2603,7 +2603,7 @@ int zen_cuda_dev_attention_prefill(const float* d_q, const float* d_k_cache, con
 int zen_cuda_dev_silu_mul(const float* d_gate, const float* d_up, float* d_out, size_t count, void* stream) {
     ZC_DEV_ENTER("dev_silu_mul");
     if (!d_gate || !d_up || !d_out || !count) return set_error(s, "dev_silu_mul: bad arguments") ? 1 : 0;
-    const cudaError_t e = launch_pdl(s, zk::silu_mul_kernel, dim3(static_cast<unsigned>(std::min<size_t>((count + 255) / 256, 4 * static_cast<size_t>(s.sm_count)))),
+    const cudaError_t e = launch_pdl(s, zk::silu_mul_kernel, dim3(static_cast<unsigned>(std::min<size_t>((count + 1023) / 1024, 8 * static_cast<size_t>(s.sm_count)))),
                                      dim3(256), 0, st, d_gate, d_up, d_out, count);
     ZC_DEV_LEAVE(e);
 }
