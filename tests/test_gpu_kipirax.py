@@ -44,6 +44,12 @@ def test_dense_gemv(be, rows, cols, act):
     be.dev_free(h)
 
 
+# Units of 256 columns that the warps of a row group do not share evenly (9, 17, 20, 31 and 72 units), over several row groups of a CTA.
+@pytest.mark.parametrize("rows,cols", [(2500, 2304), (2400, 5000), (1300, 4300), (4000, 7930), (2500, 18432)])
+def test_dense_gemv_of_uneven_units(be, rows, cols):
+    test_dense_gemv(be, rows, cols, DENSE_PLAIN)
+
+
 def test_dense_gemv_several_tasks(be):
     shapes = [(70, 40), (333, 1100), (5, 256), (201, 8)]
     mats = [bf16_matrix(be, r, c, i) for i, (r, c) in enumerate(shapes)]
