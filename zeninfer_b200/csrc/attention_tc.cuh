@@ -18,8 +18,8 @@
 // The scores of block j + 1 are formed while block j is exponentiated (a block leaves TMEM before anything else); keys and values
 // have one buffer each in shared memory (Q's planes take 96 KB of the 192), refilled while the other one's product runs.
 //
-// What bounds it: a block's chain through the row warps, about 3.5 us a block of 64 keys, of which the exponentials are a third, and
-// beside them the tensor pipe (72 products a block).  B200, 512 tokens, 32 heads on 8, at position 0 / 1488: 54 / 190 us, with fp32
+// What bounds it: a block's chain through the row warps, about 6 us a block of 64 keys, of which the exponentials are a third; the
+// tensor pipe (72 products a block) is busy for a third of that, memory hardly at all.  B200, 512 tokens, 32 heads on 8, at position 0 / 1488: 54 / 190 us, with fp32
 // multiply-adds on the CUDA cores 142 / 551; error against 64 bits (2-norm, unit normal inputs) 2.0e-7 / 2.9e-7, before 2.1e-7 /
 // 7.5e-7.  Five tokens at position 0 / 1500: 9.7 / 96 us, before 6.7 / 301; the host does not know the position, so all sizes go here.
 #pragma once
