@@ -402,6 +402,38 @@ def test_attention_prefill_precision_and_infinite_keys(be):
     assert err.max() < 1e-5, err.max()
 
 
+# Rows held in registers (128 to 512 threads a row), rows too long for that, rows of no whole words, one row fewer than there are SMs.
+@pytest.mark.parametrize("rows,n", [(147, 4096), (148, 4), (160, 2048), (150, 2052), (200, 4096), (150, 4100), (150, 8192), (149, 8196), (160, 30)])
+@pytest.mark.parametrize("with_delta", [False, True])
+def test_rms_norm_of_many_rows(be, rows, n, with_delta):
+    import torch
+    rng = np.random.default_rng(rows + n)
+    x, d, w = rng.standard_normal((rows, n), dtype=np.float32), rng.standard_normal((rows, n), dtype=np.float32), rng.standard_normal(n, dtype=np.float32)
+    dx, dd, dw, y = dev(x), dev(d), dev(w), torch.zeros((rows, n), device="cuda")
+    torch.cuda.synchronize()
+    be.dev_rms_norm(dx.data_ptr(), dd.data_ptr() if with_delta else None, dw.data_ptr(), y.data_ptr(), n, rows, 1e-5, 0)
+    torch.cuda.synchronize()
+    z = x + d if with_delta else x
+    assert np.array_equal(dx.cpu().numpy(), z)
+    want = z / np.sqrt((z.astype(np.float64) ** 2).mean(1, keepdims=True) + 1e-5) * w
+    assert_parity(y.cpu().numpy(), want, 1e-6, "rms norm")      # three fp32 roundings per value
+
+
+@pytest.mark.parametrize("count,offset", [(1, 0), (7, 0), (4096, 0), (4099, 1), (300000, 0), (300003, 3)])
+def test_silu_mul_words_and_tails(be, count, offset):
+    import torch
+    rng = np.random.default_rng(count)
+    g, u = rng.standard_normal(count + offset, dtype=np.float32) * 4, rng.standard_normal(count + offset, dtype=np.float32)
+    dg, du, out = dev(g), dev(u), torch.full((count + offset + 1,), 7.0, device="cuda")
+    torch.cuda.synchronize()
+    be.dev_silu_mul(dg.data_ptr() + 4 * offset, du.data_ptr() + 4 * offset, out.data_ptr() + 4 * offset, count, 0)
+    torch.cuda.synchronize()
+    z = g[offset:].astype(np.float64)
+    got = out.cpu().numpy()
+    assert_parity(got[offset:-1], z / (1 + np.exp(-z)) * u[offset:], 1e-6, "silu mul")     # expf, a division and two products in fp32
+    assert (got[:offset] == 7).all() and got[-1] == 7
+
+
 def test_embed_and_rope_rows(be):
     import torch
     rows, cols, T = 300, 256, 19
