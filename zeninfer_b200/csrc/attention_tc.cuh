@@ -115,7 +115,7 @@ __global__ void __launch_bounds__(kTcThreads, 1) attention_prefill_tc_kernel(con
     if (warp == kTcIssueWarp) tmem_alloc(tmem_slot, kTcColumns);
     pdl_launch_dependents();
     pdl_wait();
-    const int pos0 = *pos_ptr;
+    const int pos0 = __ldcg(pos_ptr);
     const bool good = pos0 >= 0 && static_cast<uint64_t>(pos0) + tokens <= max_positions;
     if (!good && threadIdx.x == 0 && blockIdx.x == 0) atomicExch(error_word, kErrBadPosition);
 
@@ -136,7 +136,7 @@ __global__ void __launch_bounds__(kTcThreads, 1) attention_prefill_tc_kernel(con
             float x[8] = {};
             if (t < t_end) {
                 const float4* src = reinterpret_cast<const float4*>(q + static_cast<size_t>(t) * qw + static_cast<size_t>(kh * group + row % group) * kTcDim + chunk * 8);
-                const float4 a = src[0], b = src[1];
+                const float4 a = __ldcg(src), b = __ldcg(src + 1);        // the launch before may write them
                 x[0] = a.x; x[1] = a.y; x[2] = a.z; x[3] = a.w; x[4] = b.x; x[5] = b.y; x[6] = b.z; x[7] = b.w;
             }
             uint4 plane[3];

@@ -141,13 +141,14 @@ __global__ void gg_zero_split_tiles_kernel(const __grid_constant__ GroupGemmPara
 
 // acc[c / 2] += (uw256 * ux[c]) * float(256 * a[c] + b[c]) for sixteen token columns; ux: their activation units.  The
 // two sums are combined as integers (|256 A + B| <= 256 * 256 * 127^2 + 512 * 127 * 128 < 2^31), so a column costs one
-// conversion, the scarce instruction here, instead of two.
-__device__ __forceinline__ void gg_fold16(const uint32_t (&a)[16], const uint32_t (&b)[16], float uw256, const float* __restrict__ ux, uint64_t* __restrict__ acc) {
+// conversion, the scarce instruction here, instead of two.  The units are plain loads, behind pdl_wait: the launch in front writes
+// them while this kernel is already resident, which the non-coherent path does not allow.
+__device__ __forceinline__ void gg_fold16(const uint32_t (&a)[16], const uint32_t (&b)[16], float uw256, const float* ux, uint64_t* __restrict__ acc) {
     const uint64_t uw2 = pack2(uw256, uw256);
     auto both = [&](int c) { return static_cast<float>(static_cast<int>(a[c]) * 256 + static_cast<int>(b[c])); };
 #pragma unroll
     for (int c = 0; c < 16; c += 4) {
-        const float4 u4 = __ldg(reinterpret_cast<const float4*>(ux + c));
+        const float4 u4 = *reinterpret_cast<const float4*>(ux + c);
         acc[c / 2] = fma2(pack2(both(c), both(c + 1)), mul2(pack2(u4.x, u4.y), uw2), acc[c / 2]);
         acc[c / 2 + 1] = fma2(pack2(both(c + 2), both(c + 3)), mul2(pack2(u4.z, u4.w), uw2), acc[c / 2 + 1]);
     }
@@ -485,7 +486,7 @@ __global__ void __launch_bounds__(256) group_digits_acts_kernel(const float* __r
     if (wid >= static_cast<size_t>(tokens) * groups) return;
     const uint32_t t = static_cast<uint32_t>(wid / groups), g = static_cast<uint32_t>(wid % groups);
     const size_t e0 = static_cast<size_t>(t) * K + static_cast<size_t>(g) * kGgGroup + lane * 8;
-    const float4 a = *reinterpret_cast<const float4*>(x + e0), b = *reinterpret_cast<const float4*>(x + e0 + 4);
+    const float4 a = __ldcg(reinterpret_cast<const float4*>(x + e0)), b = __ldcg(reinterpret_cast<const float4*>(x + e0 + 4));   // the launch before may write x
     float v[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
     if (int8_mode) {
         uint2 c1, c2;
