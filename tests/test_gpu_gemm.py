@@ -269,3 +269,29 @@ def test_group_scale_tiles_split_between_two_ctas(tokens):
     be.dev_free(h)
     want = group_product(blocks.dequantize(Q8_0, w, rows, cols), x)
     assert np.abs(got.astype(np.float64) - want).max() <= 2e-6 * np.abs(want).max()
+
+
+def test_group_scale_product_in_place():
+    # the output over the activations, 160 tiles (most of them split and cleared first): cleared only once the digits are formed, in a
+    # launch of its own
+    import torch
+    from zeninfer_b200 import Backend
+    be, n, tokens = Backend(), 2560, 1000
+    w, x = seeded_weights(Q8_0, n, n, 731), seeded_acts(tokens, n, 732)
+    h = be.dev_upload("Q8_0", w, n, n)
+    ws_bytes = be.gemm_workspace_bytes(tokens, n, ACT_FP32)
+    ws, y, d_x = torch.zeros(ws_bytes, dtype=torch.uint8, device="cuda"), torch.full((tokens, n), float("nan"), device="cuda"), torch.from_numpy(x).cuda()
+    torch.cuda.synchronize()
+
+    def product(out):
+        before = be.stats()["dispatches"]
+        be.dev_gemm_q8_0([h], [out.data_ptr()], d_x.data_ptr(), tokens, ws.data_ptr(), ws_bytes, act_mode=ACT_FP32)
+        be.dev_check()
+        return be.stats()["dispatches"] - before
+
+    product(y)
+    launches = product(y)
+    want = y.cpu().numpy()
+    assert product(d_x) == launches + 1
+    be.dev_free(h)
+    assert np.array_equal(d_x.cpu().numpy(), want)

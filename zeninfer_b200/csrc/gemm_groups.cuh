@@ -132,7 +132,8 @@ __device__ __forceinline__ void gg_zero_split_tile(const GroupGemmParams& p, uin
         if (t < p.tokens && r < rows) out[static_cast<size_t>(t) * rows + r] = 0.0f;
     }
 }
-// For the launches behind the first of one call (the first one's tiles are cleared beside the activations' digits).
+// For the launches behind the first of one call, and for products in place (otherwise the first one's tiles are cleared beside the
+// activations' digits).
 __global__ void gg_zero_split_tiles_kernel(const __grid_constant__ GroupGemmParams p) {
     pdl_launch_dependents();
     pdl_wait();

@@ -19,6 +19,7 @@
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
+#include <functional>
 #include <mutex>
 #include <string>
 #include <type_traits>
@@ -1004,6 +1005,13 @@ cudaError_t launch_gemm_groups(State& s, const zk::GroupGemmParams& p, unsigned 
     return launch_pdl(s, zk::gemm_groups_kernel<kN>, dim3(grid), dim3(zk::gg_threads<kN>()), zk::gemm_groups_smem_bytes<kN>(), st, p);
 }
 
+// Whether an output of the launch shares memory with the `n` floats at d_x.
+bool outputs_overlap(const zk::GroupGemmParams& p, const float* d_x, size_t n) {
+    for (uint32_t j = 0; j < p.tensors; ++j)
+        if (std::less<const float*>()(p.out[j], d_x + n) && std::less<const float*>()(d_x, p.out[j] + static_cast<size_t>(p.tokens) * p.rows[j])) return true;
+    return false;
+}
+
 // All tensors have their two-digit planes (ensure_group_digits) and share the columns; `ws` holds gemm_groups_ws_bytes.
 bool enqueue_gemm_groups(State& s, const zen_cuda_weights* const* w, float* const* d_out, size_t count, const float* d_x, size_t tokens, uint8_t* ws,
                          cudaStream_t st, int act_mode) {
@@ -1045,13 +1053,17 @@ bool enqueue_gemm_groups(State& s, const zen_cuda_weights* const* w, float* cons
         const unsigned tiles = p.m_tiles * p.n_tiles;
         const unsigned grid = std::min<unsigned>(tiles, static_cast<unsigned>(s.sm_count));
         p.stream_k = (s.gemm_stream_k && tiles % grid != 0 && static_cast<uint64_t>(tiles) * groups / grid >= groups) ? 1u : 0u;
+        // The first launch's split tiles are cleared beside the digits, unless an output lies over the activations (a product in
+        // place): the digits are then formed first, and the tiles cleared in a launch of their own.
+        const bool clear_beside = p.stream_k && i0 == 0 && !outputs_overlap(p, d_x, tokens * cols);
         if (i0 == 0) {
-            const uint32_t zero_ctas = p.stream_k ? grid : 0u;
+            const uint32_t zero_ctas = clear_beside ? grid : 0u;
             if (launch_pdl(s, zk::group_digits_acts_kernel, dim3(digit_ctas + zero_ctas), dim3(256), 0, st, d_x, xh, xl, x_unit, static_cast<uint32_t>(tokens),
                            static_cast<uint32_t>(cols), t_ld, act_mode == ZEN_CUDA_ACT_INT8 ? 1 : 0, zero_ctas, p) != cudaSuccess)
                 return set_error(s, "gemm: activation digits launch failed");
             ++s.stats.dispatches;
-        } else if (p.stream_k) {
+        }
+        if (p.stream_k && !clear_beside) {
             if (launch_pdl(s, zk::gg_zero_split_tiles_kernel, dim3(grid), dim3(256), 0, st, p) != cudaSuccess) return set_error(s, "gemm: clearing the split tiles failed");
             ++s.stats.dispatches;
         }
