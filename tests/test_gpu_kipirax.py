@@ -220,6 +220,34 @@ def test_window_attention_tiles(be, heads, kv, dim, vdim, window, keep):
     test_window_attention(be, heads, kv, dim, vdim, window, keep)
 
 
+def test_window_attention_infinite_values(be):
+    # a value that is not finite reaches the tokens that see its position: kept ones all later tokens, others those of the window
+    heads, kv, dim, vdim, window, keep, T, eps = 4, 2, 128, 120, 20, 5, 150, 1e-5
+    q, k, v, qw, kw = cases.standout_attention(T, heads, kv, dim, vdim, [], window)
+    planted = [(2, 0, 1, np.inf), (60, 0, 2, -np.inf), (61, 0, 2, np.inf), (100, 1, 3, np.nan), (149, 0, 119, np.inf)]
+    for j, h, col, x in planted:
+        v[j, h, col] = 0.0
+    scale = dim ** -0.5
+    qn, kn = ref.rms(q.astype(np.float64), eps) * qw, ref.rms(k.astype(np.float64), eps) * kw
+    want = ref.window_attention(qn, kn, v.astype(np.float64), scale, window, keep)
+    t = np.arange(T)
+    with np.errstate(invalid="ignore"):
+        for j, h, col, x in planted:
+            v[j, h, col] = x
+            want[(t >= j) & ((t - j < window) | (j < keep)), h * 2:h * 2 + 2, col] += x
+    row = heads * dim + kv * dim + kv * vdim
+    proj = dev(np.concatenate([q.reshape(T, -1), k.reshape(T, -1), v.reshape(T, -1)], axis=1))
+    kc, vc, qb, out = zeros(T, kv, 128), zeros(T, kv, 128), zeros(T, heads, 128), zeros(T, heads, 128)
+    dq, dk, pos = dev(qw), dev(kw), dev([0], np.int32)
+    a = WindowAttention(heads, kv, dim, vdim, 128, window, keep, 1, T, scale, eps, dq.data_ptr(), dk.data_ptr(), kc.data_ptr(), vc.data_ptr())
+    at = lambda col: proj.data_ptr() + 4 * col
+    be.dev_window_attention_rows(a, at(0), at(heads * dim), at((heads + kv) * dim), row, T, pos.data_ptr(), qb.data_ptr(), out.data_ptr())
+    be.dev_check(0)
+    got, ok = host(out)[:, :, :vdim], np.isfinite(want)
+    assert np.array_equal(np.isnan(got), np.isnan(want)) and np.array_equal(got[~ok & ~np.isnan(want)], want[~ok & ~np.isnan(want)])
+    close(got[ok], want[ok], 1e-4)
+
+
 def test_attention_reports_a_position_past_the_cache(be):
     heads, kv, dim, vdim, T = 2, 1, 8, 8, 4
     kc, vc, out, w = zeros(T, kv, 32), zeros(T, kv, 32), zeros(8, heads, 32), dev(np.ones(dim))

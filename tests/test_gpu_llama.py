@@ -402,6 +402,37 @@ def test_attention_prefill_precision_and_infinite_keys(be):
     assert err.max() < 1e-5, err.max()
 
 
+# A value that is not finite reaches the rows that attend its position and no others, as itself; early and late in a tile, in blocks that
+# the tile's first rows do not attend, left behind by a window, and two of them in one column.
+@pytest.mark.parametrize("H,KH,T,pos0,window", [(4, 1, 40, 150, 0), (4, 2, 70, 100, 30), (8, 8, 130, 20, 0), (2, 2, 12, 0, 0)])
+def test_attention_prefill_infinite_values(be, H, KH, T, pos0, window):
+    import torch
+    D, P = 128, pos0 + T
+    rng = np.random.default_rng(T)
+    q, kc, vc = (rng.standard_normal(shape).astype(np.float32) for shape in ((T, H, D), (P, KH, D), (P, KH, D)))
+    planted = [(pos0 // 2, 0, 3, np.inf), (P - 1, 0, 5, -np.inf), (P - 8, KH - 1, 70, np.nan), (P - T // 2, 0, 100, np.inf), (P - T // 2 + 3, 0, 100, -np.inf), (pos0 + 1, KH - 1, 127, -np.inf)]
+    finite = vc.copy()
+    for pos, kh, col, v in planted:
+        vc[pos, kh, col], finite[pos, kh, col] = v, 0.0
+    dq, dkc, dvc, dpos, out = dev(q), dev(kc), dev(vc), dev(np.array([pos0], np.int32)), torch.zeros((T, H, D), device="cuda")
+    torch.cuda.synchronize()
+    be.dev_attention_prefill(dq.data_ptr(), dkc.data_ptr(), dvc.data_ptr(), dpos.data_ptr(), out.data_ptr(), T, H, KH, D, P, 0.0, window, 0)
+    torch.cuda.synchronize()
+    be.dev_check(0)
+    at, tt = np.arange(P)[None, :], np.arange(pos0, P)[:, None]
+    seen = (at <= tt) & ((at > tt - window) if window else True)
+    sc = np.einsum("thd,nhd->htn", q.astype(np.float64), np.repeat(kc, H // KH, 1).astype(np.float64)) / np.sqrt(D)
+    sc = np.where(seen[None], sc, -np.inf)
+    a = np.exp(sc - sc.max(-1, keepdims=True))
+    want = np.einsum("htn,nhd->thd", a / a.sum(-1, keepdims=True), np.repeat(finite, H // KH, 1).astype(np.float64))
+    with np.errstate(invalid="ignore"):
+        for pos, kh, col, v in planted:
+            want[seen[:, pos], kh * (H // KH):(kh + 1) * (H // KH), col] += v
+    got, ok = out.cpu().numpy(), np.isfinite(want)
+    assert np.array_equal(np.isnan(got), np.isnan(want)) and np.array_equal(got[~ok & ~np.isnan(want)], want[~ok & ~np.isnan(want)])
+    assert_parity(got[ok], want[ok], 1e-5, "finite outputs")
+
+
 # Rows held in registers (128 to 512 threads a row), rows too long for that, rows of no whole words, one row fewer than there are SMs.
 @pytest.mark.parametrize("rows,n", [(147, 4096), (148, 4), (160, 2048), (150, 2052), (200, 4096), (150, 4100), (150, 8192), (149, 8196), (160, 30)])
 @pytest.mark.parametrize("with_delta", [False, True])

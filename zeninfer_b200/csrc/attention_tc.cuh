@@ -18,6 +18,10 @@
 // The scores of block j + 1 are formed while block j is exponentiated (a block leaves TMEM before anything else); keys and values
 // have one buffer each in shared memory (Q's planes take 96 KB of the 192), refilled while the other one's product runs.
 //
+// Rows whose output is not finite are formed once more with fp32 multiply-adds at the end, over the positions they attend alone: the
+// products multiply every value of a block by every row's weights, zeros among them, so that an infinite or NaN value would reach
+// rows of the tile that do not attend it.
+//
 // What bounds it: a block's chain through the row warps, about 6 us a block of 64 keys, of which the exponentials are a third; the
 // tensor pipe (72 products a block) is busy for a third of that, memory hardly at all.  B200, 512 tokens, 32 heads on 8, at position 0 / 1488: 54 / 190 us, with fp32
 // multiply-adds on the CUDA cores 142 / 551; error against 64 bits (2-norm, unit normal inputs) 2.0e-7 / 2.9e-7, before 2.1e-7 /
@@ -36,7 +40,8 @@ constexpr uint32_t kTcSmem = 1024 + 3 * (kTcQPlane + kTcKPlane + kTcVPlane) + 4 
 // TMEM columns: leading scores of three parts of the head, corrections; three planes of P; O'
 constexpr uint32_t kTcCorrections = 3 * kTcKeys, kTcP = 256, kTcOut = 384, kTcColumns = 512;
 
-// x = plane 0 + plane 1 + plane 2, exactly, as the upper halves of the returned words; where x is not finite plane 0 alone says so.
+// x = plane 0 + plane 1 + plane 2, exactly, as the upper halves of the returned words; where x is infinite plane 0 says so and the
+// others are NaN.
 __device__ __forceinline__ void split3(float x, uint32_t& a, uint32_t& b, uint32_t& c) {
     a = __float_as_uint(x);
     const float r = x - __uint_as_float(a & 0xffff0000u);
@@ -152,6 +157,7 @@ __global__ void __launch_bounds__(kTcThreads, 1) attention_prefill_tc_kernel(con
     tc_fence_after_sync();
     const uint32_t tmem = *tmem_slot;
 
+    uint32_t todo = 0, first_row = 0, lanes_of = 2;           // rows left to this warp below: bits from first_row on; half of the head it stores (2: both)
     // A wait that runs out ends its role's loop, and the others' follow.
     if (!good) {
     } else if (warp < kTcKeyWarp) {                           // rows
@@ -170,6 +176,7 @@ __global__ void __launch_bounds__(kTcThreads, 1) attention_prefill_tc_kernel(con
                 : "=r"(any) : "r"(quad + 1), "r"(64u), "r"(static_cast<uint32_t>(failed)) : "memory");
             return any != 0;
         };
+        bool again = false;
         float acc[kTcDim / 2], m = -INFINITY, factor = 0.0f;
         double l = 0.0;
 #pragma unroll
@@ -284,12 +291,19 @@ __global__ void __launch_bounds__(kTcThreads, 1) attention_prefill_tc_kernel(con
                 atomicExch(error_word, kErrNonFinite);
             } else {
                 const float inv = 1.0f / static_cast<float>(l);
+                float nonfinite = 0.0f;
+#pragma unroll
+                for (int i = 0; i < static_cast<int>(kTcDim / 2); ++i) { acc[i] *= inv; nonfinite = fmaf(acc[i], 0.0f, nonfinite); }
+                again = nonfinite != 0.0f;
                 float4* dst = reinterpret_cast<float4*>(out + static_cast<size_t>(t) * qw + static_cast<size_t>(h) * kTcDim + half * (kTcDim / 2));
 #pragma unroll
                 for (int i = 0; i < static_cast<int>(kTcDim / 8); ++i)
-                    dst[i] = make_float4(acc[4 * i] * inv, acc[4 * i + 1] * inv, acc[4 * i + 2] * inv, acc[4 * i + 3] * inv);
+                    if (!again) dst[i] = make_float4(acc[4 * i], acc[4 * i + 1], acc[4 * i + 2], acc[4 * i + 3]);
             }
         }
+        first_row = quad * 32;
+        todo = __ballot_sync(0xffffffffu, again);
+        lanes_of = half;
     } else if (warp < kTcValueWarp) {                         // keys: a thread takes eight values of a key at a time
         constexpr uint32_t kId = (kTcValueWarp - kTcKeyWarp) * 32, kItems = kTcKeys * kTcDim / 8, kEach = kItems / kId;
         const uint32_t id = threadIdx.x - kTcKeyWarp * 32;
@@ -403,6 +417,92 @@ __global__ void __launch_bounds__(kTcThreads, 1) attention_prefill_tc_kernel(con
             p0 = p1;
         }
         if (!ok) atomicExch(error_word, kErrFullWaitTimeout);
+    }
+    __syncwarp();
+    // Rows again with fp32 multiply-adds, four at a time and four keys a round, a lane holding four columns: those with an output that is
+    // not finite.  The products above multiply every value of a block, by zero where a row does not attend it, and a value's lower
+    // planes are NaN where it is infinite; here a row meets the values it attends and no others, each as it is.
+    while (todo) {
+        uint32_t rows[4], mine = 0;
+        float4 x[4], o[4];
+#pragma unroll
+        for (uint32_t r = 0; r < 4; ++r) {                    // fewer rows than four: the last one several times
+            rows[r] = todo ? first_row + __ffs(todo) - 1 : rows[r - (r > 0)];
+            todo &= todo - 1u;                                // 0 stays 0
+            if (lane >> 3 == r) mine = rows[r];
+            uint2 plane[3];
+            const uint32_t at = (lane / 16) * (kTcQPlane / 2) + rows[r] * 128 + (((lane % 16 / 2) ^ (rows[r] & 7)) << 4) + (lane & 1) * 8;
+#pragma unroll
+            for (int p = 0; p < 3; ++p) plane[p] = *reinterpret_cast<const uint2*>(q_smem + p * kTcQPlane + at);
+            auto sum3 = [&](auto part) { return part(plane[0]) + (part(plane[1]) + part(plane[2])); };     // exact, smallest first
+            x[r] = make_float4(sum3([](uint2 w) { return __uint_as_float(w.x << 16); }), sum3([](uint2 w) { return __uint_as_float(w.x & 0xffff0000u); }),
+                               sum3([](uint2 w) { return __uint_as_float(w.y << 16); }), sum3([](uint2 w) { return __uint_as_float(w.y & 0xffff0000u); }));
+            o[r] = make_float4(0.f, 0.f, 0.f, 0.f);
+        }
+        // a lane keeps the state of row lane / 8 and the score of key lane / 2 % 4
+        const uint32_t t = t0 + mine / group, my_last = static_cast<uint32_t>(pos0) + t, end = static_cast<uint32_t>(pos0) + t0 + rows[3] / group;
+        const uint32_t my_first = (window && my_last + 1 > window) ? my_last + 1 - window : 0u;
+        const float slope = kWindowed && win.biased ? attn_slope(kh * group + mine % group, heads) : 0.0f;
+        const size_t column = static_cast<size_t>(kh) * kTcDim + lane * 4;
+        float m = -INFINITY;
+        double l = 0.0;
+        for (uint32_t p0 = start; p0 <= end; p0 = kWindowed && p0 < kept_end && p0 + 4 >= kept_end ? first_any : p0 + 4) {
+            const uint32_t last = part_last(p0), pos = p0 + lane / 2 % 4;
+            const bool attended = pos <= min(my_last, last) && (pos >= my_first || (kWindowed && pos < win.keep_first));
+            if (!__any_sync(0xffffffffu, attended)) continue;
+            float4 key[4], value[4];
+#pragma unroll
+            for (uint32_t k = 0; k < 4; ++k) {
+                const size_t off = static_cast<size_t>(min(p0 + k, last)) * kw + column;
+                key[k] = __ldca(reinterpret_cast<const float4*>(k_cache + off));
+                value[k] = __ldca(reinterpret_cast<const float4*>(v_cache + off));
+            }
+            float s[16];                                      // summed over the lanes, which at each exchange keep half of the sums they carry
+#pragma unroll
+            for (int i = 0; i < 16; ++i) s[i] = fmaf(x[i / 4].w, key[i % 4].w, fmaf(x[i / 4].z, key[i % 4].z, fmaf(x[i / 4].y, key[i % 4].y, x[i / 4].x * key[i % 4].x)));
+#pragma unroll
+            for (int h = 8; h > 0; h >>= 1) {
+                const bool up = lane & (2 * h);
+#pragma unroll
+                for (int i = 0; i < h; ++i) s[i] = (up ? s[i + h] : s[i]) + __shfl_xor_sync(0xffffffffu, up ? s[i] : s[i + h], 2 * h);
+            }
+            float score = (s[0] + __shfl_xor_sync(0xffffffffu, s[0], 1)) * scale;
+            if (kWindowed) score -= slope * static_cast<float>(static_cast<int>(my_last) - static_cast<int>(pos));
+            float most = attended ? fmaxf(m, score) : m;
+            most = fmaxf(most, __shfl_xor_sync(0xffffffffu, most, 2));
+            most = fmaxf(most, __shfl_xor_sync(0xffffffffu, most, 4));
+            const bool moved = most > m;
+            if (__any_sync(0xffffffffu, moved)) {
+                const float f = moved ? expf(m - most) : 1.0f;
+                l *= f;
+                m = most;
+#pragma unroll
+                for (int r = 0; r < 4; ++r) {
+                    const float fr = __shfl_sync(0xffffffffu, f, 8 * r);
+                    o[r].x *= fr; o[r].y *= fr; o[r].z *= fr; o[r].w *= fr;
+                }
+            }
+            const float e = attended ? expf(score - (m == -INFINITY ? 0.0f : m)) : -1.0f;      // below zero: not attended
+            if (attended) l += e;
+#pragma unroll
+            for (int i = 0; i < 16; ++i) {
+                const float p = __shfl_sync(0xffffffffu, e, 2 * i);
+                if (p < 0.0f) continue;
+                float4& to = o[i / 4];
+                const float4& v = value[i % 4];
+                to.x = fmaf(p, v.x, to.x); to.y = fmaf(p, v.y, to.y); to.z = fmaf(p, v.z, to.z); to.w = fmaf(p, v.w, to.w);
+            }
+        }
+        l += __shfl_xor_sync(0xffffffffu, l, 2);
+        l += __shfl_xor_sync(0xffffffffu, l, 4);
+        const float inv = 1.0f / static_cast<float>(l);
+#pragma unroll
+        for (int r = 0; r < 4; ++r) {
+            const float to = __shfl_sync(0xffffffffu, inv, 8 * r);
+            if (lanes_of < 2 && lane / 16 != lanes_of) continue;
+            *reinterpret_cast<float4*>(out + static_cast<size_t>(t0 + rows[r] / group) * qw + static_cast<size_t>(kh * group + rows[r] % group) * kTcDim + lane * 4) =
+                make_float4(o[r].x * to, o[r].y * to, o[r].z * to, o[r].w * to);
+        }
     }
     tc_fence_before_sync();
     __syncthreads();
