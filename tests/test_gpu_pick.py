@@ -162,6 +162,24 @@ def test_sampling_matches_the_reference_distribution(be, n, temperature, top_k, 
         assert int(d_trunc.item()) == (0 if fits else 1)
 
 
+def test_many_draws_of_one_row_agree(be):
+    # the candidates are selected, sorted and summed through shared memory: launch after launch the same tokens and probabilities
+    import torch
+    rng = np.random.default_rng(11)
+    logits = (rng.standard_normal(32000) * 2.0).astype(np.float32)
+    want = reference_distribution(logits, 0.9, 40, 0.95)
+    kept, draws = np.flatnonzero(want), 4000
+    d_logits, d_pick = torch.from_numpy(logits).cuda(), torch.full((draws,), -7, dtype=torch.int64, device="cuda")
+    d_ids, d_count = torch.full((draws, 1024), -1, dtype=torch.int32, device="cuda"), torch.zeros(draws, dtype=torch.int32, device="cuda")
+    torch.cuda.synchronize()
+    for i in range(draws):
+        be.dev_sample(d_logits.data_ptr(), logits.size, 0.9, 40, 0.95, 0.5, d_pick[i].data_ptr(), 0, d_kept_ids=d_ids[i].data_ptr(), d_kept_count=d_count[i].data_ptr())
+    torch.cuda.synchronize()
+    be.dev_check(0)
+    assert (d_count == kept.size).all() and (d_ids[:, :kept.size].cpu().numpy() == kept).all()
+    assert (d_pick == d_pick[0]).all() and int(d_pick[0]) == kept[np.searchsorted(np.cumsum(want[kept]), 0.5)]
+
+
 def test_sampling_ties_and_degenerate_rows(be):
     import torch
     # all logits equal: top_k = 5 keeps the five lowest ids with equal probabilities

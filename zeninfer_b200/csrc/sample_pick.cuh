@@ -104,6 +104,7 @@ __global__ void __launch_bounds__(kSampleThreads) sample_top_kernel(const Sample
         mask |= 255u << shift;
     }
     const uint32_t threshold = s_prefix, need_ties = s_remaining, ties = s_count;
+    __syncthreads();           // all have read them: s_count is counted anew below
 
     // ---- collect: everything above T, and of the keys equal to T the `need_ties` lowest indices
     if (tid == 0) { s_count = 0; s_ties_taken = 0; }
