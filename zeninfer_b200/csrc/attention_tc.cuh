@@ -58,12 +58,7 @@ __device__ __forceinline__ void split3_8(const float (&x)[8], uint4 (&plane)[3])
     for (int p = 0; p < 3; ++p)
         plane[p] = make_uint4(upper_halves(w[p][0], w[p][1]), upper_halves(w[p][2], w[p][3]), upper_halves(w[p][4], w[p][5]), upper_halves(w[p][6], w[p][7]));
 }
-// D[tmem] (+)= A * B[smem], bf16 x bf16 -> fp32; A in shared memory, or in TMEM: a row per lane, two columns of K per 32-bit word.
-__device__ __forceinline__ void tc_mma_f16_ss(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc, uint32_t accumulate) {
-    asm volatile(
-        "{ .reg .pred p; setp.ne.b32 p, %4, 0; tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p; }"
-        ::"r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate) : "memory");
-}
+// D[tmem] (+)= A[tmem] * B[smem], bf16 x bf16 -> fp32; A: a row per lane, two columns of K per 32-bit word.
 __device__ __forceinline__ void tc_mma_f16_ts(uint32_t d_tmem, uint32_t a_tmem, uint64_t b_desc, uint32_t idesc, uint32_t accumulate) {
     asm volatile(
         "{ .reg .pred p; setp.ne.b32 p, %4, 0; tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p; }"
@@ -381,7 +376,7 @@ __global__ void __launch_bounds__(kTcThreads, 1) attention_prefill_tc_kernel(con
             }
         }
     } else if (lane == 0) {                                   // the tensor cores
-        auto idesc = [](uint32_t n) { return (1u << 4) | (1u << 7) | (1u << 10) | ((n >> 3) << 17) | ((kTcRows >> 4) << 24); };
+        constexpr uint32_t score_desc = umma_idesc_bf16(kTcRows, kTcKeys), out_desc = umma_idesc_bf16(kTcRows, kTcDim);
         constexpr uint32_t kFirst[6] = {2, 0, 1, 1, 0, 0}, kSecond[6] = {0, 2, 1, 0, 1, 0};      // planes of the two operands, the smallest products first
         const uint64_t q_desc = umma_desc_k_sw128(smem_u32(q_smem)), k_desc = umma_desc_k_sw128(smem_u32(k_smem)), v_desc = umma_desc_k_sw128(smem_u32(v_smem));
         // a descriptor's start address counts 16-byte units; 16 columns of K are two of them
@@ -390,8 +385,8 @@ __global__ void __launch_bounds__(kTcThreads, 1) attention_prefill_tc_kernel(con
             for (int c = 0; c < 6; ++c)
 #pragma unroll
                 for (uint32_t k = 0; k < 8; ++k)
-                    tc_mma_f16_ss(tmem + (c == 5 ? k / 3 * kTcKeys : kTcCorrections), q_desc + ((kFirst[c] * kTcQPlane + (k / 4) * (kTcQPlane / 2)) >> 4) + 2 * (k % 4),
-                                  k_desc + ((kSecond[c] * kTcKPlane + (k / 4) * (kTcKPlane / 2)) >> 4) + 2 * (k % 4), idesc(kTcKeys), c == 5 ? k % 3 > 0 : (c | k) > 0);
+                    tc_mma_f16(tmem + (c == 5 ? k / 3 * kTcKeys : kTcCorrections), q_desc + ((kFirst[c] * kTcQPlane + (k / 4) * (kTcQPlane / 2)) >> 4) + 2 * (k % 4),
+                                  k_desc + ((kSecond[c] * kTcKPlane + (k / 4) * (kTcKPlane / 2)) >> 4) + 2 * (k % 4), score_desc, c == 5 ? k % 3 > 0 : (c | k) > 0);
             tc_commit(s_full);
         };
         bool ok = mbar_wait(k_full, 0);
@@ -412,7 +407,7 @@ __global__ void __launch_bounds__(kTcThreads, 1) attention_prefill_tc_kernel(con
             for (int c = 0; c < 6; ++c)
 #pragma unroll
                 for (uint32_t k = 0; k < 4; ++k)
-                    tc_mma_f16_ts(tmem + kTcOut, tmem + kTcP + 32 * kFirst[c] + 8 * k, v_desc + (kSecond[c] * kTcVPlane >> 4) + 2 * k, idesc(kTcDim), (c | k) > 0);
+                    tc_mma_f16_ts(tmem + kTcOut, tmem + kTcP + 32 * kFirst[c] + 8 * k, v_desc + (kSecond[c] * kTcVPlane >> 4) + 2 * k, out_desc, (c | k) > 0);
             tc_commit(o_full);
             p0 = p1;
         }

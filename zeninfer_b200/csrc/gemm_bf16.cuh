@@ -40,16 +40,6 @@ __host__ __device__ constexpr uint32_t gemm_bf16_stage_bytes() { return kBgAByte
 template <int kNTile>
 __host__ __device__ constexpr uint32_t gemm_bf16_smem_bytes() { return 1024 + gemm_bf16_stages<kNTile>() * gemm_bf16_stage_bytes<kNTile>() + 256; }
 
-// Instruction descriptor, kind::f16: bf16 x bf16 -> fp32, both operands K-major, dense.
-__host__ __device__ constexpr uint32_t umma_idesc_bf16(uint32_t m, uint32_t n) {
-    return (1u << 4) | (1u << 7) | (1u << 10) | ((n >> 3) << 17) | ((m >> 4) << 24);
-}
-__device__ __forceinline__ void tc_mma_f16(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc, uint32_t accumulate) {
-    asm volatile(
-        "{ .reg .pred p; setp.ne.b32 p, %4, 0; tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p; }"
-        ::"r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate) : "memory");
-}
-
 template <int kNTile>
 __global__ void __launch_bounds__(kBgThreads, 1) gemm_bf16_kernel(const __grid_constant__ GemmBf16Params p) {
     constexpr int kStages = gemm_bf16_stages<kNTile>();
