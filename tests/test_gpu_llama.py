@@ -379,6 +379,15 @@ def test_attention_prefill_tiles(be, H, KH, T, pos0, window):
     test_attention_prefill_block(be, H, KH, 128, T, pos0, window)
 
 
+# Few keys go without the tensor cores: one key, the last number of keys and one more, by how many rows a warp then has (one; two, with
+# half the keys) and over several CTAs per tile or one; windows that leave few keys late in a sequence; the limits on tokens and tiles.
+@pytest.mark.parametrize("H,KH,T,pos0,window", [(4, 1, 1, 0, 0), (4, 1, 32, 96, 0), (4, 1, 32, 97, 0), (32, 32, 16, 0, 0), (32, 32, 16, 112, 0), (32, 32, 17, 47, 0), (32, 32, 17, 48, 0),
+                                                (1, 1, 128, 0, 0), (1, 1, 129, 0, 0), (8, 8, 40, 200, 20), (8, 1, 16, 230, 7), (4, 4, 100, 60, 29), (48, 24, 5, 3, 0), (50, 25, 33, 0, 0),
+                                                (128, 1, 2, 120, 3), (8, 8, 7, 0, 0)])
+def test_attention_prefill_of_few_keys(be, H, KH, T, pos0, window):
+    test_attention_prefill_block(be, H, KH, 128, T, pos0, window)
+
+
 def test_attention_prefill_precision_and_infinite_keys(be):
     # scores of widely different sizes, values up to 1e6 beside small ones; a key whose score is minus infinity has no weight
     import torch

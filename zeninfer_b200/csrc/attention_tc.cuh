@@ -2,8 +2,8 @@
 // other sizes, and the arithmetic's references).
 //
 // fp32 throughout, by splitting: a float is the exact sum of three bfloat16 values (its 24 mantissa bits, eight at a time, by
-// truncation), so a product of two floats is six products of bfloat16 values (the three left out are below 2^-23 of it), each exact
-// in the fp32 accumulator.  Six bf16 products run at 270 TFLOP/s where fp32 multiply-adds run at 70, and they leave the issue slots
+// truncation), so a product of two floats is six products of bfloat16 values (the three left out are below 2^-21 of it together, and of its
+// sign), each exact in the fp32 accumulator.  Six bf16 products run at 270 TFLOP/s where fp32 multiply-adds run at 70, and they leave the issue slots
 // to the softmax, which with the fp32 form waits behind them.
 //
 // A CTA takes 128 rows: 128 / group consecutive tokens times the query heads of one KV head, so that keys and values serve the whole
@@ -23,17 +23,22 @@
 // rows of the tile that do not attend it.
 //
 // What bounds it: a block's chain through the row warps, about 6 us a block of 64 keys, of which the exponentials are a third; the
-// tensor pipe (72 products a block) is busy for a third of that, memory hardly at all.  B200, 512 tokens, 32 heads on 8, at position 0 / 1488: 54 / 190 us, with fp32
-// multiply-adds on the CUDA cores 142 / 551; error against 64 bits (2-norm, unit normal inputs) 2.0e-7 / 2.9e-7, before 2.1e-7 /
-// 7.5e-7.  Five tokens at position 0 / 1500: 9.7 / 96 us, before 6.7 / 301; the host does not know the position, so all sizes go here.
+// tensor pipe (72 products a block) is busy for a third of that, memory hardly at all.  The row warps have 128 registers, of which 64 hold
+// the output and 32 the scores: 160 bytes a thread are spilled (244 with windows).  B200, 512 tokens, 32 heads on 8, at position 0 /
+// 1488: 54 / 190 us, with fp32 multiply-adds on the CUDA cores 142 / 551; error against 64 bits (2-norm, unit normal inputs) 2.0e-7 /
+// 2.9e-7, before 2.1e-7 / 7.5e-7.  Five tokens at position 1500: 95 us, before 301.  The host does not know the position: all sizes of
+// these heads come here, and a tile of few keys leaves the tensor cores aside (attention_tc_few).
 #pragma once
 #include <cuda_bf16.h>
+
+#include <algorithm>
 
 #include "attention.cuh"
 
 namespace zk {
 
 constexpr uint32_t kTcRows = 128, kTcKeys = 64, kTcDim = 128;
+constexpr uint32_t kTcFewKeys = 128, kTcFewCtas = 24;
 constexpr uint32_t kTcKeyWarp = 8, kTcValueWarp = 12, kTcIssueWarp = 15, kTcThreads = 16 * 32;       // first warps of the roles
 constexpr uint32_t kTcQPlane = kTcRows * kTcDim * 2, kTcKPlane = kTcKeys * kTcDim * 2, kTcVPlane = kTcDim * kTcKeys * 2;
 constexpr uint32_t kTcSmem = 1024 + 3 * (kTcQPlane + kTcKPlane + kTcVPlane) + 4 * kTcRows * 4 + 2 * kTcRows * 8 + 128;
@@ -85,7 +90,28 @@ inline size_t attention_tc_ctas(size_t head_dim, size_t tokens, size_t heads, si
     return (tokens + tile_tokens - 1) / tile_tokens * kv_heads;
 }
 
-// Arguments as attention_prefill_kernel's.  heads / kv_heads divides 128; grid: token tiles x kv_heads, the last tokens' tiles first.
+// Whether a tile of so many rows and keys, in `parts` CTAs, goes without the tensor cores: a warp then takes a row at a time, about 0.7 us
+// for eight keys while a CTA has eight rows at most, twice that with sixteen (its loads queue); the tensor cores take 9 us for the
+// first block of 64 keys and 4 for the next, whatever the rows.  B200, us, few keys / tensor cores / the fp32 kernel for other heads:
+// 5 tokens at position 0, 32 heads on 8: 6.0 / 9.7 / 6.2; 33 tokens at 0 / 80: 6.0 / 13.1 / 9.9 and 16.0 / 17.6 / 26.3; 16 tokens of 32
+// heads on 32 (sixteen rows a CTA) at 0 / 40 / 100: 4.4 / 10.0 / 5.1, 9.8 / 10.4 / 12.2 and 17.8 / 14.7 / 23.5.
+__host__ __device__ inline bool attention_tc_few(uint32_t rows, uint32_t keys, uint32_t parts) {
+    const uint32_t turns = (rows + 8 * parts - 1) / (8 * parts);               // of eight warps
+    return turns <= 2 ? keys <= kTcFewKeys / 4 * (5 - turns) : static_cast<uint64_t>(keys) * turns <= kTcFewKeys;
+}
+
+// CTAs per tile (the grid's y): more than one where the last tile may have few keys, as many as leave a CTA four rows, on SMs that
+// would have no tile.  Where such a call then takes the tensor cores, the CTAs that leave at once cost it 0.3 to 0.6 us (12 to 25 us
+// calls); with 32 tiles and four parts, calls back to back took 90 us instead of 70 (16 tokens at 1000), so beyond 24 tiles there are none.
+inline unsigned attention_tc_parts(size_t ctas, size_t tokens, size_t heads, size_t kv_heads, int sms) {
+    if (tokens > kTcFewKeys || ctas > kTcFewCtas) return 1;
+    const uint32_t rows = static_cast<uint32_t>(std::min<size_t>(kTcRows, tokens * (heads / kv_heads)));
+    const uint32_t parts = std::min((rows + 3) / 4, static_cast<uint32_t>(sms / ctas));
+    return parts > 1 && attention_tc_few(rows, static_cast<uint32_t>(tokens), parts) ? parts : 1;
+}
+
+// Arguments as attention_prefill_kernel's.  heads / kv_heads divides 128; grid: token tiles x kv_heads, the last tokens' tiles first,
+// times attention_tc_parts.
 template <bool kWindowed>
 __global__ void __launch_bounds__(kTcThreads, 1) attention_prefill_tc_kernel(const float* __restrict__ q, const float* __restrict__ k_cache,
                                                                               const float* __restrict__ v_cache, const int* __restrict__ pos_ptr,
@@ -112,25 +138,28 @@ __global__ void __launch_bounds__(kTcThreads, 1) attention_prefill_tc_kernel(con
         mbar_init(s_full, 1); mbar_init(s_empty, 8); mbar_init(p_full, 8); mbar_init(o_full, 1); mbar_init(o_empty, 8);
         mbar_fence_init();
     }
-    if (warp == kTcIssueWarp) tmem_alloc(tmem_slot, kTcColumns);
+    if (warp == kTcIssueWarp && blockIdx.y == 0) tmem_alloc(tmem_slot, kTcColumns);
+    const uint32_t group = heads / kv_heads, tile_tokens = kTcRows / group, kw = kv_heads * kTcDim, qw = heads * kTcDim;
+    const uint32_t n_tiles = gridDim.x / kv_heads, tile = n_tiles - 1 - blockIdx.x / kv_heads, kh = blockIdx.x % kv_heads;
+    const uint32_t t0 = tile * tile_tokens, t_end = min(tokens, t0 + tile_tokens);
+    const uint32_t live_rows = (t_end - t0) * group, each = (live_rows + gridDim.y * (kTcThreads / 32) - 1) / (gridDim.y * (kTcThreads / 32));
     pdl_launch_dependents();
     pdl_wait();
     const int pos0 = __ldcg(pos_ptr);
     const bool good = pos0 >= 0 && static_cast<uint64_t>(pos0) + tokens <= max_positions;
-    if (!good && threadIdx.x == 0 && blockIdx.x == 0) atomicExch(error_word, kErrBadPosition);
+    if (!good && threadIdx.x == 0 && blockIdx.x == 0 && blockIdx.y == 0) atomicExch(error_word, kErrBadPosition);
 
-    const uint32_t group = heads / kv_heads, tile_tokens = kTcRows / group, kw = kv_heads * kTcDim, qw = heads * kTcDim;
-    const uint32_t n_tiles = gridDim.x / kv_heads, tile = n_tiles - 1 - blockIdx.x / kv_heads, kh = blockIdx.x % kv_heads;
-    const uint32_t t0 = tile * tile_tokens, t_end = min(tokens, t0 + tile_tokens);
     const uint32_t last_pos = static_cast<uint32_t>(pos0) + t_end - 1;
     const uint32_t first_any = (window && static_cast<uint32_t>(pos0) + t0 + 1 > window) ? static_cast<uint32_t>(pos0) + t0 + 1 - window : 0u;
     const uint32_t kept_end = kWindowed ? min(win.keep_first, first_any) : 0u;      // kept tokens the window of the tile's first token has left behind
     const uint32_t start = kWindowed && kept_end ? 0u : first_any;
+    const bool few = good && attention_tc_few(live_rows, last_pos + 1 - first_any + kept_end, gridDim.y);
+    if (blockIdx.y && !few) return;
     auto next_block = [&](uint32_t p0) { return kWindowed && p0 < kept_end && p0 + kTcKeys >= kept_end ? first_any : p0 + kTcKeys; };
     auto part_last = [&](uint32_t p0) { return kWindowed && p0 < kept_end ? kept_end - 1 : last_pos; };      // last position of the part a block lies in
     auto gave_up = [&](int code) { if (lane == 0) atomicExch(error_word, code); };
 
-    if (good) {                                               // Q in three planes, all threads; rows past the block are zeros
+    if (good && !few) {                                       // Q in three planes, all threads; rows past the block are zeros
         for (uint32_t i = threadIdx.x; i < kTcRows * (kTcDim / 8); i += kTcThreads) {
             const uint32_t row = i / (kTcDim / 8), chunk = i % (kTcDim / 8), t = t0 + row / group;
             float x[8] = {};
@@ -150,11 +179,14 @@ __global__ void __launch_bounds__(kTcThreads, 1) attention_prefill_tc_kernel(con
     tc_fence_before_sync();
     __syncthreads();
     tc_fence_after_sync();
-    const uint32_t tmem = *tmem_slot;
+    const uint32_t tmem = *tmem_slot;                         // (parts other than the first have none and use none)
 
     uint32_t todo = 0, first_row = 0, lanes_of = 2;           // rows left to this warp below: bits from first_row on; half of the head it stores (2: both)
     // A wait that runs out ends its role's loop, and the others' follow.
     if (!good) {
+    } else if (few) {                                         // fp32 multiply-adds alone, the warps of all parts
+        first_row = (warp * gridDim.y + blockIdx.y) * each;
+        if (first_row < live_rows) todo = (1u << min(each, live_rows - first_row)) - 1u;
     } else if (warp < kTcKeyWarp) {                           // rows
         const uint32_t quad = warp & 3, half = warp >> 2, row = quad * 32 + lane, lane_base = (quad * 32) << 16;
         const uint32_t t = t0 + row / group, h = kh * group + row % group;
@@ -286,10 +318,10 @@ __global__ void __launch_bounds__(kTcThreads, 1) attention_prefill_tc_kernel(con
                 atomicExch(error_word, kErrNonFinite);
             } else {
                 const float inv = 1.0f / static_cast<float>(l);
-                float nonfinite = 0.0f;
+                float nonfinite[4] = {};
 #pragma unroll
-                for (int i = 0; i < static_cast<int>(kTcDim / 2); ++i) { acc[i] *= inv; nonfinite = fmaf(acc[i], 0.0f, nonfinite); }
-                again = nonfinite != 0.0f;
+                for (int i = 0; i < static_cast<int>(kTcDim / 2); ++i) { acc[i] *= inv; nonfinite[i & 3] = fmaf(acc[i], 0.0f, nonfinite[i & 3]); }
+                again = (nonfinite[0] + nonfinite[1]) + (nonfinite[2] + nonfinite[3]) != 0.0f;
                 float4* dst = reinterpret_cast<float4*>(out + static_cast<size_t>(t) * qw + static_cast<size_t>(h) * kTcDim + half * (kTcDim / 2));
 #pragma unroll
                 for (int i = 0; i < static_cast<int>(kTcDim / 8); ++i)
@@ -414,94 +446,84 @@ __global__ void __launch_bounds__(kTcThreads, 1) attention_prefill_tc_kernel(con
         if (!ok) atomicExch(error_word, kErrFullWaitTimeout);
     }
     __syncwarp();
-    // Rows again with fp32 multiply-adds, four at a time and four keys a round, a lane holding four columns: those with an output that is
-    // not finite.  The products above multiply every value of a block, by zero where a row does not attend it, and a value's lower
-    // planes are NaN where it is infinite; here a row meets the values it attends and no others, each as it is.
-    while (todo) {
-        uint32_t rows[4], mine = 0;
-        float4 x[4], o[4];
-#pragma unroll
-        for (uint32_t r = 0; r < 4; ++r) {                    // fewer rows than four: the last one several times
-            rows[r] = todo ? first_row + __ffs(todo) - 1 : rows[r - (r > 0)];
-            todo &= todo - 1u;                                // 0 stays 0
-            if (lane >> 3 == r) mine = rows[r];
+    // Rows with fp32 multiply-adds, one after another, eight keys a round, a lane holding four columns.  Few keys: all rows, since a block's
+    // chain above costs more than they do.  Otherwise those with an output that is not finite: the products above multiply every value of
+    // a block, by zero where a row does not attend it, and a value's lower planes are NaN where it is infinite; here a row meets the
+    // values it attends and no others, each as it is.
+    for (; todo; todo &= todo - 1u) {
+        const uint32_t row = first_row + __ffs(todo) - 1, t = t0 + row / group, h = kh * group + row % group;
+        const uint32_t my_last = static_cast<uint32_t>(pos0) + t, my_first = (window && my_last + 1 > window) ? my_last + 1 - window : 0u;
+        const size_t at_row = static_cast<size_t>(t) * qw + static_cast<size_t>(h) * kTcDim + lane * 4;
+        float4 x, o = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (few) {
+            x = __ldcg(reinterpret_cast<const float4*>(q + at_row));
+        } else {                                              // out may lie over q: from the planes, exactly, the smallest first
+            const uint32_t at = (lane / 16) * (kTcQPlane / 2) + row * 128 + (((lane % 16 / 2) ^ (row & 7)) << 4) + (lane & 1) * 8;
             uint2 plane[3];
-            const uint32_t at = (lane / 16) * (kTcQPlane / 2) + rows[r] * 128 + (((lane % 16 / 2) ^ (rows[r] & 7)) << 4) + (lane & 1) * 8;
 #pragma unroll
             for (int p = 0; p < 3; ++p) plane[p] = *reinterpret_cast<const uint2*>(q_smem + p * kTcQPlane + at);
-            auto sum3 = [&](auto part) { return part(plane[0]) + (part(plane[1]) + part(plane[2])); };     // exact, smallest first
-            x[r] = make_float4(sum3([](uint2 w) { return __uint_as_float(w.x << 16); }), sum3([](uint2 w) { return __uint_as_float(w.x & 0xffff0000u); }),
-                               sum3([](uint2 w) { return __uint_as_float(w.y << 16); }), sum3([](uint2 w) { return __uint_as_float(w.y & 0xffff0000u); }));
-            o[r] = make_float4(0.f, 0.f, 0.f, 0.f);
+            auto sum3 = [&](auto part) { return part(plane[0]) + (part(plane[1]) + part(plane[2])); };
+            x = make_float4(sum3([](uint2 w) { return __uint_as_float(w.x << 16); }), sum3([](uint2 w) { return __uint_as_float(w.x & 0xffff0000u); }),
+                            sum3([](uint2 w) { return __uint_as_float(w.y << 16); }), sum3([](uint2 w) { return __uint_as_float(w.y & 0xffff0000u); }));
         }
-        // a lane keeps the state of row lane / 8 and the score of key lane / 2 % 4
-        const uint32_t t = t0 + mine / group, my_last = static_cast<uint32_t>(pos0) + t, end = static_cast<uint32_t>(pos0) + t0 + rows[3] / group;
-        const uint32_t my_first = (window && my_last + 1 > window) ? my_last + 1 - window : 0u;
-        const float slope = kWindowed && win.biased ? attn_slope(kh * group + mine % group, heads) : 0.0f;
+        const float slope = kWindowed && win.biased ? attn_slope(h, heads) : 0.0f;
         const size_t column = static_cast<size_t>(kh) * kTcDim + lane * 4;
+        constexpr uint32_t kRound = 8;                        // a lane keeps key lane / 4 of a round
         float m = -INFINITY;
         double l = 0.0;
-        for (uint32_t p0 = start; p0 <= end; p0 = kWindowed && p0 < kept_end && p0 + 4 >= kept_end ? first_any : p0 + 4) {
-            const uint32_t last = part_last(p0), pos = p0 + lane / 2 % 4;
+        for (uint32_t p0 = start; p0 <= my_last; p0 = kWindowed && p0 < kept_end && p0 + kRound >= kept_end ? first_any : p0 + kRound) {
+            const uint32_t last = part_last(p0), pos = p0 + lane / 4;
             const bool attended = pos <= min(my_last, last) && (pos >= my_first || (kWindowed && pos < win.keep_first));
             if (!__any_sync(0xffffffffu, attended)) continue;
-            float4 key[4], value[4];
+            float4 key[kRound], value[kRound];
 #pragma unroll
-            for (uint32_t k = 0; k < 4; ++k) {
+            for (uint32_t k = 0; k < kRound; ++k) {
                 const size_t off = static_cast<size_t>(min(p0 + k, last)) * kw + column;
                 key[k] = __ldca(reinterpret_cast<const float4*>(k_cache + off));
                 value[k] = __ldca(reinterpret_cast<const float4*>(v_cache + off));
             }
-            float s[16];                                      // summed over the lanes, which at each exchange keep half of the sums they carry
+            float s[kRound];                                  // summed over the lanes, which at each exchange keep half of the sums they carry
 #pragma unroll
-            for (int i = 0; i < 16; ++i) s[i] = fmaf(x[i / 4].w, key[i % 4].w, fmaf(x[i / 4].z, key[i % 4].z, fmaf(x[i / 4].y, key[i % 4].y, x[i / 4].x * key[i % 4].x)));
+            for (uint32_t k = 0; k < kRound; ++k) s[k] = fmaf(x.w, key[k].w, fmaf(x.z, key[k].z, fmaf(x.y, key[k].y, x.x * key[k].x)));
 #pragma unroll
-            for (int h = 8; h > 0; h >>= 1) {
-                const bool up = lane & (2 * h);
+            for (int n = kRound / 2; n > 0; n >>= 1) {
+                const bool up = lane & (4 * n);
 #pragma unroll
-                for (int i = 0; i < h; ++i) s[i] = (up ? s[i + h] : s[i]) + __shfl_xor_sync(0xffffffffu, up ? s[i] : s[i + h], 2 * h);
+                for (int i = 0; i < n; ++i) s[i] = (up ? s[i + n] : s[i]) + __shfl_xor_sync(0xffffffffu, up ? s[i] : s[i + n], 4 * n);
             }
-            float score = (s[0] + __shfl_xor_sync(0xffffffffu, s[0], 1)) * scale;
+            float score = s[0] + __shfl_xor_sync(0xffffffffu, s[0], 2);
+            score = (score + __shfl_xor_sync(0xffffffffu, score, 1)) * scale;
             if (kWindowed) score -= slope * static_cast<float>(static_cast<int>(my_last) - static_cast<int>(pos));
             float most = attended ? fmaxf(m, score) : m;
-            most = fmaxf(most, __shfl_xor_sync(0xffffffffu, most, 2));
-            most = fmaxf(most, __shfl_xor_sync(0xffffffffu, most, 4));
-            const bool moved = most > m;
-            if (__any_sync(0xffffffffu, moved)) {
-                const float f = moved ? expf(m - most) : 1.0f;
+#pragma unroll
+            for (int n = 4; n < 32; n *= 2) most = fmaxf(most, __shfl_xor_sync(0xffffffffu, most, n));
+            if (most > m) {
+                const float f = expf(m - most);               // exp(-inf) = 0 on the first position
                 l *= f;
                 m = most;
-#pragma unroll
-                for (int r = 0; r < 4; ++r) {
-                    const float fr = __shfl_sync(0xffffffffu, f, 8 * r);
-                    o[r].x *= fr; o[r].y *= fr; o[r].z *= fr; o[r].w *= fr;
-                }
+                o.x *= f; o.y *= f; o.z *= f; o.w *= f;
             }
             const float e = attended ? expf(score - (m == -INFINITY ? 0.0f : m)) : -1.0f;      // below zero: not attended
             if (attended) l += e;
 #pragma unroll
-            for (int i = 0; i < 16; ++i) {
-                const float p = __shfl_sync(0xffffffffu, e, 2 * i);
+            for (uint32_t k = 0; k < kRound; ++k) {
+                const float p = __shfl_sync(0xffffffffu, e, 4 * k);
                 if (p < 0.0f) continue;
-                float4& to = o[i / 4];
-                const float4& v = value[i % 4];
-                to.x = fmaf(p, v.x, to.x); to.y = fmaf(p, v.y, to.y); to.z = fmaf(p, v.z, to.z); to.w = fmaf(p, v.w, to.w);
+                o.x = fmaf(p, value[k].x, o.x); o.y = fmaf(p, value[k].y, o.y); o.z = fmaf(p, value[k].z, o.z); o.w = fmaf(p, value[k].w, o.w);
             }
         }
-        l += __shfl_xor_sync(0xffffffffu, l, 2);
-        l += __shfl_xor_sync(0xffffffffu, l, 4);
-        const float inv = 1.0f / static_cast<float>(l);
 #pragma unroll
-        for (int r = 0; r < 4; ++r) {
-            const float to = __shfl_sync(0xffffffffu, inv, 8 * r);
-            if (lanes_of < 2 && lane / 16 != lanes_of) continue;
-            *reinterpret_cast<float4*>(out + static_cast<size_t>(t0 + rows[r] / group) * qw + static_cast<size_t>(kh * group + rows[r] % group) * kTcDim + lane * 4) =
-                make_float4(o[r].x * to, o[r].y * to, o[r].z * to, o[r].w * to);
+        for (int n = 4; n < 32; n *= 2) l += __shfl_xor_sync(0xffffffffu, l, n);
+        if (!(l > 0.0) || !isfinite(l)) {
+            atomicExch(error_word, kErrNonFinite);
+        } else if (lanes_of > 1 || lane / 16 == lanes_of) {
+            const float inv = 1.0f / static_cast<float>(l);
+            *reinterpret_cast<float4*>(out + at_row) = make_float4(o.x * inv, o.y * inv, o.z * inv, o.w * inv);
         }
     }
     tc_fence_before_sync();
     __syncthreads();
-    if (warp == kTcIssueWarp) {
+    if (warp == kTcIssueWarp && blockIdx.y == 0) {
         tc_fence_after_sync();
         tmem_dealloc(tmem, kTcColumns);
     }

@@ -2577,9 +2577,10 @@ int zen_cuda_dev_attention_prefill(const float* d_q, const float* d_k_cache, con
             ZC_CUDA(s, cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(zk::kTcSmem)));
             opted_in = true;
         }
-        ZC_DEV_LEAVE(launch_pdl(s, kernel, dim3(static_cast<unsigned>(ctas)), dim3(zk::kTcThreads), zk::kTcSmem, st, d_q, d_k_cache, d_v_cache, d_pos, d_out,
-                                static_cast<uint32_t>(tokens), static_cast<uint32_t>(heads), static_cast<uint32_t>(kv_heads), scale, static_cast<uint32_t>(window),
-                                static_cast<uint32_t>(max_positions), s.d_error, zk::AttnWindow{}));
+        const dim3 grid(static_cast<unsigned>(ctas), zk::attention_tc_parts(ctas, tokens, heads, kv_heads, s.sm_count));
+        ZC_DEV_LEAVE(launch_pdl(s, kernel, grid, dim3(zk::kTcThreads), zk::kTcSmem, st, d_q, d_k_cache, d_v_cache, d_pos, d_out, static_cast<uint32_t>(tokens),
+                                static_cast<uint32_t>(heads), static_cast<uint32_t>(kv_heads), scale, static_cast<uint32_t>(window), static_cast<uint32_t>(max_positions),
+                                s.d_error, zk::AttnWindow{}));
     }
     // query heads per thread: the largest of 4, 2, 1 that divides the group and keeps 2 * R * head_dim / 8 row values in registers
     const size_t group = heads / kv_heads;

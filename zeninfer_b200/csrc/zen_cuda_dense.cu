@@ -303,7 +303,8 @@ int zen_cuda_dev_window_attention_rows(const zen_cuda_window_attention* a, const
     }
     if (const size_t tiles = zk::attention_tc_ctas(a->pitch, tokens, a->heads, a->kv_heads)) {
         if (tiles > 0x7fffffffu) return e.fail("window_attention_rows: too many tiles");
-        r = launch(e, zk::attention_prefill_tc_kernel<true>, dim3(u32(tiles)), dim3(zk::kTcThreads), zk::kTcSmem, static_cast<const float*>(d_q),
+        const dim3 grid(u32(tiles), zk::attention_tc_parts(tiles, tokens, a->heads, a->kv_heads, e.sm_count));
+        r = launch(e, zk::attention_prefill_tc_kernel<true>, grid, dim3(zk::kTcThreads), zk::kTcSmem, static_cast<const float*>(d_q),
                    static_cast<const float*>(a->k_cache), static_cast<const float*>(a->v_cache), d_pos, d_out, u32(tokens), a->heads, a->kv_heads, a->scale, a->window,
                    a->max_positions, e.d_error, win);
         return e.leave(r, "window_attention_rows");
