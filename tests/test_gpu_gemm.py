@@ -271,6 +271,37 @@ def test_group_scale_tiles_split_between_two_ctas(tokens):
     assert np.abs(got.astype(np.float64) - want).max() <= 2e-6 * np.abs(want).max()
 
 
+# Split tiles of several token tiles: 96 columns (149 row tiles, 180 tokens) and 128 (40 row tiles, 500 tokens).
+@pytest.mark.parametrize("tokens,rows,cols", [(180, 19072, 512), (500, 5120, 512)])
+def test_group_scale_split_tiles_of_several_token_tiles(tokens, rows, cols):
+    check_split_products(tokens, [rows], cols)
+
+
+def test_group_scale_second_launch_with_split_tiles():
+    # four tensors: the first three are one launch, whose split tiles are cleared beside the digits, the fourth another behind a
+    # launch that clears its own
+    check_split_products(30, [12800, 3190, 3200, 19072], 512)
+
+
+def check_split_products(tokens, rows, cols):
+    import torch
+    from helpers import group_product
+    from zeninfer_b200 import Backend
+    be = Backend()
+    ws, x = [seeded_weights(Q8_0, r, cols, 741 + i) for i, r in enumerate(rows)], seeded_acts(tokens, cols, 740)
+    handles = [be.dev_upload("Q8_0", w, r, cols) for w, r in zip(ws, rows)]
+    nbytes = be.gemm_workspace_bytes(tokens, cols, ACT_FP32)
+    scratch, d_x = torch.zeros(nbytes, dtype=torch.uint8, device="cuda"), torch.from_numpy(x).cuda()
+    outs = [torch.full((tokens, r), float("nan"), device="cuda") for r in rows]
+    torch.cuda.synchronize()
+    be.dev_gemm_q8_0(handles, [o.data_ptr() for o in outs], d_x.data_ptr(), tokens, scratch.data_ptr(), nbytes, act_mode=ACT_FP32)
+    be.dev_check()
+    for h, w, o, r in zip(handles, ws, outs, rows):
+        be.dev_free(h)
+        want = group_product(blocks.dequantize(Q8_0, w, r, cols), x)
+        assert np.abs(o.cpu().numpy().astype(np.float64) - want).max() <= 2e-6 * np.abs(want).max()     # two partial sums: two roundings
+
+
 def test_group_scale_product_in_place():
     # the output over the activations, 160 tiles (most of them split and cleared first): cleared only once the digits are formed, in a
     # launch of its own

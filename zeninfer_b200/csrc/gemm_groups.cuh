@@ -32,11 +32,11 @@
 // weight rows, N = kN tokens, K = 32; accumulator sets alternate between the two halves of TMEM.  Then 4 kN / 32 epilogue warps,
 // thread = weight row = TMEM lane, 32 token columns per warp.
 //
-// What bounds the kernel are the operand bytes that pass through an SM's shared memory, 256 (128 + kN) per 128 columns of K and
-// tile; a tile of few tokens brings its 32 KB of weights and little else.  So the tile's width (32, 64, 96 or 128 tokens) is the one
-// with the fewest bytes through the busiest SM (gg_tile_columns); with tiles of 128 only, eight tokens cost what 128 do.
-// B200, with the two launches in front merged into one and overlapped: 128256 x 4096 times 8 tokens 271 -> 176 us, 11008 x 4096
-// times 77 40.3 -> 37.1, 14336 x 4096 times 512 116.8 -> 114.8.
+// What bounds the kernel is the time of a ring step: the operand bytes that pass through an SM's shared memory, 256 (128 + kN) per 128
+// columns of K and tile, and a part that does not depend on the width; a tile of few tokens brings its 32 KB of weights and little
+// else.  The tile's width (32, 64, 96 or 128 tokens) is chosen for the busiest SM (gg_tile_columns).  B200, us, with tiles of 128 and
+// the digits, their padding, the clearing and the product as launches of their own / now: 128256 x 4096 times 8 tokens 287 / 164,
+// 11008 x 4096 times 77 41.1 / 29.4, 14336 x 4096 times 512 100.1 / 93.4.
 #pragma once
 #include <cuda.h>
 #include <cuda_fp16.h>
@@ -74,15 +74,21 @@ struct GroupGemmParams {
 
 template <int kN> __host__ __device__ constexpr size_t gemm_groups_smem_bytes() { return 1024 + static_cast<size_t>(gg_stages<kN>()) * gg_stage_bytes<kN>() + 256; }
 
-// The tile's columns: fewest operand bytes through the busiest SM.  Tiles beyond the SMs are shared out evenly (stream-K), fewer
-// run side by side.
-inline uint32_t gg_tile_columns(uint32_t m_tiles, uint32_t tokens, uint32_t sms) {
+// The tile's columns, by the time of the busiest SM in units of a group of one tile: 240 + n (a step of the ring has its own time, and
+// brings 32 KB of weights whatever n is).  Up to one tile per SM a CTA has one tile.  More are shared out evenly (stream-K), which
+// costs the split tiles' clearing and atomic additions and the CTAs' common walk over the weights: three groups and a fifth of K.  Fitted to 409 measured shapes of 1024 to 28672 rows, 1024 to 14336 columns and 16 to 700 tokens, each with all four widths: the
+// width it picks is 0.3 % slower than the best one on average (at 1024 columns up to 15 %), at most 1.1 % slower than tiles of 128.
+// Counting operand bytes alone took splits where whole tiles fit: 6400 x 14336 times 77 tokens in tiles of 32 / 64 / 128: 93.7 /
+// 77.6 / 84.7 us; 11008 x 4096 times 77 in tiles of 64 / 96 / 128: 35.1 / 29.4 / 32.8; 4096 x 4096 times 300: 33.1 / 30.8 / 33.6.
+inline uint32_t gg_tile_columns(uint32_t m_tiles, uint32_t tokens, uint32_t groups, uint32_t sms) {
     uint32_t best = kGgNTile;
     double best_cost = 0.0;
     for (uint32_t n : {128u, 96u, 64u, 32u}) {
         const uint32_t n_tiles = (tokens + n - 1) / n;
         if (n_tiles * n > (tokens + kGgNTile - 1) / kGgNTile * kGgNTile) continue;      // the unit plane ends there
-        const double cost = std::max(1.0, static_cast<double>(m_tiles) * n_tiles / sms) * (kGemmM + n);
+        const uint64_t tiles = static_cast<uint64_t>(m_tiles) * n_tiles;
+        const bool split = tiles > sms && tiles % sms;
+        const double cost = (std::max(1.0, static_cast<double>(tiles) / sms) * groups + (split ? 3.0 + 0.2 * groups : 0.0)) * (240 + n);
         if (best_cost == 0.0 || cost < best_cost) { best_cost = cost; best = n; }
     }
     return best;

@@ -1038,7 +1038,7 @@ bool enqueue_gemm_groups(State& s, const zen_cuda_weights* const* w, float* cons
             p.m_start[j] = m_tiles;
             m_tiles += (p.rows[j] + zk::kGemmM - 1) / zk::kGemmM;
         }
-        const uint32_t columns = zk::gg_tile_columns(m_tiles, static_cast<uint32_t>(tokens), static_cast<uint32_t>(s.sm_count));
+        const uint32_t columns = zk::gg_tile_columns(m_tiles, static_cast<uint32_t>(tokens), groups, static_cast<uint32_t>(s.sm_count));
         if (!make_map_2d(s, &p.map_xh, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, xh, cols, tokens, cols, zk::kGemmKTile, columns, CU_TENSOR_MAP_SWIZZLE_128B)) return false;
         if (!make_map_2d(s, &p.map_xl, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, xl, cols, tokens, cols, zk::kGemmKTile, columns, CU_TENSOR_MAP_SWIZZLE_128B)) return false;
         p.x_unit = x_unit;
