@@ -497,6 +497,15 @@ def test_generate(be, name):
     dec.close()
 
 
+def test_a_callback_sees_the_tokens_of_a_run_without_one(be):
+    c, _, dec = decoder(be, "ragged", chunk=32)
+    prompt = cases.tokens_for(c, 41, 3)
+    for options in ({}, dict(temperature=1.2, top_k=30, seed=2)):
+        seen = []
+        assert dec.generate(prompt, 24, on_token=seen.append, **options) == seen == dec.generate(prompt, 24, **options)
+    dec.close()
+
+
 def test_missing_and_misshapen_tensors_are_refused(be):
     c, cfg, bits, _ = cases.model("last_bare")
     with pytest.raises(KeyError):

@@ -209,6 +209,25 @@ def test_int8_activation_mode_is_deterministic(be, golden):
         dec.close()
 
 
+def test_a_callback_sees_the_tokens_of_a_run_without_one(be, golden):
+    # with a callback the host feeds each token back, without one the next step is launched before the token is read
+    cfg, meta, prompt, _, _ = golden
+    dec = LlamaDecoder(be, cfg, synthetic_tensors(cfg, meta["seed"], meta["weight_std"]), act_mode=ACT_INT8)
+    try:
+        for captured in (False, True):
+            if captured:
+                dec.capture()
+            for options in ({}, dict(temperature=0.9, top_k=40, top_p=0.95, seed=5)):
+                seen = []
+                fed = dec.generate(prompt.tolist(), 12, on_token=seen.append, **options)
+                logits = dec.last_logits()
+                assert fed == seen == dec.generate(prompt.tolist(), 12, **options)
+                assert np.array_equal(logits, dec.last_logits())
+        assert dec.generate(prompt.tolist(), 0) == []
+    finally:
+        dec.close()
+
+
 def test_context_overflow_is_an_error(be, golden):
     cfg, meta, prompt, _, _ = golden
     dec = LlamaDecoder(be, cfg, synthetic_tensors(cfg, meta["seed"], meta["weight_std"]), max_positions=16)
