@@ -50,6 +50,12 @@ def test_dense_gemv_of_uneven_units(be, rows, cols):
     test_dense_gemv(be, rows, cols, DENSE_PLAIN)
 
 
+# Inputs that leave room for a ring of three steps, of two, and for none (a row's sums are over as many fp32 products).
+@pytest.mark.parametrize("cols", [33000, 33100, 40000, 42000, 50000])
+def test_dense_gemv_of_long_inputs(be, cols):
+    test_dense_gemv(be, 300, cols, DENSE_PLAIN)
+
+
 def test_dense_gemv_several_tasks(be):
     shapes = [(70, 40), (333, 1100), (5, 256), (201, 8)]
     mats = [bf16_matrix(be, r, c, i) for i, (r, c) in enumerate(shapes)]
@@ -147,6 +153,33 @@ def test_sublayer_end(be, n, T, groups, two, view):
         close(host(x_out), x)
         assert np.array_equal(host(keep), a["x"][-1])
         be.dev_free(h)
+
+
+# A decode product's prologue with the row in registers (a multiple of 32 values, at most 4096, in 1, 2, 4 or 8 parts) and beside that range.
+@pytest.mark.parametrize("n,groups", [(32, 1), (96, 8), (1024, 4), (1056, 2), (2048, 4), (2080, 1), (4064, 1), (4096, 8), (4096, 16), (2056, 4), (4128, 1)])
+@pytest.mark.parametrize("two", [False, True])
+@pytest.mark.parametrize("view", ["plain", "shift", "norm"])
+def test_sublayer_end_in_a_product(be, n, groups, two, view):
+    a, d, end, x_out, keep, x, seen = sublayer_case(n, 1, groups, two, view, seed=n)
+    h, w = bf16_matrix(be, 300, n, 9)
+    y = zeros(300)
+    be.dev_dense_gemv([(h, None, y.data_ptr())], pre=end)
+    close(host(y), w @ seen[0])
+    close(host(x_out), x)
+    assert np.array_equal(host(keep), a["x"][-1])
+    be.dev_free(h)
+
+
+def test_sublayer_end_in_a_product_of_words_that_are_not_aligned(be):
+    a, d, end, x_out, keep, x, seen = sublayer_case(256, 1, 1, False, "norm", seed=5)
+    moved = zeros(257)
+    moved[1:] = d["ya"][0]
+    end.y_a = moved.data_ptr() + 4
+    h, w = bf16_matrix(be, 40, 256, 9)
+    y = zeros(40)
+    be.dev_dense_gemv([(h, None, y.data_ptr())], pre=end)
+    close(host(y), w @ seen[0])
+    be.dev_free(h)
 
 
 def test_embedding_rows(be):

@@ -1,9 +1,15 @@
 // Decode-time products of bfloat16 matrices with one fp32 vector, memory-bound by design.
 //
-//   * one CTA per SM owns a contiguous slice of the launch's rows (over all its tensors); its sixteen warps split K in units of
-//     256 columns (and, where K has fewer units than warps, the row groups too), eight rows per step: a lane holds 16 bytes of
-//     each of eight rows and eight values of x, and two steps' loads (sixteen 16-byte words per lane) are in flight;
-//   * weights are constants: the first two steps' loads go out before the previous grid has finished (griddepcontrol);
+//   * one CTA per SM owns a contiguous slice of the launch's rows (over all its tensors); its eight warps split K in units of
+//     256 columns (and, where K has fewer units than warps, the row groups too), eight rows per step: a lane takes 16 bytes of
+//     each of eight rows and eight values of x;
+//   * weights arrive by cp.async in a ring of shared memory that belongs to one lane: a lane reads back the words it asked for
+//     itself, so a step needs no barrier, and the bytes in flight (three steps, 96 KB per CTA) cost no registers.  The first are
+//     asked for before the previous grid has finished (weights are constants; griddepcontrol).  B200, one product behind the
+//     other: 45056 x 4096 with a norm in front 65.0 -> 56.1 us, 4096 x 18432 30.6 -> 26.8, 6416 x 2048 with norm and shift
+//     9.0 -> 8.1, against sixteen warps that held two steps in registers (128 KB).  More in flight is slower (five steps: 58.6),
+//     sixteen warps too (58.9), and so is a CTA small enough to have the next launch's beside it: the SMs that finish first then
+//     take two of those each, and the pair above goes from 82.7 to 97.8;
 //   * the prologue can finish the sublayer before it (row_ops.cuh: grouped norm, residual add, token shift or output norm), so
 //     a decode step needs no launches for them: every CTA forms the input vector itself, CTA 0 stores the residual stream;
 //   * the epilogue adds a bias and applies the product's activation (squared ReLU, or the logits' soft cap) in fp32; a matrix may
@@ -14,10 +20,13 @@
 
 namespace zk {
 
-constexpr int kDenseThreads = 512, kDenseWarps = kDenseThreads / 32;
+constexpr int kDenseThreads = 256, kDenseWarps = kDenseThreads / 32;
 constexpr uint32_t kDenseUnit = 256;          // columns a warp takes at a time: eight per lane
 constexpr int kDenseRows = 8;                 // rows per step
 constexpr int kDenseMaxTasks = 4;
+constexpr uint32_t kDenseStepBytes = kDenseRows * kDenseUnit * 2;                                       // of one warp
+__host__ __device__ constexpr uint32_t dense_ring_bytes(int slots) { return slots * kDenseWarps * kDenseStepBytes; }
+constexpr int kPreQuads = 4;                  // four-value words of a row a lane keeps in the prologue: rows of up to 4096 values
 
 enum : int { kActNone = 0, kActSquaredRelu = 1, kActSoftcap = 2 };
 
@@ -40,6 +49,7 @@ struct DenseGemvParams {
     uint32_t k_split;         // warps that share a row group: a power of two, at most kDenseWarps
     uint32_t row_unit;        // a CTA's slice begins at a multiple of this many rows: 2 where a task has pairs
     uint32_t has_prologue;    // 1: one task, whose input is the prologue's view
+    uint32_t row_in_registers;  // the prologue by sublayer_in_registers; otherwise by row_ops.cuh's functions
     uint32_t scratch_floats;
     SublayerEnd pre;
 };
@@ -59,8 +69,123 @@ __device__ __forceinline__ void dense_fma8(const uint4& w, const float (&x)[8], 
         acc = fmaf(__uint_as_float(u[i] & 0xffff0000u), x[2 * i + 1], acc);
     }
 }
+__device__ __forceinline__ unsigned long long dense_pair(float lo, float hi) {
+    unsigned long long v;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(v) : "f"(lo), "f"(hi));
+    return v;
+}
+// The same with even and odd columns in the two halves of acc.
+__device__ __forceinline__ void dense_fma8_pairs(const uint4& w, const unsigned long long (&x)[4], unsigned long long& acc) {
+    const uint32_t u[4] = {w.x, w.y, w.z, w.w};
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+        asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(acc) : "l"(dense_pair(__uint_as_float(u[i] << 16), __uint_as_float(u[i] & 0xffff0000u))), "l"(x[i]));
+}
+// 16 bytes global -> shared, or 16 zero bytes.
+__device__ __forceinline__ void dense_copy(uint32_t dst, const void* src, bool real) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(real ? 16u : 0u) : "memory");
+}
 
-__global__ void __launch_bounds__(kDenseThreads, 1) gemv_bf16_kernel(const __grid_constant__ DenseGemvParams p) {
+// The prologue of rows of up to 4096 values (a multiple of 32, in 1, 2, 4 or 8 parts, every array 16-byte aligned), formed as
+// sublayer_row and sublayer_view form it: a warp holds an eighth of the row in registers, all arrays are asked for at once, and the
+// constants among them (norm weights, shift) before the previous grid has finished, when they may still have to come from HBM.
+// row_ops.cuh's functions go over the row in shared memory three to five times with a barrier after each.
+struct RowWords { float4 v[kPreQuads]; };
+__device__ __forceinline__ void row_words(RowWords& r, const float* src, uint32_t first, uint32_t chunk, uint32_t lane) {
+#pragma unroll
+    for (int q = 0; q < kPreQuads; ++q) {
+        const uint32_t i = 4 * (lane + 32 * q);
+        r.v[q] = src && i < chunk ? __ldcg(reinterpret_cast<const float4*>(src + first + i)) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    }
+}
+__device__ __forceinline__ float row_square_sum(const RowWords& r) {
+    float s = 0.0f;
+#pragma unroll
+    for (int q = 0; q < kPreQuads; ++q) s += (r.v[q].x * r.v[q].x + r.v[q].y * r.v[q].y) + (r.v[q].z * r.v[q].z + r.v[q].w * r.v[q].w);
+    return s;
+}
+template <typename F> __device__ __forceinline__ void row_each(RowWords& r, F f) {
+#pragma unroll
+    for (int q = 0; q < kPreQuads; ++q) {
+        f(r.v[q].x, q, 0);
+        f(r.v[q].y, q, 1);
+        f(r.v[q].z, q, 2);
+        f(r.v[q].w, q, 3);
+    }
+}
+__device__ __forceinline__ float row_at(const RowWords& r, int q, int c) { return c == 0 ? r.v[q].x : c == 1 ? r.v[q].y : c == 2 ? r.v[q].z : r.v[q].w; }
+
+struct PrologueConstants { RowWords norm, post; };      // norm_weight; shift or out_norm
+__device__ __forceinline__ void prologue_constants(PrologueConstants& c, const SublayerEnd& p) {
+    const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31, chunk = p.n / kDenseWarps;
+    row_words(c.norm, p.norm_weight, warp * chunk, chunk, lane);
+    row_words(c.post, p.shift ? p.shift : p.out_norm, warp * chunk, chunk, lane);
+}
+// xs [n] and a barrier; scratch: 4 * kDenseWarps floats.
+__device__ __forceinline__ void sublayer_in_registers(const SublayerEnd& p, const PrologueConstants& c, float* xs, float* scratch) {
+    const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31, chunk = p.n / kDenseWarps, first = warp * chunk;
+    const float part_size = static_cast<float>(p.n / p.groups);
+    const uint32_t per = kDenseWarps / p.groups, part = warp / per * per;      // the warps that share this warp's part of the norm
+    auto inverse_rms = [&](const float* sums, uint32_t from, uint32_t count, float size) {
+        float s = 0.0f;
+        for (uint32_t w = 0; w < count; ++w) s += sums[from + w];
+        return 1.0f / sqrtf(s / size + p.eps);
+    };
+    RowWords x, y, z;
+    row_words(x, p.x_in, first, chunk, lane);
+    row_words(y, p.y_a, first, chunk, lane);
+    row_words(z, p.y_b ? p.y_b : p.shift ? p.before : nullptr, first, chunk, lane);
+    if (p.y_b) {
+        RowWords a, b;
+        row_words(a, p.weight_a, first, chunk, lane);
+        row_words(b, p.weight_b, first, chunk, lane);
+        const float sa = warp_sum(row_square_sum(y)), sb = warp_sum(row_square_sum(z));
+        row_each(y, [&](float& v, int q, int k) { v *= row_at(a, q, k); });
+        row_each(z, [&](float& v, int q, int k) { v *= row_at(b, q, k); });
+        if (lane == 0) { scratch[warp] = sa; scratch[kDenseWarps + warp] = sb; }
+        __syncthreads();
+        const float ra = inverse_rms(scratch, 0, kDenseWarps, static_cast<float>(p.n)), rb = inverse_rms(scratch, kDenseWarps, kDenseWarps, static_cast<float>(p.n));
+        row_each(y, [&](float& v, int q, int k) { v = 0.5f * (v * ra + row_at(z, q, k) * rb); });
+        if (p.shift) row_words(z, p.before, first, chunk, lane);
+    }
+    if (p.y_a && p.norm_weight) {
+        const float s = warp_sum(row_square_sum(y));
+        if (lane == 0) scratch[2 * kDenseWarps + warp] = s;
+        __syncthreads();
+        const float r = inverse_rms(scratch, 2 * kDenseWarps + part, per, part_size);
+        row_each(y, [&](float& v, int q, int k) { v = row_at(x, q, k) + v * r * row_at(c.norm, q, k); });
+    } else {
+        row_each(y, [&](float& v, int q, int k) { v += row_at(x, q, k); });      // y_a null: y is zero
+    }
+    if (blockIdx.x == 0) {
+#pragma unroll
+        for (int q = 0; q < kPreQuads; ++q) {
+            const uint32_t i = 4 * (lane + 32 * q);
+            if (i < chunk && p.x_out) *reinterpret_cast<float4*>(p.x_out + first + i) = y.v[q];
+            if (i < chunk && p.keep) *reinterpret_cast<float4*>(p.keep + first + i) = x.v[q];
+        }
+    }
+    if (p.shift) {
+        row_each(y, [&](float& v, int q, int k) { v += (row_at(z, q, k) - v) * row_at(c.post, q, k); });
+    } else if (p.out_norm) {
+        const float s = warp_sum(row_square_sum(y));
+        if (lane == 0) scratch[3 * kDenseWarps + warp] = s;
+        __syncthreads();
+        const float r = inverse_rms(scratch, 3 * kDenseWarps + part, per, part_size);
+        row_each(y, [&](float& v, int q, int k) { v = v * r * row_at(c.post, q, k); });
+    }
+#pragma unroll
+    for (int q = 0; q < kPreQuads; ++q) {
+        const uint32_t i = 4 * (lane + 32 * q);
+        if (i < chunk) *reinterpret_cast<float4*>(xs + first + i) = y.v[q];
+    }
+    __syncthreads();
+}
+
+// kSlots: steps of a warp on their way at any time, in shared memory; 0: weights straight from memory, for inputs that leave no
+// room for a ring.
+template <int kSlots>
+__global__ void __launch_bounds__(kDenseThreads, 2) gemv_bf16_kernel(const __grid_constant__ DenseGemvParams p) {
     extern __shared__ __align__(16) float dense_smem[];
     const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const uint64_t row_units = (p.total_rows + p.row_unit - 1) / p.row_unit;
@@ -69,127 +194,165 @@ __global__ void __launch_bounds__(kDenseThreads, 1) gemv_bf16_kernel(const __gri
     const uint32_t team = warp / p.k_split, part = warp % p.k_split, teams = kDenseWarps / p.k_split;
     pdl_launch_dependents();
 
-    // a warp's steps: (task, row group, K unit), walked in that order.  Where the warps that share a row group do not divide its units
-    // evenly, the ones with a unit more are others in the next group: with the same warps every time, rows of 18432 columns (72
-    // units on 16 warps) kept half of the warps waiting for a tenth of the launch.  B200, sikivik 4096 x 4 layers,
-    // 301 + 32 tokens: 16129 -> 15892 us.
-    struct Walk { uint32_t ti, r, r_end, u; };
-    auto turn = [&](uint32_t units) { return units > p.k_split ? units & (p.k_split - 1) : 0u; };
+    // A warp's steps: (task, row group, K unit), walked in that order, once to ask for the weights and once to use them; what a step
+    // needs of its task stays in registers.  Where the warps that share a row group do not divide its units evenly, the ones with
+    // a unit more are others in the next group: with the same warps every time, rows of 18432 columns (72 units on 16 warps) kept
+    // half of the warps waiting for a tenth of the launch.
+    struct Walk {
+        const __nv_bfloat16* src;     // the lane's word of row r
+        uint32_t ti, r, r_end, u, units, ld, x;
+    };
+    auto place = [&](Walk& w) { w.src = p.task[w.ti].w + static_cast<size_t>(w.r) * w.ld + w.u * kDenseUnit + lane * 8; };
     auto enter = [&](Walk& w) {      // the next task of the slice with work for this warp
         for (; w.ti < p.tasks; ++w.ti) {
             const DenseTask& t = p.task[w.ti];
             const uint32_t a = max(slice0, t.first_row), b = min(slice1, t.first_row + t.rows);
-            if (a < b && a + team * kDenseRows < b && part < dense_units(t.ld)) {
+            w.ld = t.ld;
+            w.units = dense_units(t.ld);
+            if (a < b && a + team * kDenseRows < b && part < w.units) {
                 w.r = a - t.first_row + team * kDenseRows;
                 w.r_end = b - t.first_row;
                 w.u = part;
+                place(w);
                 return;
+            }
+            w.x += w.units * kDenseUnit;
+        }
+    };
+    auto advance = [&](Walk& w) {    // to the step after w
+        w.u += p.k_split;
+        w.src += p.k_split * kDenseUnit;
+        if (w.u >= w.units) {
+            w.u = (w.u + (w.units > p.k_split ? w.units : 0u)) & (p.k_split - 1);
+            w.r += teams * kDenseRows;
+            if (w.r < w.r_end) {
+                place(w);
+            } else {
+                w.x += w.units * kDenseUnit;
+                ++w.ti;
+                enter(w);
             }
         }
     };
-    auto load = [&](const Walk& w, uint4 (&v)[kDenseRows]) {
-        const DenseTask& t = p.task[w.ti];
-        const uint32_t col = w.u * kDenseUnit + lane * 8;
-        const __nv_bfloat16* base = t.w + static_cast<size_t>(w.r) * t.ld + col;
+    // the lane's words of a step lie 512 bytes apart, lane behind lane: neither the copies nor the reads meet bank conflicts
+    uint8_t* const mine = reinterpret_cast<uint8_t*>(dense_smem) + warp * kSlots * kDenseStepBytes + lane * 16;
+    auto ask = [&](const Walk& w, int slot) {      // rows past the slice's end keep what the slot held: their sums are not used
+        const uint32_t dst = smem_u32(mine) + slot * kDenseStepBytes;
+        const bool real = w.u * kDenseUnit + lane * 8 < w.ld;
+        const __nv_bfloat16* src = real ? w.src : w.src - lane * 8;
 #pragma unroll
         for (int i = 0; i < kDenseRows; ++i)
-            v[i] = (w.r + i < w.r_end && col < t.ld) ? __ldg(reinterpret_cast<const uint4*>(base + static_cast<size_t>(i) * t.ld)) : make_uint4(0, 0, 0, 0);
+            if (w.r + i < w.r_end) dense_copy(dst + i * 512, src + static_cast<size_t>(i) * w.ld, real);
     };
-    auto advance = [&](Walk& w) {    // to the step after w
-        const uint32_t units = dense_units(p.task[w.ti].ld);
-        const bool row_done = w.u + p.k_split >= units;
-        w.u += p.k_split;
-        if (row_done) {
-            w.u = (w.u + turn(units)) & (p.k_split - 1);
-            w.r += teams * kDenseRows;
-            if (w.r >= w.r_end) { ++w.ti; enter(w); }
-        }
-    };
-    // two steps' weights are in flight at any time: while one buffer is used up, the other's loads are on their way
-    uint4 buf0[kDenseRows], buf1[kDenseRows];
-    Walk w0{0, 0, 0, 0}, w1;
-    enter(w0);
-    if (w0.ti < p.tasks) load(w0, buf0);
-    w1 = w0;
-    if (w1.ti < p.tasks) advance(w1);
-    if (w1.ti < p.tasks) load(w1, buf1);
+    Walk in{}, at;
+    enter(in);
+    at = in;
+#pragma unroll
+    for (int s = 0; s < kSlots; ++s) {
+        if (in.ti < p.tasks) { ask(in, s); advance(in); }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    }
 
     // the input vectors in shared memory, each padded with zeros to whole units; then per-row partial sums of the slice
-    float* xs = dense_smem;
+    float* const xs = dense_smem + dense_ring_bytes(kSlots) / sizeof(float);
     uint32_t x_floats = 0;
-    pdl_wait();
+    // the bias of the thread's first row, which would otherwise come from HBM at the very end
+    float bias = 0.0f;
+    {
+        const uint32_t row = slice0 + threadIdx.x;
+        if (row < slice1) {
+            uint32_t ti = 0;
+            while (row >= p.task[ti].first_row + p.task[ti].rows) ++ti;
+            const DenseTask& t = p.task[ti];
+            const uint32_t r = row - t.first_row;
+            if (t.bias && r >= 2 * t.pairs) bias = __ldg(t.bias + r - 2 * t.pairs);
+        }
+    }
     if (p.has_prologue) {
         x_floats = dense_units(p.task[0].ld) * kDenseUnit;
-        float* scratch = dense_smem + x_floats;
-        sublayer_row<kDenseThreads>(p.pre, 0, xs, scratch);
-        if (blockIdx.x == 0) {
-            if (p.pre.x_out)
-                for (uint32_t i = threadIdx.x; i < p.pre.n; i += kDenseThreads) p.pre.x_out[i] = xs[i];
-            if (p.pre.keep)
-                for (uint32_t i = threadIdx.x; i < p.pre.n; i += kDenseThreads) p.pre.keep[i] = p.pre.x_in[i];
-        }
+        float* scratch = xs + x_floats;
         for (uint32_t i = p.pre.n + threadIdx.x; i < x_floats; i += kDenseThreads) xs[i] = 0.0f;
-        sublayer_view<kDenseThreads>(p.pre, xs, p.pre.before, scratch);
+        if (p.row_in_registers) {
+            PrologueConstants constants;
+            prologue_constants(constants, p.pre);
+            pdl_wait();
+            sublayer_in_registers(p.pre, constants, xs, scratch);
+        } else {
+            pdl_wait();
+            sublayer_row<kDenseThreads>(p.pre, 0, xs, scratch);
+            if (blockIdx.x == 0) {
+                if (p.pre.x_out)
+                    for (uint32_t i = threadIdx.x; i < p.pre.n; i += kDenseThreads) p.pre.x_out[i] = xs[i];
+                if (p.pre.keep)
+                    for (uint32_t i = threadIdx.x; i < p.pre.n; i += kDenseThreads) p.pre.keep[i] = p.pre.x_in[i];
+            }
+            sublayer_view<kDenseThreads>(p.pre, xs, p.pre.before, scratch);
+        }
     } else {
+        pdl_wait();
         for (uint32_t ti = 0; ti < p.tasks; ++ti) {
             const DenseTask& t = p.task[ti];
-            const uint32_t padded = dense_units(t.ld) * kDenseUnit;
+            const uint32_t padded = dense_units(t.ld) * kDenseUnit, words = reinterpret_cast<uintptr_t>(t.x) % 16 ? 0u : t.K / 4;
+            float4* dst = reinterpret_cast<float4*>(xs + x_floats);
 #pragma unroll 8
-            for (uint32_t i = threadIdx.x; i < padded; i += kDenseThreads) xs[x_floats + i] = i < t.K ? __ldcg(t.x + i) : 0.0f;
+            for (uint32_t i = threadIdx.x; i < words; i += kDenseThreads) dst[i] = __ldcg(reinterpret_cast<const float4*>(t.x) + i);
+            for (uint32_t i = 4 * words + threadIdx.x; i < padded; i += kDenseThreads) xs[x_floats + i] = i < t.K ? __ldcg(t.x + i) : 0.0f;
             x_floats += padded;
         }
         __syncthreads();
     }
-    float* sums = dense_smem + x_floats + p.scratch_floats;      // [rows of the slice][k_split]
+    float* sums = xs + x_floats + p.scratch_floats;      // [rows of the slice][k_split]
 
-    float acc[kDenseRows];
+    unsigned long long acc2[kDenseRows];
 #pragma unroll
-    for (int i = 0; i < kDenseRows; ++i) acc[i] = 0.0f;
-    auto consume = [&](const Walk& at, const uint4 (&w)[kDenseRows]) {
-        const DenseTask& t = p.task[at.ti];
-        uint32_t x_base = 0;                                      // where the task's input starts in xs
-        for (uint32_t i = 0; i < at.ti; ++i) x_base += dense_units(p.task[i].ld) * kDenseUnit;
-        const float4* xv = reinterpret_cast<const float4*>(xs + x_base + at.u * kDenseUnit + lane * 8);
+    for (int i = 0; i < kDenseRows; ++i) acc2[i] = 0ull;
+    auto consume = [&](const Walk& at, int slot) {
+        const float4* xv = reinterpret_cast<const float4*>(xs + at.x + at.u * kDenseUnit + lane * 8);
         const float4 x0 = xv[0], x1 = xv[1];
-        const float x[8] = {x0.x, x0.y, x0.z, x0.w, x1.x, x1.y, x1.z, x1.w};
+        const unsigned long long x[4] = {dense_pair(x0.x, x0.y), dense_pair(x0.z, x0.w), dense_pair(x1.x, x1.y), dense_pair(x1.z, x1.w)};
+        if constexpr (kSlots > 0) {
 #pragma unroll
-        for (int i = 0; i < kDenseRows; ++i) dense_fma8(w[i], x, acc[i]);
-        if (at.u + p.k_split < dense_units(t.ld)) return;
-        // the row group is done: eight sums over 32 lanes; at each of the first three exchanges a lane keeps half of the rows it carries
+            for (int i = 0; i < kDenseRows; ++i) dense_fma8_pairs(*reinterpret_cast<const uint4*>(mine + slot * kDenseStepBytes + i * 512), x, acc2[i]);
+        } else if (at.u * kDenseUnit + lane * 8 < at.ld) {
 #pragma unroll
-        for (int i = 0; i < 4; ++i) {
-            const bool hi = lane & 16;
-            const float keep = hi ? acc[i + 4] : acc[i], give = hi ? acc[i] : acc[i + 4];
-            acc[i] = keep + __shfl_xor_sync(0xffffffffu, give, 16);
+            for (int i = 0; i < kDenseRows; ++i)
+                if (at.r + i < at.r_end) dense_fma8_pairs(__ldg(reinterpret_cast<const uint4*>(at.src + static_cast<size_t>(i) * at.ld)), x, acc2[i]);
         }
+        if (at.u + p.k_split < at.units) return;
+        // the row group is done: its sums over 32 lanes; at each of the first exchanges a lane keeps half of the rows it carries
+        float acc[kDenseRows];
 #pragma unroll
-        for (int i = 0; i < 2; ++i) {
-            const bool hi = lane & 8;
-            const float keep = hi ? acc[i + 2] : acc[i], give = hi ? acc[i] : acc[i + 2];
-            acc[i] = keep + __shfl_xor_sync(0xffffffffu, give, 8);
+        for (int i = 0; i < kDenseRows; ++i) {
+            float lo, hi;
+            asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(acc2[i]));
+            acc[i] = lo + hi;
+            acc2[i] = 0ull;
         }
-        {
-            const bool hi = lane & 4;
-            const float keep = hi ? acc[1] : acc[0], give = hi ? acc[0] : acc[1];
-            acc[0] = keep + __shfl_xor_sync(0xffffffffu, give, 4);
-        }
-        acc[0] += __shfl_xor_sync(0xffffffffu, acc[0], 2);
-        acc[0] += __shfl_xor_sync(0xffffffffu, acc[0], 1);
-        const uint32_t mine = ((lane >> 4) & 1) * 4 + ((lane >> 3) & 1) * 2 + ((lane >> 2) & 1);
-        if ((lane & 3) == 0 && at.r + mine < at.r_end) sums[static_cast<size_t>(t.first_row + at.r + mine - slice0) * p.k_split + (at.u & (p.k_split - 1))] = acc[0];
+        uint32_t kept = 0;
 #pragma unroll
-        for (int i = 0; i < kDenseRows; ++i) acc[i] = 0.0f;
+        for (int n = kDenseRows / 2, o = 16; o > 0; n >>= 1, o >>= 1) {
+            if (n > 0) {
+                const bool up = lane & o;
+#pragma unroll
+                for (int i = 0; i < n; ++i) {
+                    const float keep = up ? acc[i + n] : acc[i], give = up ? acc[i] : acc[i + n];
+                    acc[i] = keep + __shfl_xor_sync(0xffffffffu, give, o);
+                }
+                kept += up ? n : 0;
+            } else {
+                acc[0] += __shfl_xor_sync(0xffffffffu, acc[0], o);
+            }
+        }
+        if ((lane & (32 / kDenseRows - 1)) == 0 && at.r + kept < at.r_end) sums[static_cast<size_t>(p.task[at.ti].first_row + at.r + kept - slice0) * p.k_split + (at.u & (p.k_split - 1))] = acc[0];
     };
-    while (w0.ti < p.tasks) {
-        consume(w0, buf0);
-        w0 = w1;
-        if (w0.ti < p.tasks) advance(w0);
-        if (w0.ti < p.tasks) load(w0, buf0);
-        if (w1.ti >= p.tasks) break;
-        consume(w1, buf1);
-        w1 = w0;
-        if (w1.ti < p.tasks) advance(w1);
-        if (w1.ti < p.tasks) load(w1, buf1);
+    for (int slot = 0; at.ti < p.tasks; advance(at)) {
+        if constexpr (kSlots > 0) asm volatile("cp.async.wait_group %0;" ::"n"(kSlots - 1) : "memory");
+        consume(at, slot);
+        if constexpr (kSlots > 0) {
+            if (in.ti < p.tasks) { ask(in, slot); advance(in); }      // into the slot that was just read by the same lane
+            asm volatile("cp.async.commit_group;" ::: "memory");
+            if (++slot == kSlots) slot = 0;
+        }
     }
     __syncthreads();
     for (uint32_t i = threadIdx.x; i < slice1 - slice0; i += kDenseThreads) {
@@ -207,7 +370,7 @@ __global__ void __launch_bounds__(kDenseThreads, 1) gemv_bf16_kernel(const __gri
         if (r < paired) {
             if (!(r & 1)) t.gated[r / 2] = silu_f(total(i)) * total(i + 1);
         } else {
-            t.y[r - paired] = dense_activation(total(i) + (t.bias ? __ldg(t.bias + r - paired) : 0.0f), t.act, t.cap);
+            t.y[r - paired] = dense_activation(total(i) + (i < kDenseThreads ? bias : t.bias ? __ldg(t.bias + r - paired) : 0.0f), t.act, t.cap);
         }
     }
 }

@@ -57,6 +57,16 @@ zk::SublayerEnd device_form(const zen_cuda_sublayer_end& s) {
     return zk::SublayerEnd{s.x_in, s.x_out, s.y_a, s.y_b, s.weight_a, s.weight_b, s.norm_weight, s.keep, s.shift, s.before, s.out_norm, s.n, s.groups, s.eps};
 }
 
+// Whether gemv_bf16's prologue takes the row in registers (zk::sublayer_in_registers).
+bool row_fits_registers(const zen_cuda_sublayer_end& s) {
+    if (s.n % (4 * zk::kDenseWarps) || s.n > zk::kDenseThreads * 4 * zk::kPreQuads || s.groups > zk::kDenseWarps || zk::kDenseWarps % s.groups) return false;
+    for (const void* a : {static_cast<const void*>(s.x_in), static_cast<const void*>(s.x_out), static_cast<const void*>(s.y_a), static_cast<const void*>(s.y_b),
+                          static_cast<const void*>(s.weight_a), static_cast<const void*>(s.weight_b), static_cast<const void*>(s.norm_weight), static_cast<const void*>(s.keep),
+                          static_cast<const void*>(s.shift), static_cast<const void*>(s.before), static_cast<const void*>(s.out_norm)})
+        if (reinterpret_cast<uintptr_t>(a) % 16) return false;
+    return true;
+}
+
 using EncodeTiledFn = CUresult (*)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*, const cuuint32_t*,
                                    const cuuint32_t*, CUtensorMapInterleave, CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
 // [outer][pitch] bf16, boxes of 64 columns x box_rows, 128-byte swizzle; what lies outside reads as zero.
@@ -200,13 +210,18 @@ int zen_cuda_dev_dense_gemv(const zen_cuda_dense_task* tasks, size_t count, cons
     if (pre) {
         p.has_prologue = 1;
         p.pre = device_form(*pre);
-        p.scratch_floats = (zk::row_scratch_floats(zk::kDenseThreads, pre->groups) + 3u) & ~3u;
+        p.row_in_registers = row_fits_registers(*pre);
+        p.scratch_floats = p.row_in_registers ? 4 * zk::kDenseWarps : (zk::row_scratch_floats(zk::kDenseThreads, pre->groups) + 3u) & ~3u;
     }
     const uint32_t row_units = u32((rows + p.row_unit - 1) / p.row_unit), grid = std::min<uint32_t>(u32(e.sm_count), row_units);
     const size_t slice = static_cast<size_t>((row_units + grid - 1) / grid) * p.row_unit;
-    const size_t smem = (x_floats + p.scratch_floats + slice * p.k_split) * sizeof(float);
-    if (smem > e.smem_optin) return e.fail("dense_gemv: the input vector and a slice's sums do not fit shared memory");
-    return e.leave(launch(e, zk::gemv_bf16_kernel, dim3(grid), dim3(zk::kDenseThreads), smem, p), "dense_gemv");
+    const size_t base = (x_floats + p.scratch_floats + slice * p.k_split) * sizeof(float);
+    const int slots = base + zk::dense_ring_bytes(3) <= e.smem_optin ? 3 : base + zk::dense_ring_bytes(2) <= e.smem_optin ? 2 : 0;
+    if (base + zk::dense_ring_bytes(slots) > e.smem_optin) return e.fail("dense_gemv: the input vector and a slice's sums do not fit shared memory");
+    // more than half of an SM's shared memory in any case: one CTA per SM (gemv_bf16.cuh)
+    const size_t smem = std::max(base + zk::dense_ring_bytes(slots), e.smem_optin / 2 + 1024);
+    auto go = [&](auto kernel) { return e.leave(launch(e, kernel, dim3(grid), dim3(zk::kDenseThreads), smem, p), "dense_gemv"); };
+    return slots == 3 ? go(zk::gemv_bf16_kernel<3>) : slots == 2 ? go(zk::gemv_bf16_kernel<2>) : go(zk::gemv_bf16_kernel<0>);
 }
 
 int zen_cuda_dev_dense_gemm(const zen_cuda_weights* w, const void* d_x, size_t x_ld, size_t tokens, void* d_out, size_t out_ld, int out_bf16,
