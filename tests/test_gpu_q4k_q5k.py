@@ -9,7 +9,7 @@ import os
 import numpy as np
 import pytest
 
-from helpers import assert_parity, seeded_acts
+from helpers import assert_parity, seeded_acts, seeded_weights
 from zeninfer_b200 import blocks
 
 pytestmark = pytest.mark.gpu
@@ -112,3 +112,102 @@ def test_tensor_core_product_vs_oracle(be, zo, fmt, name, tag, rows, cols, token
     host = be.gemm(name, w, x, tokens, rows, cols)
     assert np.array_equal(host, outs[True])       # the same kernels on the same bytes
     be.release_weights(w)
+
+
+# ---- the matrix instructions' kernel (gemv_kq_mma.cuh), all formats ----
+ALL = {"Q4_0": blocks.Q4_0, "Q6_K": blocks.Q6_K, "Q4_K": blocks.Q4_K, "Q5_K": blocks.Q5_K}
+
+
+def _weights(fmt, rows, cols, seed):
+    return blocks.random_k_blocks(fmt, rows, cols, seed) if fmt in (blocks.Q4_K, blocks.Q5_K) else seeded_weights(fmt, rows, cols, seed)
+
+
+def _products(be, name, w, x, rows, cols):
+    """dev_gemv of all rows of x in one launch."""
+    import torch
+    tokens = x.shape[0]
+    h = be.dev_upload(name, w, rows, cols)
+    d_x, y = torch.from_numpy(x).cuda(), torch.full((tokens, rows), float("nan"), device="cuda")
+    be.dev_gemv([h], [y.data_ptr()], d_x.data_ptr(), tokens, 2)
+    be.dev_check()
+    be.dev_free(h)
+    return y.cpu().numpy()
+
+
+def _close_to_f64(got, fmt, w, x, some_rows, cols, repeat):
+    """Within 2^-22 of an activation per product (two f16 digits) and the rounding of fp32 sums over a row, of the terms' magnitudes (a
+    Q4_K / Q5_K weight is the difference of two terms, the smaller of at most 63 * 1.5e-4, random_k_blocks); and per product
+    2^-14 of a block's step times its largest activation: what the matrix instruction keeps of a product beside the largest of its
+    sixteen, 24 bits below the exponent of an f16 number of ten mantissa bits."""
+    decoded = blocks.dequantize(fmt, w[:some_rows], some_rows, cols).astype(np.float64)
+    want, terms = x.astype(np.float64) @ decoded.T, np.abs(x).astype(np.float64) @ (np.abs(decoded) + (0.019 if fmt in (blocks.Q4_K, blocks.Q5_K) else 0.0)).T
+    n = 16 if fmt == blocks.Q6_K else 32
+    values = np.sort(decoded.reshape(some_rows, -1, n), axis=2)
+    gaps = np.diff(values, axis=2)
+    step = np.where(gaps > 1e-9 * np.abs(values).max(), gaps, np.inf).min(axis=2)          # [rows][blocks]
+    largest = np.abs(x).astype(np.float64).reshape(x.shape[0], -1, n).max(axis=2)
+    bound = terms * (2.0 ** -22 + 64 * 2.0 ** -24) + n * 2.0 ** -14 * largest @ np.where(np.isfinite(step), step, 0.0).T + 1e-30
+    for first in range(0, got.shape[1], some_rows):
+        part = got[:, first:first + some_rows]
+        assert np.all(np.abs(part - want[:, :part.shape[1]]) <= bound[:, :part.shape[1]])
+        if not repeat:
+            break
+
+
+# edges of tiles (16 rows), of units (256 columns; Q4_0 ends inside one), of warps' shares; one or more groups of four tokens;
+# 16384 columns by three tokens and 14336 by two or three go over the row in several passes
+@pytest.mark.parametrize("name", list(ALL))
+@pytest.mark.parametrize("rows,cols,tokens", [(1, 256, 3), (15, 256, 4), (17, 512, 5), (33, 768, 8), (1200, 4096, 3), (2405, 1280, 4), (2405, 1280, 7), (300, 14336, 2), (300, 14336, 3),
+                                              (140, 11008, 3), (5000, 256, 6)])
+def test_several_rows_at_once(be, name, rows, cols, tokens):
+    fmt = ALL[name]
+    if name == "Q6_K" and cols * tokens > 32768:
+        tokens = 2
+    if name == "Q6_K" and tokens == 2:
+        rows = 4700                     # 64 M weights
+    elif name == "Q6_K":
+        rows += (1 << 20) // cols + 1   # more than a million
+    w, x = _weights(fmt, rows, cols, rows + tokens), seeded_acts(tokens, cols, cols)
+    _close_to_f64(_products(be, name, w, x, rows, cols), fmt, w, x, rows, cols, False)
+
+
+@pytest.mark.parametrize("rows,cols,tokens", [(37, 32, 3), (70, 96, 4), (129, 544, 8), (64, 4128, 2), (18, 16384, 3)])
+def test_q4_0_rows_that_end_inside_a_unit(be, rows, cols, tokens):
+    w, x = _weights(blocks.Q4_0, rows, cols, rows), seeded_acts(tokens, cols, cols)
+    _close_to_f64(_products(be, "Q4_0", w, x, rows, cols), blocks.Q4_0, w, x, rows, cols, False)
+
+
+# one activation row comes here from 64 M weights on (Q4_0) or 32 M (Q4_K, Q5_K); the rows of a small matrix over and over
+@pytest.mark.parametrize("name,rows,cols", [("Q4_0", 16500, 4096), ("Q4_0", 16400, 4128), ("Q4_0", 4700, 14336), ("Q4_0", 262200, 256), ("Q4_K", 8200, 4096), ("Q4_K", 3077, 11008),
+                                            ("Q5_K", 8200, 4096), ("Q5_K", 32800, 1024)])
+def test_one_row_of_a_large_matrix(be, name, rows, cols):
+    fmt, some = ALL[name], 50
+    part = _weights(fmt, some, cols, rows)
+    w, x = np.ascontiguousarray(np.tile(part, (rows // some + 1, 1))[:rows]), seeded_acts(1, cols, cols)
+    _close_to_f64(_products(be, name, w, x, rows, cols), fmt, w, x, some, cols, True)
+
+
+def test_more_rows_than_their_sums_fit(be):
+    rows, some, tokens = 700_000, 64, 8
+    part = _weights(blocks.Q4_0, some, 32, 3)
+    w, x = np.ascontiguousarray(np.tile(part, (rows // some + 1, 1))[:rows]), seeded_acts(tokens, 32, 4)
+    _close_to_f64(_products(be, "Q4_0", w, x, rows, 32), blocks.Q4_0, w, x, some, 32, True)
+
+
+@pytest.mark.parametrize("name", list(ALL))
+def test_activations_of_any_size(be, name):
+    """The operands are scaled by a power of two per 256 columns: vectors of very large, very small and no values, and both in one."""
+    fmt, rows, cols = ALL[name], 1100, 1024
+    w, x = _weights(fmt, rows, cols, 9), seeded_acts(5, cols, 10)
+    x[0] *= np.float32(2.0 ** 100)
+    x[1] *= np.float32(2.0 ** -80)
+    x[2] = 0
+    x[3, :256] *= np.float32(2.0 ** 40)
+    x[3, 256:512] *= np.float32(2.0 ** -40)
+    x[4, 300] = np.float32(3e5)
+    got = _products(be, name, w, x, rows, cols)
+    assert not got[2].any()
+    _close_to_f64(got, fmt, w, x, rows, cols, False)
+    x[1, 17], x[4, 5] = np.nan, np.inf              # a row's own business
+    bad = _products(be, name, w, x, rows, cols)
+    assert np.array_equal(bad[[0, 2, 3]], got[[0, 2, 3]]) and not np.isfinite(bad[[1, 4]]).any()

@@ -199,10 +199,10 @@ __global__ void __launch_bounds__(kDenseThreads, 2) gemv_bf16_kernel(const __gri
     // a unit more are others in the next group: with the same warps every time, rows of 18432 columns (72 units on 16 warps) kept
     // half of the warps waiting for a tenth of the launch.
     struct Walk {
-        const __nv_bfloat16* src;     // the lane's word of row r
+        const __nv_bfloat16* w;       // the lane's word of row r
         uint32_t ti, r, r_end, u, units, ld, x;
     };
-    auto place = [&](Walk& w) { w.src = p.task[w.ti].w + static_cast<size_t>(w.r) * w.ld + w.u * kDenseUnit + lane * 8; };
+    auto place = [&](Walk& w) { w.w = p.task[w.ti].w + static_cast<size_t>(w.r) * w.ld + w.u * kDenseUnit + lane * 8; };
     auto enter = [&](Walk& w) {      // the next task of the slice with work for this warp
         for (; w.ti < p.tasks; ++w.ti) {
             const DenseTask& t = p.task[w.ti];
@@ -221,7 +221,7 @@ __global__ void __launch_bounds__(kDenseThreads, 2) gemv_bf16_kernel(const __gri
     };
     auto advance = [&](Walk& w) {    // to the step after w
         w.u += p.k_split;
-        w.src += p.k_split * kDenseUnit;
+        w.w += p.k_split * kDenseUnit;
         if (w.u >= w.units) {
             w.u = (w.u + (w.units > p.k_split ? w.units : 0u)) & (p.k_split - 1);
             w.r += teams * kDenseRows;
@@ -239,7 +239,7 @@ __global__ void __launch_bounds__(kDenseThreads, 2) gemv_bf16_kernel(const __gri
     auto ask = [&](const Walk& w, int slot) {      // rows past the slice's end keep what the slot held: their sums are not used
         const uint32_t dst = smem_u32(mine) + slot * kDenseStepBytes;
         const bool real = w.u * kDenseUnit + lane * 8 < w.ld;
-        const __nv_bfloat16* src = real ? w.src : w.src - lane * 8;
+        const __nv_bfloat16* src = real ? w.w : w.w - lane * 8;
 #pragma unroll
         for (int i = 0; i < kDenseRows; ++i)
             if (w.r + i < w.r_end) dense_copy(dst + i * 512, src + static_cast<size_t>(i) * w.ld, real);
@@ -316,7 +316,7 @@ __global__ void __launch_bounds__(kDenseThreads, 2) gemv_bf16_kernel(const __gri
         } else if (at.u * kDenseUnit + lane * 8 < at.ld) {
 #pragma unroll
             for (int i = 0; i < kDenseRows; ++i)
-                if (at.r + i < at.r_end) dense_fma8_pairs(__ldg(reinterpret_cast<const uint4*>(at.src + static_cast<size_t>(i) * at.ld)), x, acc2[i]);
+                if (at.r + i < at.r_end) dense_fma8_pairs(__ldg(reinterpret_cast<const uint4*>(at.w + static_cast<size_t>(i) * at.ld)), x, acc2[i]);
         }
         if (at.u + p.k_split < at.units) return;
         // the row group is done: its sums over 32 lanes; at each of the first exchanges a lane keeps half of the rows it carries

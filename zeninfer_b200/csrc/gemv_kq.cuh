@@ -1,4 +1,5 @@
-// Decode-time matrix-vector products for Q4_0, Q6_K, Q4_K and Q5_K (batch 1..8).
+// Decode-time matrix-vector products for Q4_0, Q6_K, Q4_K and Q5_K with one activation row, and for Q6_K with up to eight; which launches
+// come here and which to the matrix instructions of gemv_kq_mma.cuh: kq_takes_mma there.
 //
 // The reference evaluates both formats with fp32 activations: Q4_0 through its generic
 // dequantise-then-dot route (src/quant.cpp:1135-1162 over gemv_avx2, kernels/avx2.cpp:16-40) and
@@ -211,6 +212,7 @@ __global__ void __launch_bounds__(kGemvThreads, 1) gemv_kq_kernel(const __grid_c
     using F = KqFormat<kFormat>;
     constexpr int kStages = F::kStages;
     static_assert(kStages % kTeams == 0, "ring depth must be a multiple of the number of consumer teams");
+    static_assert(kBatch == 1 || kFormat == 14 || kFormat == kFormatQ6KCodes, "more rows: gemv_kq_mma.cuh");
     constexpr uint32_t kStageBytes = kq_stage_bytes<kFormat>();
     extern __shared__ __align__(128) uint8_t smem[];
     const uint32_t kpad = p.nseg * kKqSegElems;
@@ -619,78 +621,7 @@ __global__ void __launch_bounds__(kGemvThreads, 1) gemv_kq_kernel(const __grid_c
                     const uint8_t* st = ring + stage * kStageBytes;
                     const uint32_t e_base = s * kKqSegElems;
                     const uint32_t elems = min(static_cast<uint32_t>(kKqSegElems), p.K - e_base);
-                    if (kFormat == 2) {
-                        // ---- Q4_0: a lane owns a 32-weight block: 16 nibble bytes + one scale ----
-                        const uint4* nib = reinterpret_cast<const uint4*>(st + kq_plane_offset<kFormat>(0) + twarp * F::seg_bytes(0));
-                        const __half* ws = reinterpret_cast<const __half*>(st + kq_plane_offset<kFormat>(1) + twarp * F::seg_bytes(1));
-    #pragma unroll
-                        for (int i = 0; i < kKqSegElems / 32 / 32; ++i) {
-                            const uint32_t bl = i * 32 + lane;
-                            if (bl * 32 < elems) {
-                                const uint4 w = nib[bl];
-                                const float dw = __half2float(ws[bl]);
-                                // low nibbles are elements 0..15, high nibbles elements 16..31 (src/quant.cpp:391-397)
-                                const uint4 lo = make_uint4(w.x & 0x0F0F0F0Fu, w.y & 0x0F0F0F0Fu, w.z & 0x0F0F0F0Fu, w.w & 0x0F0F0F0Fu);
-                                const uint4 hi = make_uint4((w.x >> 4) & 0x0F0F0F0Fu, (w.y >> 4) & 0x0F0F0F0Fu, (w.z >> 4) & 0x0F0F0F0Fu, (w.w >> 4) & 0x0F0F0F0Fu);
-                                const uint32_t b = e_base / 32 + bl;
-    #pragma unroll
-                                for (int tk = 0; tk < kBatch; ++tk) {
-                                    const uint4* x1 = reinterpret_cast<const uint4*>(xd + static_cast<size_t>(tk) * 2 * kpad + b * 32);
-                                    const uint4* x2 = reinterpret_cast<const uint4*>(xd + static_cast<size_t>(tk) * 2 * kpad + kpad + b * 32);
-                                    const int i1 = dot16(lo, x1[0]) + dot16(hi, x1[1]);
-                                    const int i2 = dot16(lo, x2[0]) + dot16(hi, x2[1]);
-                                    const int isum = i1 * 256 + i2 - 8 * xsum[static_cast<size_t>(tk) * (kpad / 32) + b];
-                                    acc[tk] = fmaf(dw * xscale[static_cast<size_t>(tk) * (kpad / 32) + b], static_cast<float>(isum), acc[tk]);
-                                }
-                            }
-                        }
-                    } else if (kq_is_k45<kFormat>) {
-                        // ---- Q4_K / Q5_K: a lane owns 16 nibble bytes (16 weights of sub-block 2j and 16 of 2j+1); a warp covers four super-blocks a pass ----
-                        constexpr int kScm = F::kPlanes - 2, kDd = F::kPlanes - 1;
-                        const uint8_t* qs = st + kq_plane_offset<kFormat>(0) + twarp * F::seg_bytes(0);
-                        const uint8_t* q5p = st + kq_plane_offset<kFormat>(1) + twarp * F::seg_bytes(1);
-                        const uint8_t* scm = st + kq_plane_offset<kFormat>(kScm) + twarp * F::seg_bytes(kScm);
-                        const __half2* dd = reinterpret_cast<const __half2*>(st + kq_plane_offset<kFormat>(kDd) + twarp * F::seg_bytes(kDd));
-                        const uint32_t j = (static_cast<uint32_t>(lane) >> 1) & 3, h = lane & 1;
-    #pragma unroll
-                        for (int i = 0; i < kKqSegElems / 256 / 4; ++i) {
-                            const uint32_t sbl = i * 4 + (lane >> 3);
-                            if (sbl * 256 < elems) {
-                                const uint4 w = *reinterpret_cast<const uint4*>(qs + sbl * 128 + j * 32 + h * 16);
-                                const uint32_t m = 0x0F0F0F0Fu;
-                                uint4 lo = make_uint4(w.x & m, w.y & m, w.z & m, w.w & m);
-                                uint4 hi = make_uint4((w.x >> 4) & m, (w.y >> 4) & m, (w.z >> 4) & m, (w.w >> 4) & m);
-                                if (kFormat == 13) {
-                                    const uint4 q5 = *reinterpret_cast<const uint4*>(q5p + sbl * 32 + h * 16);
-                                    const uint32_t s_lo = 2 * j, s_hi = 2 * j + 1, one = 0x01010101u;
-                                    lo.x |= ((q5.x >> s_lo) & one) << 4; lo.y |= ((q5.y >> s_lo) & one) << 4; lo.z |= ((q5.z >> s_lo) & one) << 4; lo.w |= ((q5.w >> s_lo) & one) << 4;
-                                    hi.x |= ((q5.x >> s_hi) & one) << 4; hi.y |= ((q5.y >> s_hi) & one) << 4; hi.z |= ((q5.z >> s_hi) & one) << 4; hi.w |= ((q5.w >> s_hi) & one) << 4;
-                                }
-                                const uint32_t sc2 = *reinterpret_cast<const uint16_t*>(scm + sbl * 16 + j * 2);
-                                const uint32_t mn2 = *reinterpret_cast<const uint16_t*>(scm + sbl * 16 + 8 + j * 2);
-                                const float2 dm = __half22float2(dd[sbl]);
-                                const float ds_lo = dm.x * static_cast<float>(sc2 & 0xffu), ds_hi = dm.x * static_cast<float>(sc2 >> 8);   // (d * scale), (dmin * m):
-                                const float ms_lo = dm.y * static_cast<float>(mn2 & 0xffu), ms_hi = dm.y * static_cast<float>(mn2 >> 8);   // the reference's factors
-                                const uint32_t e_lo = e_base + sbl * 256 + j * 64 + h * 16, e_hi = e_lo + 32;
-                                const uint4 ones = make_uint4(0x01010101u, 0x01010101u, 0x01010101u, 0x01010101u);
-    #pragma unroll
-                                for (int tk = 0; tk < kBatch; ++tk) {
-                                    const uint8_t* xt = xd + static_cast<size_t>(tk) * 2 * kpad;
-                                    const uint4 a1 = *reinterpret_cast<const uint4*>(xt + e_lo), b1 = *reinterpret_cast<const uint4*>(xt + e_hi);
-                                    const uint4 a2 = *reinterpret_cast<const uint4*>(xt + kpad + e_lo), b2 = *reinterpret_cast<const uint4*>(xt + kpad + e_hi);
-                                    const float xs_lo = xscale[static_cast<size_t>(tk) * (kpad / 32) + e_lo / 32], xs_hi = xscale[static_cast<size_t>(tk) * (kpad / 32) + e_hi / 32];
-                                    const int i_lo = dot16(lo, a1) * 256 + dot16(lo, a2), i_hi = dot16(hi, b1) * 256 + dot16(hi, b2);
-                                    const int s_lo = dot16(ones, a1) * 256 + dot16(ones, a2), s_hi = dot16(ones, b1) * 256 + dot16(ones, b2);
-                                    float v = acc[tk];
-                                    v = fmaf(ds_lo * xs_lo, static_cast<float>(i_lo), v);
-                                    v = fmaf(ds_hi * xs_hi, static_cast<float>(i_hi), v);
-                                    v = fmaf(-ms_lo * xs_lo, static_cast<float>(s_lo), v);
-                                    v = fmaf(-ms_hi * xs_hi, static_cast<float>(s_hi), v);
-                                    acc[tk] = v;
-                                }
-                            }
-                        }
-                    } else if (kFormat == kFormatQ6KCodes) {
+                    if (kFormat == kFormatQ6KCodes) {
                         // ---- Q6_K, unpacked codes: a lane owns one 16-weight group in element order; two super-blocks a pass ----
                         const uint8_t* qc = st + kq_plane_offset<kFormat>(0) + twarp * F::seg_bytes(0);
                         const int8_t* sc = reinterpret_cast<const int8_t*>(st + kq_plane_offset<kFormat>(1) + twarp * F::seg_bytes(1));

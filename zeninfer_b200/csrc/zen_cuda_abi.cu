@@ -31,6 +31,7 @@
 #include "gemm_q8_0_i8.cuh"
 #include "gemm_groups.cuh"
 #include "gemv_kq.cuh"
+#include "gemv_kq_mma.cuh"
 #include "gemv_list.cuh"
 #include "gemv_q8_0.cuh"
 #include "greedy_pick.cuh"
@@ -527,19 +528,80 @@ cudaError_t launch_gemv_kq(const zk::KqParams& p, unsigned grid, size_t smem, cu
     return cudaLaunchKernelEx(&cfg, fn, p);
 }
 
-template <int kFormat>
-cudaError_t dispatch_kq(int batch, const zk::KqParams& p, unsigned grid, size_t smem, cudaStream_t st, bool pdl) {
-    switch (batch) {
-    case 1: return launch_gemv_kq<kFormat, 1>(p, grid, smem, st, pdl);
-    case 2: return launch_gemv_kq<kFormat, 2>(p, grid, smem, st, pdl);
-    case 3: return launch_gemv_kq<kFormat, 3>(p, grid, smem, st, pdl);
-    case 4: return launch_gemv_kq<kFormat, 4>(p, grid, smem, st, pdl);
-    case 5: return launch_gemv_kq<kFormat, 5>(p, grid, smem, st, pdl);
-    case 6: return launch_gemv_kq<kFormat, 6>(p, grid, smem, st, pdl);
-    case 7: return launch_gemv_kq<kFormat, 7>(p, grid, smem, st, pdl);
-    case 8: return launch_gemv_kq<kFormat, 8>(p, grid, smem, st, pdl);
-    default: return cudaErrorInvalidValue;
+template <int kFormat, int kWide>
+cudaError_t launch_gemv_kq_mma(State& s, zk::KqmParams& p, unsigned grid, bool stash, cudaStream_t st) {
+    constexpr uint32_t kWarps = zk::kqm_threads<kWide>() / 32;
+    const uint32_t units = zk::kqm_units(p.K);
+    const size_t unit = static_cast<size_t>(p.tokens) * zk::kqm_unit_bytes<kFormat>(), most = s.smem_optin;
+    const bool choose = grid == 0;      // otherwise the gather's, whose outputs are collected in shared memory (stash)
+    if (choose) grid = std::max(1u, std::min<unsigned>((p.total_rows + 7) / 8, static_cast<unsigned>(s.sm_count)));
+    // The warps of a CTA share tiles and units so that the busiest has the fewest steps; with equal counts a tile goes to fewer
+    // warps, whose partial sums take less shared memory.  Sums and activations have to leave room for the ring.
+    size_t fixed = 0;
+    auto split = [&] {
+        const uint32_t slice = (p.total_rows + grid - 1) / grid, tiles = (slice + zk::kKqTile - 1) / zk::kKqTile;
+        uint32_t best = 0;
+        for (uint32_t k = 1; k <= kWarps && k <= units; k *= 2) {
+            const size_t sums = static_cast<size_t>(slice) * p.tokens * (k + (stash && k > 1 ? 1 : 0)) * sizeof(float);
+            const size_t bytes = zk::kqm_ring_bytes<kFormat, kWide>() + 16 + sums;
+            if (bytes + k * unit > most) break;
+            const uint32_t teams = kWarps / k, steps = (tiles + teams - 1) / teams * ((units + k - 1) / k);
+            if (!best || steps < best) { best = steps; p.k_split = k; fixed = bytes; }
+        }
+        return best != 0;
+    };
+    while (!split()) {           // so many rows that their sums do not fit: several CTAs after one another
+        if (!choose || grid >= p.total_rows) return cudaErrorInvalidValue;
+        grid = std::min(2 * grid, p.total_rows);
     }
+    p.pass_units = static_cast<uint32_t>(std::min<size_t>(units, (most - fixed) / unit));
+    if (p.pass_units < units) p.pass_units -= p.pass_units % p.k_split;
+    // more than half of an SM's shared memory in any case: one CTA per SM (gemv_bf16.cuh)
+    const size_t smem = std::max(fixed + p.pass_units * unit, most / 2 + 1024);
+    auto* fn = &zk::gemv_kq_mma_kernel<kFormat, kWide>;
+    static size_t configured = 0;
+    if (smem > configured) {
+        cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
+        if (e == cudaSuccess) e = cudaFuncSetAttribute(fn, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
+        if (e != cudaSuccess) return e;
+        configured = smem;
+    }
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(grid);
+    cfg.blockDim = dim3(zk::kqm_threads<kWide>());
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    cudaLaunchAttribute attr{};
+    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr.val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = &attr;
+    cfg.numAttrs = s.pdl ? 1 : 0;
+    return cudaLaunchKernelEx(&cfg, fn, p);
+}
+
+template <int kFormat>
+cudaError_t dispatch_kq_mma(State& s, zk::KqmParams& p, unsigned grid, bool stash, cudaStream_t st) {
+    if constexpr (!zk::kq_is_q6<kFormat>)
+        if (p.tokens == 1) return launch_gemv_kq_mma<kFormat, 0>(s, p, grid, stash, st);
+    return p.tokens <= 4 ? launch_gemv_kq_mma<kFormat, 1>(s, p, grid, stash, st) : launch_gemv_kq_mma<kFormat, 2>(s, p, grid, stash, st);
+}
+
+template <int kFormat>
+cudaError_t dispatch_kq(size_t tokens, const zk::KqParams& p, unsigned grid, size_t smem, cudaStream_t st, bool pdl) {
+    if (tokens == 1) return launch_gemv_kq<kFormat, 1>(p, grid, smem, st, pdl);
+    if constexpr (zk::kq_is_q6<kFormat>) {
+        switch (tokens) {
+        case 2: return launch_gemv_kq<kFormat, 2>(p, grid, smem, st, pdl);
+        case 3: return launch_gemv_kq<kFormat, 3>(p, grid, smem, st, pdl);
+        case 4: return launch_gemv_kq<kFormat, 4>(p, grid, smem, st, pdl);
+        case 5: return launch_gemv_kq<kFormat, 5>(p, grid, smem, st, pdl);
+        case 6: return launch_gemv_kq<kFormat, 6>(p, grid, smem, st, pdl);
+        case 7: return launch_gemv_kq<kFormat, 7>(p, grid, smem, st, pdl);
+        case 8: return launch_gemv_kq<kFormat, 8>(p, grid, smem, st, pdl);
+        default: break;
+        }
+    }
+    return cudaErrorInvalidValue;
 }
 
 size_t gemv_smem_bytes(int format, size_t cols, size_t tokens, int act_mode) {   // format: a kernel format (zen_cuda_weights::kernel_format)
@@ -599,12 +661,30 @@ bool enqueue_gemv_kq(State& s, const zen_cuda_weights* const* w, float* const* d
                                  : std::max(1u, std::min<unsigned>((total_rows + zk::kGemvWarps - 1) / zk::kGemvWarps, static_cast<unsigned>(s.sm_count)));
     const size_t smem = gemv_smem_bytes(fmt, w[0]->cols, tokens, ZEN_CUDA_ACT_FP32)
                         + (gather ? zk::gather_stash_bytes(total_rows, grid, static_cast<int>(tokens)) : 0);
+    // the limit of the entry points, which callers split their tokens by; the matrix instructions' kernel takes longer inputs in passes
     if (smem > s.smem_optin) return set_error(s, "gemv: activation rows do not fit shared memory (columns x tokens too large)");
-    const cudaError_t e = fmt == ZEN_CUDA_Q4_0   ? dispatch_kq<ZEN_CUDA_Q4_0>(static_cast<int>(tokens), p, grid, smem, st, s.pdl)
-                          : fmt == ZEN_CUDA_Q4_K ? dispatch_kq<ZEN_CUDA_Q4_K>(static_cast<int>(tokens), p, grid, smem, st, s.pdl)
-                          : fmt == ZEN_CUDA_Q5_K ? dispatch_kq<ZEN_CUDA_Q5_K>(static_cast<int>(tokens), p, grid, smem, st, s.pdl)
-                          : fmt == zk::kFormatQ6KCodes ? dispatch_kq<zk::kFormatQ6KCodes>(static_cast<int>(tokens), p, grid, smem, st, s.pdl)
-                                                 : dispatch_kq<ZEN_CUDA_Q6_K>(static_cast<int>(tokens), p, grid, smem, st, s.pdl);
+    const bool q6 = fmt == ZEN_CUDA_Q6_K || fmt == zk::kFormatQ6KCodes;
+    cudaError_t e;
+    if (zk::kq_takes_mma(fmt == ZEN_CUDA_Q4_0, q6, tokens, static_cast<uint64_t>(total_rows) * p.K)) {
+        zk::KqmParams m{};
+        std::copy(std::begin(p.task), std::end(p.task), std::begin(m.task));
+        std::copy(std::begin(p.pitch), std::end(p.pitch), std::begin(m.pitch));
+        m.ntasks = p.ntasks; m.total_rows = total_rows; m.x = d_x; m.K = p.K; m.error_word = s.d_error; m.gather = p.gather;
+        m.tokens = static_cast<uint32_t>(tokens);
+        m.token_magic = static_cast<uint32_t>(((uint64_t(1) << 32) + tokens - 1) / tokens);
+        const unsigned g = gather ? grid : 0;
+        e = fmt == ZEN_CUDA_Q4_0   ? dispatch_kq_mma<ZEN_CUDA_Q4_0>(s, m, g, gather != nullptr, st)
+            : fmt == ZEN_CUDA_Q4_K ? dispatch_kq_mma<ZEN_CUDA_Q4_K>(s, m, g, gather != nullptr, st)
+            : fmt == ZEN_CUDA_Q5_K ? dispatch_kq_mma<ZEN_CUDA_Q5_K>(s, m, g, gather != nullptr, st)
+            : fmt == zk::kFormatQ6KCodes ? dispatch_kq_mma<zk::kFormatQ6KCodes>(s, m, g, gather != nullptr, st)
+                                         : dispatch_kq_mma<ZEN_CUDA_Q6_K>(s, m, g, gather != nullptr, st);
+    } else {
+        e = fmt == ZEN_CUDA_Q4_0   ? dispatch_kq<ZEN_CUDA_Q4_0>(tokens, p, grid, smem, st, s.pdl)
+            : fmt == ZEN_CUDA_Q4_K ? dispatch_kq<ZEN_CUDA_Q4_K>(tokens, p, grid, smem, st, s.pdl)
+            : fmt == ZEN_CUDA_Q5_K ? dispatch_kq<ZEN_CUDA_Q5_K>(tokens, p, grid, smem, st, s.pdl)
+            : fmt == zk::kFormatQ6KCodes ? dispatch_kq<zk::kFormatQ6KCodes>(tokens, p, grid, smem, st, s.pdl)
+                                         : dispatch_kq<ZEN_CUDA_Q6_K>(tokens, p, grid, smem, st, s.pdl);
+    }
     if (e != cudaSuccess) return set_error(s, std::string("gemv launch: ") + cudaGetErrorString(e));
     ++s.stats.dispatches;
     return true;
