@@ -410,6 +410,10 @@ typedef struct zen_cuda_pick_segment {
     uint32_t reserved;
 } zen_cuda_pick_segment;
 int zen_cuda_dev_greedy_pick(const zen_cuda_pick_segment* segments, size_t count, size_t tokens, int64_t* d_pick, void* stream);
+/* The same, and the first row's pick once more at note[*d_position % notes] (note: page-locked host memory, or null): a host that waits
+ * for an event behind the launch then has the token without a copy in the stream. */
+int zen_cuda_dev_greedy_pick_noted(const zen_cuda_pick_segment* segments, size_t count, size_t tokens, int64_t* d_pick, int64_t* note, size_t notes,
+                                   const int32_t* d_position, void* stream);
 
 /* Temperature / top-k / top-p sampling on the device: the non-greedy branch of the reference's sampler
  * (sampling_distribution + sample_distribution, src/adapters/dense_transformer_runtime.cpp:349-390).  Among the finite

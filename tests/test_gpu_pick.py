@@ -206,3 +206,24 @@ def test_sampling_ties_and_degenerate_rows(be):
     from zeninfer_b200 import BackendError
     with pytest.raises(BackendError):
         be.dev_sample(d_flat.data_ptr(), 4000, 0.0, 0, 0.9, 0.5, d_pick.data_ptr(), 0)     # temperature must be positive
+
+
+def test_a_noted_pick_is_in_host_memory_behind_the_launch(be, zo):
+    import torch
+    from zeninfer_b200.backend import BackendError
+    rng = np.random.default_rng(5)
+    pick, pos, notes = torch.zeros(1, dtype=torch.int64, device="cuda"), torch.zeros(1, dtype=torch.int32, device="cuda"), torch.full((3,), -7, dtype=torch.int64).pin_memory()
+    want = [-7, -7, -7]
+    for position in (0, 1, 5, 2_000_000_000):
+        row = rng.standard_normal((1, 5000)).astype(np.float32)
+        d = torch.from_numpy(row).cuda()
+        pos.fill_(position)
+        torch.cuda.synchronize()
+        be.dev_greedy_pick([(d.data_ptr(), 5000, 0, 5000)], 1, pick.data_ptr(), 0, note=(notes.data_ptr(), 3, pos.data_ptr()))
+        be.dev_check()
+        want[position % 3] = int(oracle_pick(zo, row)[0])
+        assert int(pick) == want[position % 3] and notes.tolist() == want
+    with pytest.raises(BackendError):
+        be.dev_greedy_pick([(d.data_ptr(), 5000, 0, 5000)], 1, pick.data_ptr(), 0, note=(notes.data_ptr(), 3, 0))      # no position
+    with pytest.raises(BackendError):
+        be.dev_greedy_pick([(d.data_ptr(), 5000, 0, 5000)], 1, pick.data_ptr(), 0, note=(notes.data_ptr(), 0, pos.data_ptr()))

@@ -42,7 +42,7 @@ ABI_SYMBOLS = (
     "zen_cuda_dev_gemm_q8_0_noalloc",
     "zen_cuda_gather_region_bytes", "zen_cuda_ipc_alloc", "zen_cuda_ipc_open", "zen_cuda_ipc_close", "zen_cuda_ipc_free",
     "zen_cuda_gather_create", "zen_cuda_gather_destroy", "zen_cuda_dev_gemv_gather", "zen_cuda_dev_gather_fetch", "zen_cuda_dev_allgather", "zen_cuda_dev_allreduce_add",
-    "zen_cuda_dev_greedy_pick", "zen_cuda_dev_sample",
+    "zen_cuda_dev_greedy_pick", "zen_cuda_dev_greedy_pick_noted", "zen_cuda_dev_sample",
     "zen_cuda_dev_embed_q8_0", "zen_cuda_dev_rms_norm", "zen_cuda_dev_rope_kv_append", "zen_cuda_dev_attention", "zen_cuda_dev_silu_mul",
     "zen_cuda_dev_advance_position", "zen_cuda_dev_gemv_swiglu", "zen_cuda_dev_attention_block", "zen_cuda_dev_gemv_fused",
     "zen_cuda_dev_embed_rows_q8_0", "zen_cuda_dev_rope_kv_append_rows", "zen_cuda_dev_attention_prefill",
@@ -208,6 +208,7 @@ def load_library(path: str | None = None) -> C.CDLL:
     lib.zen_cuda_dev_allgather.argtypes = [vp, vp, sz, vp, vp]
     lib.zen_cuda_dev_allreduce_add.argtypes = [vp, vp, sz, vp, vp]
     lib.zen_cuda_dev_greedy_pick.argtypes = [C.POINTER(PickSegment), sz, sz, vp, vp]
+    lib.zen_cuda_dev_greedy_pick_noted.argtypes = [C.POINTER(PickSegment), sz, sz, vp, vp, sz, vp, vp]
     lib.zen_cuda_dev_sample.argtypes = [vp, sz, C.c_float, C.c_uint32, C.c_float, C.c_double, vp, vp, vp, vp, vp, vp]
     lib.zen_cuda_dev_embed_q8_0.argtypes = [vp, vp, vp, vp]
     lib.zen_cuda_dev_rms_norm.argtypes = [vp, vp, vp, vp, sz, sz, C.c_float, vp]
@@ -564,12 +565,14 @@ class Backend:
         if not self.lib.zen_cuda_dev_quantize_acts(d_x, d_codes, d_scales, tokens, columns, stream):
             self._fail("dev_quantize_acts")
 
-    def dev_greedy_pick(self, segments: Sequence[tuple[int, int, int, int]], tokens: int, d_pick: int, stream: int = 0) -> None:
+    def dev_greedy_pick(self, segments: Sequence[tuple[int, int, int, int]], tokens: int, d_pick: int, stream: int = 0, *,
+                        note: tuple[int, int, int] | None = None) -> None:
         """Greedy token pick (first maximum among finite logits, -1 if none) into device int64 [tokens].  A segment is
-        (device address of token 0's first entry, entries per token, index of the first entry, floats between tokens)."""
+        (device address of token 0's first entry, entries per token, index of the first entry, floats between tokens).  note:
+        (page-locked host int64 [n], n, device int32 position): the first row's pick also goes to entry position % n."""
         n = len(segments)
         segs = (PickSegment * n)(*[PickSegment(b, ln, first, stride, 0) for b, ln, first, stride in segments])
-        if not self.lib.zen_cuda_dev_greedy_pick(segs, n, tokens, d_pick, stream):
+        if not self.lib.zen_cuda_dev_greedy_pick_noted(segs, n, tokens, d_pick, *(note or (None, 0, None)), stream):
             self._fail("dev_greedy_pick")
 
     SAMPLE_MAX_CANDIDATES = 1024

@@ -40,6 +40,11 @@ struct PickParams {
     PickSegment seg[kPickMaxSegments];
     uint32_t nseg;
     long long* pick;           // [tokens]
+    // Row 0's pick once more, at note[*position % notes]: host memory the device can write, read by a host that waits for an event
+    // behind the launch.  null: none.
+    long long* note;
+    const int* position;
+    uint32_t notes;
 };
 
 __device__ __forceinline__ unsigned long long pick_key(float v, uint32_t index) {
@@ -96,7 +101,9 @@ __global__ void __cluster_dims__(kPickCtas, 1, 1) __launch_bounds__(kPickThreads
     cluster.sync();
     if (blockIdx.x == 0 && threadIdx.x == 0) {
         for (uint32_t c = 0; c < kPickCtas; ++c) best = cta_best[c] > best ? cta_best[c] : best;
-        p.pick[blockIdx.y] = best ? static_cast<long long>(0xffffffffu - static_cast<uint32_t>(best)) : -1ll;
+        const long long pick = best ? static_cast<long long>(0xffffffffu - static_cast<uint32_t>(best)) : -1ll;
+        p.pick[blockIdx.y] = pick;
+        if (p.note && blockIdx.y == 0) p.note[static_cast<uint32_t>(*reinterpret_cast<const volatile int*>(p.position)) % p.notes] = pick;
     }
 }
 

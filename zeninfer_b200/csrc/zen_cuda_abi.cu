@@ -2496,11 +2496,18 @@ int zen_cuda_dev_allreduce_add(zen_cuda_gather* g, const float* d_partial, size_
 }
 
 int zen_cuda_dev_greedy_pick(const zen_cuda_pick_segment* segments, size_t count, size_t tokens, int64_t* d_pick, void* stream) {
+    return zen_cuda_dev_greedy_pick_noted(segments, count, tokens, d_pick, nullptr, 0, nullptr, stream);
+}
+
+int zen_cuda_dev_greedy_pick_noted(const zen_cuda_pick_segment* segments, size_t count, size_t tokens, int64_t* d_pick, int64_t* note, size_t notes,
+                                   const int32_t* d_position, void* stream) {
     State& s = state();
     std::lock_guard<std::mutex> lock(s.mutex);
     if (!init_locked(s)) return 0;
-    if (!segments || !count || count > zk::kPickMaxSegments || !tokens || tokens > 65535 || !d_pick) return set_error(s, "dev_greedy_pick: bad arguments") ? 1 : 0;
+    if (!segments || !count || count > zk::kPickMaxSegments || !tokens || tokens > 65535 || !d_pick || (note && (!notes || notes > 0xffffffffu || !d_position)))
+        return set_error(s, "dev_greedy_pick: bad arguments") ? 1 : 0;
     zk::PickParams p{};
+    p.note = reinterpret_cast<long long*>(note); p.notes = static_cast<uint32_t>(notes); p.position = d_position;
     for (size_t i = 0; i < count; ++i) {
         if (!segments[i].base && segments[i].len) return set_error(s, "dev_greedy_pick: null segment") ? 1 : 0;
         if (static_cast<uint64_t>(segments[i].first_index) + segments[i].len > 0xffffffffull) return set_error(s, "dev_greedy_pick: index range too large") ? 1 : 0;

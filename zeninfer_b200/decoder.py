@@ -39,6 +39,7 @@ class SequenceState:
 
 
 class Decoder:
+    NOTES = 8               # picks in host memory, by position: more than a run has in flight
     PREFILL_CHUNK = 512     # tokens per block (buffers are sized for it)
     PREFILL_MIN = 16        # shorter blocks go token by token
     rank, world, group = 0, 1, None
@@ -54,6 +55,8 @@ class Decoder:
         self.pos = torch.zeros(1, dtype=torch.int32, device=self.dev)
         self.token = torch.zeros(1, dtype=torch.int64, device=self.dev)
         self.host_token = torch.zeros(1, dtype=torch.int64).pin_memory()   # a caller's callback sees a token before the host feeds it to the next step
+        self.notes = torch.zeros(self.NOTES, dtype=torch.int64).pin_memory()
+        self.noted = self.notes.numpy()
         self.picks = [(torch.zeros(1, dtype=torch.int64).pin_memory(), torch.cuda.Event()) for _ in range(2)]   # read-outs in flight, with what to wait for
         self.graph_layers = self.graph_step = None
         self.fed = 0            # tokens feed() has taken since the last reset
@@ -186,6 +189,11 @@ class Decoder:
                 last = i + 1 == len(prompt)
                 self._prompt_token(last)
 
+    def _pick(self) -> None:
+        """The greedy pick of self.logits into self.token, noted in host memory under the position it is for."""
+        self.be.dev_greedy_pick([(self.logits.data_ptr(), self.vocab, 0, self.vocab)], 1, self.token.data_ptr(), self.stream.cuda_stream,
+                                note=(self.notes.data_ptr(), self.NOTES, self.pos.data_ptr()))
+
     def _sample(self, temperature: float, top_k: int, top_p: float, u: float) -> None:
         """Replaces the greedy pick in self.token by a draw from the filtered distribution of self.logits."""
         self.be.dev_sample(self.logits.data_ptr(), self.vocab, temperature, top_k, top_p, u, self.token.data_ptr(), self.stream.cuda_stream)
@@ -201,7 +209,9 @@ class Decoder:
         With a callback, and on several GPUs, the host has each token before the next step begins and feeds it back from its
         side, as the reference's loop does.  Otherwise nothing a step needs passes through the host (its token is where the
         pick or the draw left it), so a step is launched before the token of the one before is read: the round trip to the
-        host runs beside the next step (B200, four layers of width 1024: 139 us a token, 160 with it between the steps).
+        host runs beside the next step (B200, four layers of width 1024: 139 us a token, 160 with it between the steps).  A greedy
+        pick is written to host memory by the kernel that makes it: a copy in the stream stood between the steps' graphs for 12 to
+        15 us a token.
         Raises when the context would overflow."""
         torch = self.torch
         if not prompt or len(prompt) + max_new > self.max_positions:
@@ -213,12 +223,14 @@ class Decoder:
         with torch.cuda.stream(self.stream):
             self.feed_prompt(prompt, batched_prefill)
             ahead = on_token is None and self.world == 1
+            noted = ahead and rng is None
 
             def draw_and_send(n: int) -> None:
                 if rng is not None:               # the step left the greedy pick in self.token: draw instead
                     self._sample(temperature, top_k, top_p, float(rng.random()))
                 host, sent = self.picks[n % 2]
-                host.copy_(self.token, non_blocking=True)
+                if not noted:
+                    host.copy_(self.token, non_blocking=True)
                 sent.record(self.stream)
 
             if max_new > 0:
@@ -229,7 +241,7 @@ class Decoder:
                     draw_and_send(n + 1)
                 host, sent = self.picks[n % 2]
                 sent.synchronize()                # device -> host read of the step's result
-                tok = int(host[0])
+                tok = int(self.noted[(len(prompt) + n) % self.NOTES]) if noted else int(host[0])
                 out.append(tok)
                 if on_token:
                     on_token(tok)

@@ -270,7 +270,7 @@ class KipiraxDecoder(DenseDecoder):
     def _enqueue_head(self) -> None:
         st = self.stream.cuda_stream
         self.be.dev_dense_gemv([(self.head, None, self.logits.data_ptr())], st, pre=self._end(self.pending, out_norm=self.final_norm), **self._logit_act())
-        self.be.dev_greedy_pick([(self.logits.data_ptr(), self.vocab, 0, self.vocab)], 1, self.token.data_ptr(), st)
+        self._pick()
 
     # ---- a block of tokens ----
     def _prefill_buffers(self) -> dict:

@@ -278,7 +278,7 @@ class LlamaDecoder(Decoder):
         self._gemv([self.h["output.weight"]], [self.logits_mine.data_ptr()], self.x.data_ptr() if fn else self.xn.data_ptr(),
                    norm=self.norm["output_norm.weight"].data_ptr() if fn else None, warm=self.h["blk.0.attn_q.weight"])
         self._gather(self.logits, self.logits_mine)
-        self.be.dev_greedy_pick([(self.logits.data_ptr(), self.cfg.vocab, 0, self.cfg.vocab)], 1, self.token.data_ptr(), self.stream.cuda_stream)
+        self._pick()
 
     # ---- prefill: a block of prompt tokens through the tensor-core products ----
     def _prefill_buffers(self):
