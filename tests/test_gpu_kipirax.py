@@ -92,6 +92,13 @@ def test_dense_gemm(be, rows, cols, tokens, exact):
     be.dev_free(h)
 
 
+# A tile is stored in chunks of 32 tokens, whole ones and the last one's rest by different loops, by two warps in turn.
+@pytest.mark.parametrize("rows", [130, 20000])
+@pytest.mark.parametrize("tokens", [31, 32, 34, 64, 65, 96, 127, 161, 256])
+def test_dense_gemm_chunks_of_tokens(be, rows, tokens):
+    test_dense_gemm(be, rows, 40, tokens, False)
+
+
 def test_products_refuse_bad_arguments(be):
     h, _ = bf16_matrix(be, 16, 24, 0)
     y = zeros(64)

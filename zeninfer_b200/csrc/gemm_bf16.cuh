@@ -1,9 +1,9 @@
 // Products of bfloat16 matrices with a block of tokens.
 //
 // gemm_bf16_kernel: tcgen05.mma kind::f16, bf16 x bf16 -> fp32.  Weight rows are M (128 per tile), tokens are N (kNTile), so that
-// a TMEM lane is a weight row and consecutive lanes store consecutive outputs of one token.  One persistent CTA per SM, six warps:
+// a TMEM lane is a weight row and consecutive lanes store consecutive outputs of one token.  One persistent CTA per SM, ten warps:
 // TMA producer (64 columns of K per stage: 128 x 128 B of weights and kNTile x 128 B of activations, 128-byte swizzle), MMA issuer,
-// four epilogue warps; two accumulators in TMEM, so the epilogue of a tile runs under the next tile's products.  K and rows that
+// eight epilogue warps; two accumulators in TMEM, so the epilogue of a tile runs under the next tile's products.  K and rows that
 // do not fill a tile arrive as zeros from the tensor maps.  The first 2 pairs rows may be (gate, up) pairs that leave as
 // silu(gate) * up: neighbouring TMEM lanes, exchanged between lanes of the epilogue warp.
 //
@@ -17,7 +17,8 @@
 namespace zk {
 
 constexpr int kBgM = 128, kBgK = 64;                       // tile rows; K columns per stage (128 bytes)
-constexpr int kBgThreads = 6 * 32;
+constexpr int kBgEpilogueWarps = 8;
+constexpr int kBgThreads = (2 + kBgEpilogueWarps) * 32;
 constexpr uint32_t kBgABytes = kBgM * kBgK * 2;
 
 struct GemmBf16Params {
@@ -32,6 +33,48 @@ struct GemmBf16Params {
     float cap;
     int* error_word;
 };
+
+// Stores a lane's row r of 32 tokens from t0 on.  What is the same for all of them (the kind of output, its activation, whether all 32
+// are there) is decided once, and eight warps share a tile: decided for every value, by four warps, the stores of a 128 x 256 tile took
+// 27 us, longer than its products up to 8192 columns.  Launches back to back on a B200, before and now: 8192 x 2048 times 512 tokens
+// 40.4 and 16.7 us (14.7 with no stores at all), 9728 x 1024 times 512 60.0 and 17.4, 45056 x 4096 times 512 188.7 and 156.8.
+template <typename T, typename F>
+__device__ __forceinline__ void gemm_bf16_column(T* out, uint32_t ld, const uint32_t (&v)[32], uint32_t count, F f) {
+    if (count >= 32) {
+#pragma unroll
+        for (int c = 0; c < 32; ++c) out[static_cast<size_t>(c) * ld] = static_cast<T>(f(__uint_as_float(v[c])));
+    } else {
+#pragma unroll
+        for (int c = 0; c < 32; ++c)
+            if (c < static_cast<int>(count)) out[static_cast<size_t>(c) * ld] = static_cast<T>(f(__uint_as_float(v[c])));
+    }
+}
+__device__ __forceinline__ void gemm_bf16_store(const GemmBf16Params& p, const uint32_t (&v)[32], uint32_t r, uint32_t t0, uint32_t lane, float bias) {
+    const uint32_t paired = 2 * p.pairs;
+    if (t0 >= p.tokens) return;
+    const uint32_t count = p.tokens - t0;
+    if (r - lane < paired) {                           // some of the warp's rows are pairs: an even lane takes one token, its partner the next
+        const bool odd = lane & 1;
+        __nv_bfloat16* to = p.gated + static_cast<size_t>(t0 + (odd ? 1u : 0u)) * p.gated_ld + r / 2;
+#pragma unroll
+        for (int c = 0; c < 32; c += 2) {
+            const float keep = __uint_as_float(odd ? v[c + 1] : v[c]);
+            const float other = __shfl_xor_sync(0xffffffffu, __uint_as_float(odd ? v[c] : v[c + 1]), 1);
+            const float gate = odd ? other : keep, up = odd ? keep : other;
+            if (r < paired && c + (odd ? 1u : 0u) < count) to[static_cast<size_t>(c) * p.gated_ld] = __float2bfloat16_rn(silu_f(gate) * up);
+        }
+    }
+    if (r >= paired && r < p.rows) {
+        const size_t at = static_cast<size_t>(t0) * p.out_ld + (r - paired);
+        auto with = [&](auto f) {
+            if (p.out) gemm_bf16_column(p.out + at, p.out_ld, v, count, f);
+            else gemm_bf16_column(p.out_bf16 + at, p.out_ld, v, count, [&](float y) { return __float2bfloat16_rn(f(y)); });
+        };
+        if (p.act == kActNone) with([&](float y) { return y + bias; });
+        else if (p.act == kActSquaredRelu) with([&](float y) { return dense_activation(y + bias, kActSquaredRelu, 0.0f); });
+        else with([&](float y) { return dense_activation(y + bias, kActSoftcap, p.cap); });
+    }
+}
 
 template <int kNTile>
 __host__ __device__ constexpr int gemm_bf16_stages() { return kNTile == 256 ? 4 : kNTile == 128 ? 6 : 8; }
@@ -56,7 +99,7 @@ __global__ void __launch_bounds__(kBgThreads, 1) gemm_bf16_kernel(const __grid_c
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     if (threadIdx.x == 0) {
         for (int s = 0; s < kStages; ++s) { mbar_init(&full[s], 1); mbar_init(&empty[s], 1); }
-        for (int b = 0; b < 2; ++b) { mbar_init(&tmem_full[b], 1); mbar_init(&tmem_empty[b], 4); }
+        for (int b = 0; b < 2; ++b) { mbar_init(&tmem_full[b], 1); mbar_init(&tmem_empty[b], kBgEpilogueWarps); }
         *abort_word = 0;
         mbar_fence_init();
         tma_prefetch_descriptor(&p.map_w);
@@ -124,6 +167,12 @@ __global__ void __launch_bounds__(kBgThreads, 1) gemm_bf16_kernel(const __grid_c
         }
     } else {
         const uint32_t quad = static_cast<uint32_t>(warp) & 3;     // the TMEM lanes a warp may touch: 32 * (warp id % 4)
+        const uint32_t half = static_cast<uint32_t>(warp - 2) >> 2;   // two warps to a quad, 32 columns by turns
+        auto release = [&](uint32_t set) {                          // the warp's sums are in registers
+            tc_fence_before_sync();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&tmem_empty[set]);
+        };
         uint32_t count = 0;
         pdl_wait();                                                // the outputs may still be read by an earlier launch
         for (uint32_t tile = blockIdx.x; tile < tiles; tile += gridDim.x, ++count) {
@@ -134,40 +183,14 @@ __global__ void __launch_bounds__(kBgThreads, 1) gemm_bf16_kernel(const __grid_c
                 break;
             }
             tc_fence_after_sync();
-            constexpr int kChunk = kNTile < 32 ? 16 : 32;
-#pragma unroll 1
-            for (uint32_t c0 = 0; c0 < static_cast<uint32_t>(kNTile); c0 += kChunk) {
-                uint32_t v[kChunk];
-                const uint32_t addr = tmem_base + set * kNTile + c0 + ((quad * 32) << 16);
-                if constexpr (kChunk == 32) tmem_ld_32x32(addr, v); else tmem_ld_32x16(addr, v);
+            uint32_t v[32];
+            for (uint32_t c0 = half * 32; c0 < static_cast<uint32_t>(kNTile); c0 += 64) {
+                tmem_ld_32x32(tmem_base + set * kNTile + c0 + ((quad * 32) << 16), v);
                 tmem_ld_wait();
-                if (c0 + kChunk == static_cast<uint32_t>(kNTile)) {
-                    tc_fence_before_sync();
-                    __syncwarp();
-                    if (lane == 0) mbar_arrive(&tmem_empty[set]);
-                }
-                if (r - lane < paired) {                           // some of the warp's rows are pairs: an even lane takes one token, its partner the next
-                    const bool odd = lane & 1;
-#pragma unroll
-                    for (int c = 0; c < kChunk; c += 2) {
-                        const float keep = __uint_as_float(odd ? v[c + 1] : v[c]);
-                        const float other = __shfl_xor_sync(0xffffffffu, __uint_as_float(odd ? v[c] : v[c + 1]), 1);
-                        const uint32_t t = n0 + c0 + c + (odd ? 1u : 0u);
-                        if (r < paired && t < p.tokens) p.gated[static_cast<size_t>(t) * p.gated_ld + r / 2] = __float2bfloat16_rn(odd ? silu_f(other) * keep : silu_f(keep) * other);
-                    }
-                }
-                if (r >= paired && r < p.rows) {
-#pragma unroll
-                    for (int c = 0; c < kChunk; ++c) {
-                        const uint32_t t = n0 + c0 + c;
-                        if (t < p.tokens) {
-                            const float y = dense_activation(__uint_as_float(v[c]) + bias, p.act, p.cap);
-                            const size_t at = static_cast<size_t>(t) * p.out_ld + (r - paired);
-                            if (p.out) p.out[at] = y; else p.out_bf16[at] = __float2bfloat16_rn(y);
-                        }
-                    }
-                }
+                if (c0 + 64 >= static_cast<uint32_t>(kNTile)) release(set);
+                gemm_bf16_store(p, v, r, n0 + c0, lane, bias);
             }
+            if (half * 32 >= static_cast<uint32_t>(kNTile)) release(set);
         }
     }
     tc_fence_before_sync();
