@@ -248,6 +248,23 @@ def test_bad_arguments_are_errors(be):
     assert be.stats()["fallbacks"] >= 1
 
 
+# One token's input is read three passes of 4096 columns ahead: less than a pass, whole ones, one block more, more passes than are ahead.
+@pytest.mark.parametrize("rows,cols", [(40, 2080), (40, 4096), (33, 4128), (40, 8192), (7, 8224), (33, 12320), (300, 16384), (5, 16416), (33, 20512)])
+@pytest.mark.parametrize("mode,int8", [(ACT_INT8, True), (ACT_FP32, False)])
+def test_gemv_of_long_inputs(be, zo, mode, int8, rows, cols):
+    w = seeded_weights(Q8_0, rows, cols, 50 + rows)
+    x = seeded_acts(1, cols, 60 + cols)[0]
+    be.set_q8_act_mode(mode)
+    y = be.gemv("Q8_0", w, x, rows, cols)
+    be.release_weights(w)
+    be.set_q8_act_mode(ACT_INT8)
+    ref = ref_int8_f64(w, *zo.quantise_acts(x[None]), rows, cols) if int8 else ref_fp32_f64(Q8_0, w, x, rows, cols)
+    rel = assert_parity(y, ref[0], what=f"long input {rows}x{cols}")
+    # a sum of up to 641 blocks is at most 21 additions of a lane and 5 across lanes, 2^-24 of the magnitudes' sum each, and that sum is
+    # some ten times the largest result
+    assert rel < (26 * 2.0 ** -24 * 10 if int8 else 1e-4)
+
+
 @pytest.mark.parametrize("rows,cols", [(4096, 14336), (1027, 4128), (300, 8192), (77, 12288), (5, 4128), (33, 14336)])
 def test_rows_of_several_segments_int8(be, zo, rows, cols):
     # more than 4096 columns, one int8 token: a warp walks two rows segment by segment with the segment's activations in
