@@ -99,6 +99,12 @@ def test_dense_gemm_chunks_of_tokens(be, rows, tokens):
     test_dense_gemm(be, rows, 40, tokens, False)
 
 
+# Every width of a tile (32 to 256 tokens) is the one of fewest bytes for some of these, with a last tile that is full, short or of one token.
+@pytest.mark.parametrize("rows,tokens", [(20000, 17), (20000, 70), (20000, 96), (20000, 150), (20000, 161), (20000, 192), (20000, 301), (4100, 300), (4100, 193), (2049, 481), (9728, 512), (45056, 301)])
+def test_dense_gemm_tile_widths(be, rows, tokens):
+    test_dense_gemm(be, rows, 72, tokens, False)
+
+
 def test_products_refuse_bad_arguments(be):
     h, _ = bf16_matrix(be, 16, 24, 0)
     y = zeros(64)

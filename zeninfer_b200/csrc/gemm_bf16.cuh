@@ -1,6 +1,6 @@
 // Products of bfloat16 matrices with a block of tokens.
 //
-// gemm_bf16_kernel: tcgen05.mma kind::f16, bf16 x bf16 -> fp32.  Weight rows are M (128 per tile), tokens are N (kNTile), so that
+// gemm_bf16_kernel: tcgen05.mma kind::f16, bf16 x bf16 -> fp32.  Weight rows are M (128 per tile), tokens are N (kNTile, 32 to 256), so that
 // a TMEM lane is a weight row and consecutive lanes store consecutive outputs of one token.  One persistent CTA per SM, ten warps:
 // TMA producer (64 columns of K per stage: 128 x 128 B of weights and kNTile x 128 B of activations, 128-byte swizzle), MMA issuer,
 // eight epilogue warps; two accumulators in TMEM, so the epilogue of a tile runs under the next tile's products.  K and rows that
@@ -77,9 +77,9 @@ __device__ __forceinline__ void gemm_bf16_store(const GemmBf16Params& p, const u
 }
 
 template <int kNTile>
-__host__ __device__ constexpr int gemm_bf16_stages() { return kNTile == 256 ? 4 : kNTile == 128 ? 6 : 8; }
-template <int kNTile>
 __host__ __device__ constexpr uint32_t gemm_bf16_stage_bytes() { return kBgABytes + kNTile * kBgK * 2; }
+template <int kNTile>      // up to 216 KB of them
+__host__ __device__ constexpr int gemm_bf16_stages() { return kNTile == 256 ? 4 : kNTile == 192 ? 5 : kNTile >= 128 ? 6 : kNTile == 96 ? 7 : 8; }
 template <int kNTile>
 __host__ __device__ constexpr uint32_t gemm_bf16_smem_bytes() { return 1024 + gemm_bf16_stages<kNTile>() * gemm_bf16_stage_bytes<kNTile>() + 256; }
 
@@ -87,7 +87,7 @@ template <int kNTile>
 __global__ void __launch_bounds__(kBgThreads, 1) gemm_bf16_kernel(const __grid_constant__ GemmBf16Params p) {
     constexpr int kStages = gemm_bf16_stages<kNTile>();
     constexpr uint32_t kStageBytes = gemm_bf16_stage_bytes<kNTile>();
-    constexpr uint32_t kTmemCols = 2 * kNTile < 32 ? 32 : 2 * kNTile;
+    constexpr uint32_t kTmemCols = kNTile > 128 ? 512 : kNTile > 64 ? 256 : 2 * kNTile;      // two accumulators, a power of two
     extern __shared__ uint8_t bg_smem_raw[];
     uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(bg_smem_raw) + 1023) & ~static_cast<uintptr_t>(1023));
     uint64_t* full = reinterpret_cast<uint64_t*>(smem + kStages * kStageBytes);

@@ -249,10 +249,13 @@ int zen_cuda_dev_dense_gemm(const zen_cuda_weights* w, const void* d_x, size_t x
     p.m_tiles = u32((w->rows + zk::kBgM - 1) / zk::kBgM);
     p.act = ep.act; p.cap = ep.cap; p.bias = ep.d_bias; p.error_word = e.d_error;
     p.gated = static_cast<__nv_bfloat16*>(ep.d_gated); p.gated_ld = u32(ep.gated_ld); p.pairs = u32(ep.gated_pairs);
-    // the tile width that moves the fewest operand bytes through the busiest SM
+    // The tile width that moves the fewest operand bytes through the busiest SM.  B200, us with tiles of 256 / 192 / 160 / 128 / 96 / 64 tokens:
+    // 45056 x 4096 times 301 tokens 139.4 / 122.8 / 117.7 / 165.6 / 204.6 / 238.3 (160 taken), times 512 156.4 / 186.9 / 214.9 / 208.6 / 303.5 / 391.9
+    // (256), 38912 x 4096 times 301 131.2 / 115.6 / 110.9 / 145.7 / 184.6 / 218.4 (160; with powers of two alone 145.7), 4096 x 18432 times 301
+    // 106.6 / 94.9 / 95.7 / 97.2 / 94.5 / 177.2 (96), 9728 x 1024 times 512 17.4 / 17.0 / 20.9 / 20.5 / 25.4 / 29.3 (192).
     int best = 0;
     uint64_t best_cost = ~0ull;
-    for (int n : {256, 128, 64, 32}) {
+    for (int n : {256, 192, 160, 128, 96, 64, 32}) {
         const uint64_t tiles = static_cast<uint64_t>(p.m_tiles) * ((tokens + n - 1) / n), waves = (tiles + e.sm_count - 1) / e.sm_count;
         const uint64_t cost = waves * static_cast<uint64_t>(zk::kBgM + n);
         if (cost < best_cost) { best_cost = cost; best = n; }
@@ -261,7 +264,13 @@ int zen_cuda_dev_dense_gemm(const zen_cuda_weights* w, const void* d_x, size_t x
     // the matrix's padding columns are zeros, so the maps may end at the pitch; x is read up to its real columns only
     if (!map_bf16(e, &p.map_w, w->plane[0], w->nbp, w->rows, w->nbp, zk::kBgM) || !map_bf16(e, &p.map_x, d_x, w->cols, tokens, x_ld, u32(best)))
         return e.fail("dense_gemm: cuTensorMapEncodeTiled failed");
-    const cudaError_t r = best == 256 ? launch_gemm<256>(e, p) : best == 128 ? launch_gemm<128>(e, p) : best == 64 ? launch_gemm<64>(e, p) : launch_gemm<32>(e, p);
+    const cudaError_t r = best == 256   ? launch_gemm<256>(e, p)
+                          : best == 192 ? launch_gemm<192>(e, p)
+                          : best == 160 ? launch_gemm<160>(e, p)
+                          : best == 128 ? launch_gemm<128>(e, p)
+                          : best == 96  ? launch_gemm<96>(e, p)
+                          : best == 64  ? launch_gemm<64>(e, p)
+                                        : launch_gemm<32>(e, p);
     return e.leave(r, "dense_gemm");
 }
 
