@@ -35,3 +35,14 @@ def test_what_the_launch_in_front_writes_is_read_coherently(name, kernel, argume
     for start in [argument, *made]:
         assert not re.search(rf"\*{start}\b(?!\*)|\b{start}\[|\*reinterpret_cast<const float4\*>\({start}\b", body), f"{kernel}: plain load of {start}"
     assert re.search(rf"__ldcg\((?:reinterpret_cast<const float4\*>\()?(?:{'|'.join([argument, *made])})\b", body)
+
+
+def test_a_decode_product_reads_only_weights_before_the_launch_in_front_has_ended():
+    """Bias, norm weights, shift and output norm may be what the launch in front writes: up to the wait they are asked into L2 at most."""
+    text = _source("gemv_bf16.cuh")
+    body = text[text.index("gemv_bf16_kernel("):]
+    before = body[:body.index("pdl_wait();")]
+    assert not re.search(r"__ldg|__ldcg|row_words\(|sublayer_", before), "loads in front of the wait"
+    for called in set(re.findall(r"\b(prologue_\w+)\(", before)):
+        of = text[text.index(called + "("):]
+        assert not re.search(r"__ldg|__ldcg|row_words\(", of[:of.index("\n}\n")]), f"{called}: loads in front of the wait"

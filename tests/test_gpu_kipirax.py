@@ -195,6 +195,36 @@ def test_sublayer_end_in_a_product_of_words_that_are_not_aligned(be):
     be.dev_free(h)
 
 
+# A product of few rows, whose successor starts on the idle SMs at once, writes a vector that the successor reads: its bias, a norm
+# weight, a shift, an output norm.  Equal to the pair with a synchronisation between.
+@pytest.mark.parametrize("n", [64, 90])          # the prologue with the row in registers, and without
+@pytest.mark.parametrize("what", ["bias", "norm_weight", "shift", "out_norm", "weight_a"])
+def test_a_product_reads_what_the_launch_in_front_wrote(be, what, n):
+    import torch
+    a, d, end, x_out, keep, _, _ = sublayer_case(n, 1, 2, True, {"shift": "shift", "out_norm": "norm"}.get(what, "plain"), seed=n)
+    long = 18432
+    first, w1 = bf16_matrix(be, n, long, 1)
+    second, w2 = bf16_matrix(be, n, n, 2)
+    made, y = zeros(n), zeros(n)
+    if what != "bias":
+        setattr(end, what, made.data_ptr())
+    stream = torch.cuda.Stream()
+    for seed in range(8):
+        dx = dev(np.random.default_rng(seed).standard_normal(long))
+        got = []
+        for apart in (True, False):
+            made.fill_(1e6)
+            torch.cuda.synchronize()
+            be.dev_dense_gemv([(first, dx.data_ptr(), made.data_ptr())], stream.cuda_stream)
+            if apart:
+                stream.synchronize()
+            be.dev_dense_gemv([(second, None, y.data_ptr())], stream.cuda_stream, pre=end, bias=made.data_ptr() if what == "bias" else None)
+            got.append(host(y).copy())
+        assert np.array_equal(got[0], got[1]) and np.abs(got[0]).max() < 1e5
+    be.dev_free(first)
+    be.dev_free(second)
+
+
 def test_embedding_rows(be):
     import torch
     c, _, bits, w = cases.model("ragged")

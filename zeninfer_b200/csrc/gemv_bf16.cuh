@@ -10,6 +10,9 @@
 //     9.0 -> 8.1, against sixteen warps that held two steps in registers (128 KB).  More in flight is slower (five steps: 58.6),
 //     sixteen warps too (58.9), and so is a CTA small enough to have the next launch's beside it: the SMs that finish first then
 //     take two of those each, and the pair above goes from 82.7 to 97.8;
+//   * nothing else is read before the previous grid has finished, because it may be what that grid writes (a residual as the bias, a
+//     norm weight or shift made per token).  The vectors among it that seldom are, bias, norm weights and shift, are only asked
+//     into L2 by then, so that they need not come from HBM later;
 //   * the prologue can finish the sublayer before it (row_ops.cuh: grouped norm, residual add, token shift or output norm), so
 //     a decode step needs no launches for them: every CTA forms the input vector itself, CTA 0 stores the residual stream;
 //   * the epilogue adds a bias and applies the product's activation (squared ReLU, or the logits' soft cap) in fp32; a matrix may
@@ -87,8 +90,7 @@ __device__ __forceinline__ void dense_copy(uint32_t dst, const void* src, bool r
 }
 
 // The prologue of rows of up to 4096 values (a multiple of 32, in 1, 2, 4 or 8 parts, every array 16-byte aligned), formed as
-// sublayer_row and sublayer_view form it: a warp holds an eighth of the row in registers, all arrays are asked for at once, and the
-// constants among them (norm weights, shift) before the previous grid has finished, when they may still have to come from HBM.
+// sublayer_row and sublayer_view form it: a warp holds an eighth of the row in registers and all arrays are asked for at once.
 // row_ops.cuh's functions go over the row in shared memory three to five times with a barrier after each.
 struct RowWords { float4 v[kPreQuads]; };
 __device__ __forceinline__ void row_words(RowWords& r, const float* src, uint32_t first, uint32_t chunk, uint32_t lane) {
@@ -115,14 +117,21 @@ template <typename F> __device__ __forceinline__ void row_each(RowWords& r, F f)
 }
 __device__ __forceinline__ float row_at(const RowWords& r, int q, int c) { return c == 0 ? r.v[q].x : c == 1 ? r.v[q].y : c == 2 ? r.v[q].z : r.v[q].w; }
 
-struct PrologueConstants { RowWords norm, post; };      // norm_weight; shift or out_norm
-__device__ __forceinline__ void prologue_constants(PrologueConstants& c, const SublayerEnd& p) {
+__device__ __forceinline__ const float* prologue_post(const SublayerEnd& p) { return p.shift ? p.shift : p.out_norm; }
+// Asks norm weights and shift into L2: no value is read, so this may go in front of the wait.
+__device__ __forceinline__ void prologue_prefetch(const SublayerEnd& p) {
     const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31, chunk = p.n / kDenseWarps;
-    row_words(c.norm, p.norm_weight, warp * chunk, chunk, lane);
-    row_words(c.post, p.shift ? p.shift : p.out_norm, warp * chunk, chunk, lane);
+    const float* const post = prologue_post(p);
+#pragma unroll
+    for (int q = 0; q < kPreQuads; ++q) {
+        const uint32_t i = 4 * (lane + 32 * q);
+        if (lane % 2 || i >= chunk) continue;      // a lane per 32 bytes
+        if (p.norm_weight) prefetch_l2(p.norm_weight + warp * chunk + i);
+        if (post) prefetch_l2(post + warp * chunk + i);
+    }
 }
 // xs [n] and a barrier; scratch: 4 * kDenseWarps floats.
-__device__ __forceinline__ void sublayer_in_registers(const SublayerEnd& p, const PrologueConstants& c, float* xs, float* scratch) {
+__device__ __forceinline__ void sublayer_in_registers(const SublayerEnd& p, float* xs, float* scratch) {
     const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31, chunk = p.n / kDenseWarps, first = warp * chunk;
     const float part_size = static_cast<float>(p.n / p.groups);
     const uint32_t per = kDenseWarps / p.groups, part = warp / per * per;      // the warps that share this warp's part of the norm
@@ -131,10 +140,12 @@ __device__ __forceinline__ void sublayer_in_registers(const SublayerEnd& p, cons
         for (uint32_t w = 0; w < count; ++w) s += sums[from + w];
         return 1.0f / sqrtf(s / size + p.eps);
     };
-    RowWords x, y, z;
+    RowWords x, y, z, norm, post;
     row_words(x, p.x_in, first, chunk, lane);
     row_words(y, p.y_a, first, chunk, lane);
     row_words(z, p.y_b ? p.y_b : p.shift ? p.before : nullptr, first, chunk, lane);
+    row_words(norm, p.norm_weight, first, chunk, lane);
+    row_words(post, prologue_post(p), first, chunk, lane);
     if (p.y_b) {
         RowWords a, b;
         row_words(a, p.weight_a, first, chunk, lane);
@@ -153,7 +164,7 @@ __device__ __forceinline__ void sublayer_in_registers(const SublayerEnd& p, cons
         if (lane == 0) scratch[2 * kDenseWarps + warp] = s;
         __syncthreads();
         const float r = inverse_rms(scratch, 2 * kDenseWarps + part, per, part_size);
-        row_each(y, [&](float& v, int q, int k) { v = row_at(x, q, k) + v * r * row_at(c.norm, q, k); });
+        row_each(y, [&](float& v, int q, int k) { v = row_at(x, q, k) + v * r * row_at(norm, q, k); });
     } else {
         row_each(y, [&](float& v, int q, int k) { v += row_at(x, q, k); });      // y_a null: y is zero
     }
@@ -166,13 +177,13 @@ __device__ __forceinline__ void sublayer_in_registers(const SublayerEnd& p, cons
         }
     }
     if (p.shift) {
-        row_each(y, [&](float& v, int q, int k) { v += (row_at(z, q, k) - v) * row_at(c.post, q, k); });
+        row_each(y, [&](float& v, int q, int k) { v += (row_at(z, q, k) - v) * row_at(post, q, k); });
     } else if (p.out_norm) {
         const float s = warp_sum(row_square_sum(y));
         if (lane == 0) scratch[3 * kDenseWarps + warp] = s;
         __syncthreads();
         const float r = inverse_rms(scratch, 3 * kDenseWarps + part, per, part_size);
-        row_each(y, [&](float& v, int q, int k) { v = v * r * row_at(c.post, q, k); });
+        row_each(y, [&](float& v, int q, int k) { v = v * r * row_at(post, q, k); });
     }
 #pragma unroll
     for (int q = 0; q < kPreQuads; ++q) {
@@ -256,8 +267,7 @@ __global__ void __launch_bounds__(kDenseThreads, 2) gemv_bf16_kernel(const __gri
     // the input vectors in shared memory, each padded with zeros to whole units; then per-row partial sums of the slice
     float* const xs = dense_smem + dense_ring_bytes(kSlots) / sizeof(float);
     uint32_t x_floats = 0;
-    // the bias of the thread's first row, which would otherwise come from HBM at the very end
-    float bias = 0.0f;
+    const float* bias_at = nullptr;      // the bias of the thread's first row
     {
         const uint32_t row = slice0 + threadIdx.x;
         if (row < slice1) {
@@ -265,18 +275,18 @@ __global__ void __launch_bounds__(kDenseThreads, 2) gemv_bf16_kernel(const __gri
             while (row >= p.task[ti].first_row + p.task[ti].rows) ++ti;
             const DenseTask& t = p.task[ti];
             const uint32_t r = row - t.first_row;
-            if (t.bias && r >= 2 * t.pairs) bias = __ldg(t.bias + r - 2 * t.pairs);
+            if (t.bias && r >= 2 * t.pairs) bias_at = t.bias + r - 2 * t.pairs;
         }
+        if (bias_at) prefetch_l2(bias_at);
     }
     if (p.has_prologue) {
         x_floats = dense_units(p.task[0].ld) * kDenseUnit;
         float* scratch = xs + x_floats;
         for (uint32_t i = p.pre.n + threadIdx.x; i < x_floats; i += kDenseThreads) xs[i] = 0.0f;
         if (p.row_in_registers) {
-            PrologueConstants constants;
-            prologue_constants(constants, p.pre);
+            prologue_prefetch(p.pre);
             pdl_wait();
-            sublayer_in_registers(p.pre, constants, xs, scratch);
+            sublayer_in_registers(p.pre, xs, scratch);
         } else {
             pdl_wait();
             sublayer_row<kDenseThreads>(p.pre, 0, xs, scratch);
@@ -302,6 +312,7 @@ __global__ void __launch_bounds__(kDenseThreads, 2) gemv_bf16_kernel(const __gri
         __syncthreads();
     }
     float* sums = xs + x_floats + p.scratch_floats;      // [rows of the slice][k_split]
+    const float bias = bias_at ? __ldcg(bias_at) : 0.0f;
 
     unsigned long long acc2[kDenseRows];
 #pragma unroll
@@ -370,7 +381,7 @@ __global__ void __launch_bounds__(kDenseThreads, 2) gemv_bf16_kernel(const __gri
         if (r < paired) {
             if (!(r & 1)) t.gated[r / 2] = silu_f(total(i)) * total(i + 1);
         } else {
-            t.y[r - paired] = dense_activation(total(i) + (i < kDenseThreads ? bias : t.bias ? __ldg(t.bias + r - paired) : 0.0f), t.act, t.cap);
+            t.y[r - paired] = dense_activation(total(i) + (i < kDenseThreads ? bias : t.bias ? __ldcg(t.bias + r - paired) : 0.0f), t.act, t.cap);
         }
     }
 }
