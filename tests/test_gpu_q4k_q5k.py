@@ -138,7 +138,8 @@ def _close_to_f64(got, fmt, w, x, some_rows, cols, repeat):
     """Within 2^-22 of an activation per product (two f16 digits) and the rounding of fp32 sums over a row, of the terms' magnitudes (a
     Q4_K / Q5_K weight is the difference of two terms, the smaller of at most 63 * 1.5e-4, random_k_blocks); and per product
     2^-14 of a block's step times its largest activation: what the matrix instruction keeps of a product beside the largest of its
-    sixteen, 24 bits below the exponent of an f16 number of ten mantissa bits."""
+    sixteen, 24 bits below the exponent of an f16 number of ten mantissa bits.  Q6_K from 4096 columns on (gemv_kq.cuh): an
+    activation is off by half a step of its second digit at most, 1 / (127 * 512) of the largest of its 32."""
     decoded = blocks.dequantize(fmt, w[:some_rows], some_rows, cols).astype(np.float64)
     want, terms = x.astype(np.float64) @ decoded.T, np.abs(x).astype(np.float64) @ (np.abs(decoded) + (0.019 if fmt in (blocks.Q4_K, blocks.Q5_K) else 0.0)).T
     n = 16 if fmt == blocks.Q6_K else 32
@@ -147,6 +148,9 @@ def _close_to_f64(got, fmt, w, x, some_rows, cols, repeat):
     step = np.where(gaps > 1e-9 * np.abs(values).max(), gaps, np.inf).min(axis=2)          # [rows][blocks]
     largest = np.abs(x).astype(np.float64).reshape(x.shape[0], -1, n).max(axis=2)
     bound = terms * (2.0 ** -22 + 64 * 2.0 ** -24) + n * 2.0 ** -14 * largest @ np.where(np.isfinite(step), step, 0.0).T + 1e-30
+    if fmt == blocks.Q6_K and cols >= 4096:
+        largest, weight = np.abs(x).reshape(x.shape[0], -1, 32).max(axis=2).astype(np.float64), np.abs(decoded).reshape(some_rows, -1, 32).sum(axis=2)
+        bound = terms * 64 * 2.0 ** -24 + largest @ weight.T / (127 * 512)
     for first in range(0, got.shape[1], some_rows):
         part = got[:, first:first + some_rows]
         assert np.all(np.abs(part - want[:, :part.shape[1]]) <= bound[:, :part.shape[1]])
@@ -154,19 +158,46 @@ def _close_to_f64(got, fmt, w, x, some_rows, cols, repeat):
             break
 
 
+def _rows_of(be, name, parts, x, cols):
+    """One launch of several tensors; their outputs."""
+    import torch
+    tokens = x.shape[0]
+    hs = [be.dev_upload(name, w, w.shape[0], cols) for w in parts]
+    d_x, ys = torch.from_numpy(x).cuda(), [torch.full((tokens, w.shape[0]), float("nan"), device="cuda") for w in parts]
+    be.dev_gemv(hs, [y.data_ptr() for y in ys], d_x.data_ptr(), tokens, 2)
+    be.dev_check()
+    for h in hs:
+        be.dev_free(h)
+    return [y.cpu().numpy() for y in ys]
+
+
+# A row's arithmetic is chosen by format and columns: neither a companion of 70 million weights nor other tokens of the launch may move it by
+# more than the rounding of its sums, some 1e-6 (the two kernels of these formats are 2e-5 apart).
+@pytest.mark.parametrize("name", list(ALL))
+@pytest.mark.parametrize("cols", [1024, 3840, 4096, 4352])
+def test_what_shares_a_launch_does_not_choose_a_rows_arithmetic(be, name, cols):
+    fmt = ALL[name]
+    w, x = _weights(fmt, 40, cols, cols), seeded_acts(8, cols, cols + 1)
+    some = _weights(fmt, 64, cols, 5)
+    large = np.ascontiguousarray(np.tile(some, ((70 << 20) // cols // 64 + 1, 1)))
+    most = 8 if cols <= 4096 else 4                  # the limit of columns x tokens
+    alone = np.concatenate([_rows_of(be, name, [w], x[t:t + 1], cols)[0] for t in range(most)])
+    apart = lambda got: np.linalg.norm(got - alone[:got.shape[0]]) / np.linalg.norm(alone[:got.shape[0]])
+    for tokens in (2, 3, most):
+        assert apart(_rows_of(be, name, [w], x[:tokens], cols)[0]) < 5e-6
+    for tokens in (1, 2, 3):
+        assert apart(_rows_of(be, name, [large, w], x[:tokens], cols)[1]) < 5e-6
+
+
 # edges of tiles (16 rows), of units (256 columns; Q4_0 ends inside one), of warps' shares; one or more groups of four tokens;
 # 16384 columns by three tokens and 14336 by two or three go over the row in several passes
 @pytest.mark.parametrize("name", list(ALL))
 @pytest.mark.parametrize("rows,cols,tokens", [(1, 256, 3), (15, 256, 4), (17, 512, 5), (33, 768, 8), (1200, 4096, 3), (2405, 1280, 4), (2405, 1280, 7), (300, 14336, 2), (300, 14336, 3),
-                                              (140, 11008, 3), (5000, 256, 6)])
+                                              (140, 11008, 3), (5000, 256, 6), (1200, 3840, 3), (300, 3840, 8), (9000, 2048, 4)])
 def test_several_rows_at_once(be, name, rows, cols, tokens):
     fmt = ALL[name]
     if name == "Q6_K" and cols * tokens > 32768:
         tokens = 2
-    if name == "Q6_K" and tokens == 2:
-        rows = 4700                     # 64 M weights
-    elif name == "Q6_K":
-        rows += (1 << 20) // cols + 1   # more than a million
     w, x = _weights(fmt, rows, cols, rows + tokens), seeded_acts(tokens, cols, cols)
     _close_to_f64(_products(be, name, w, x, rows, cols), fmt, w, x, rows, cols, False)
 
@@ -177,14 +208,19 @@ def test_q4_0_rows_that_end_inside_a_unit(be, rows, cols, tokens):
     _close_to_f64(_products(be, "Q4_0", w, x, rows, cols), blocks.Q4_0, w, x, rows, cols, False)
 
 
-# one activation row comes here from 64 M weights on (Q4_0) or 32 M (Q4_K, Q5_K); the rows of a small matrix over and over
+# one activation row; the rows of a small matrix over and over
 @pytest.mark.parametrize("name,rows,cols", [("Q4_0", 16500, 4096), ("Q4_0", 16400, 4128), ("Q4_0", 4700, 14336), ("Q4_0", 262200, 256), ("Q4_K", 8200, 4096), ("Q4_K", 3077, 11008),
                                             ("Q5_K", 8200, 4096), ("Q5_K", 32800, 1024)])
 def test_one_row_of_a_large_matrix(be, name, rows, cols):
-    fmt, some = ALL[name], 50
+    fmt, some = ALL[name], min(rows, 50)
     part = _weights(fmt, some, cols, rows)
     w, x = np.ascontiguousarray(np.tile(part, (rows // some + 1, 1))[:rows]), seeded_acts(1, cols, cols)
     _close_to_f64(_products(be, name, w, x, rows, cols), fmt, w, x, some, cols, True)
+
+
+@pytest.mark.parametrize("name,rows,cols", [(n, r, c) for n in ALL for r, c in ((1, 256), (17, 1024), (150, 3840), (9000, 2048), (2400, 512), (130, 14336))] + [("Q4_0", 37, 32), ("Q4_0", 70, 96)])
+def test_one_row(be, name, rows, cols):
+    test_one_row_of_a_large_matrix(be, name, rows, cols)
 
 
 def test_more_rows_than_their_sums_fit(be):

@@ -1,27 +1,18 @@
-// Decode-time matrix-vector products for Q4_0, Q6_K, Q4_K and Q5_K with one activation row, and for Q6_K with up to eight; which launches
-// come here and which to the matrix instructions of gemv_kq_mma.cuh: kq_takes_mma there.
+// Decode-time matrix-vector products for Q6_K from 4096 columns on (batch 1..8).  Which products come here and which to the matrix
+// instructions of gemv_kq_mma.cuh, which has the other small formats: kq_takes_mma there.
 //
-// The reference evaluates both formats with fp32 activations: Q4_0 through its generic
-// dequantise-then-dot route (src/quant.cpp:1135-1162 over gemv_avx2, kernels/avx2.cpp:16-40) and
-// Q6_K through gemv_q6k_avx2 / gemm_q6k_kblk_avx2 (kernels/avx2.cpp:380-422, :1762-1770).  Decoding
-// every weight to fp32 costs several ALU operations per weight, more than an SM can issue at HBM
-// speed, so the dot products here stay in integers: weights are used as the small integers they
+// The reference evaluates the format with fp32 activations, through gemv_q6k_avx2 / gemm_q6k_kblk_avx2
+// (kernels/avx2.cpp:380-422, :1762-1770).  Decoding every weight to fp32 costs several ALU operations per weight, more than an
+// SM can issue at HBM speed, so the dot products here stay in integers: weights are used as the small integers they
 // are, and each activation enters as two int8 digits, x ~= (d/256) * (256*q1 + q2) with an error
 // below d/512 (quantize_acts.cuh).  Results agree with the fp32-activation reference to ~1e-5.
 //
-//   Q4_0 : y += d_w * (d_x/256) * ( sum n*(256*q1+q2)  -  8 * sum(256*q1+q2) )      n = nibble 0..15
-//   Q6_K : y += d * sc_g * (d_x/256) * sum (q-32)*(256*q1+q2)                        per 16-weight group
-//   Q4_K / Q5_K (the reference: gemv_q4k_q5k_avx2, kernels/avx2.cpp:329-378, fp32 activations; its GPU entry is
-//          zen::d3d12::gemm_kquant, include/zen/d3d12_backend.h:75), per 32-weight sub-block g of a super-block:
-//          y += d * sc_g * (d_x/256) * sum q*(256*q1+q2)  -  dmin * m_g * (d_x/256) * sum (256*q1+q2)
-//          with q the 4-bit (Q4_K) or 5-bit (Q5_K: nibble + 16 * fifth bit) code
+//   y += d * sc_g * (d_x/256) * sum (q-32)*(256*q1+q2)                        per 16-weight group
 //
 // Same streaming skeleton as the Q8_0 kernel (gemv_q8_0.cuh): a persistent CTA per SM owns a
 // byte-balanced row slice, a producer warp feeds a ring of shared-memory stages with TMA bulk
 // copies, sixteen consumer warps in two teams own one row each.  Algorithmic traffic is the raw
-// GGUF size (18 B per Q4_0 block, 210 B per Q6_K super-block, 144 / 176 B per Q4_K / Q5_K super-block; the device
-// planes of the last two are 4 bytes per super-block larger, because the 12 packed bytes of 6-bit scales and minimums
-// are kept unpacked as 16, see repack.cuh).
+// GGUF size (210 B per super-block).
 #pragma once
 #include <cuda.h>
 #include <cuda_fp16.h>
@@ -30,41 +21,20 @@
 
 namespace zk {
 
-constexpr int kKqSegElems = 4096;   // weights per row per stage segment (128 Q4_0 blocks, 16 Q6_K super-blocks)
+constexpr int kKqSegElems = 4096;   // weights per row per stage segment (16 super-blocks)
 constexpr int kKqMaxPlanes = 4;
 constexpr int kKqPartialFloats = kTeams * 2 * kTeamWarps * kTeamWarps;   // [team][unit parity][K slice][row]
 
 // Per-format geometry of the planes a row is split into (repack.cuh).
 template <int kFormat> struct KqFormat;
 
-template <> struct KqFormat<2> {   // Q4_0: nibbles [K/2], f16 scales [K/32]
-    static constexpr int kPlanes = 2;
-    static constexpr int kStages = 6;   // a multiple of the team count, see kGemvStages
-    __host__ __device__ static constexpr uint32_t seg_bytes(int plane) { return plane == 0 ? kKqSegElems / 2 : kKqSegElems / 32 * 2; }
-    __host__ __device__ static constexpr uint32_t bytes_per_256(int plane) { return plane == 0 ? 128 : 16; }
-};
 template <> struct KqFormat<14> {  // Q6_K: ql [K/2], qh [K/4], int8 sc [K/16], f16 d [K/256]
     static constexpr int kPlanes = 4;
-    static constexpr int kStages = 4;
+    static constexpr int kStages = 4;   // a multiple of the team count, see kGemvStages
     __host__ __device__ static constexpr uint32_t seg_bytes(int plane) {
         return plane == 0 ? kKqSegElems / 2 : plane == 1 ? kKqSegElems / 4 : plane == 2 ? kKqSegElems / 16 : kKqSegElems / 256 * 2;
     }
     __host__ __device__ static constexpr uint32_t bytes_per_256(int plane) { return plane == 0 ? 128 : plane == 1 ? 64 : plane == 2 ? 16 : 2; }
-};
-
-template <> struct KqFormat<12> {  // Q4_K: nibbles [K/2], unpacked sub-block scales|minimums [K/16], (d, dmin) f16 pairs [K/256]
-    static constexpr int kPlanes = 3;
-    static constexpr int kStages = 6;
-    __host__ __device__ static constexpr uint32_t seg_bytes(int plane) { return plane == 0 ? kKqSegElems / 2 : plane == 1 ? kKqSegElems / 16 : kKqSegElems / 256 * 4; }
-    __host__ __device__ static constexpr uint32_t bytes_per_256(int plane) { return plane == 0 ? 128 : plane == 1 ? 16 : 4; }
-};
-template <> struct KqFormat<13> {  // Q5_K: nibbles [K/2], fifth bits [K/8], scales|minimums [K/16], (d, dmin) [K/256]
-    static constexpr int kPlanes = 4;
-    static constexpr int kStages = 4;
-    __host__ __device__ static constexpr uint32_t seg_bytes(int plane) {
-        return plane == 0 ? kKqSegElems / 2 : plane == 1 ? kKqSegElems / 8 : plane == 2 ? kKqSegElems / 16 : kKqSegElems / 256 * 4;
-    }
-    __host__ __device__ static constexpr uint32_t bytes_per_256(int plane) { return plane == 0 ? 128 : plane == 1 ? 32 : plane == 2 ? 16 : 4; }
 };
 // Q6_K with the codes unpacked on upload (kFormatQ6KCodes): q - 32 as one int8 per weight in element order, the group
 // scales and super-block scales as in the packed layout.  The device copy is 1.07 bytes per weight instead of the file's
@@ -78,9 +48,6 @@ template <> struct KqFormat<kFormatQ6KCodes> {  // codes [K] int8, sc [K/16] int
     __host__ __device__ static constexpr uint32_t seg_bytes(int plane) { return plane == 0 ? kKqSegElems : plane == 1 ? kKqSegElems / 16 : kKqSegElems / 256 * 2; }
     __host__ __device__ static constexpr uint32_t bytes_per_256(int plane) { return plane == 0 ? 256 : plane == 1 ? 16 : 2; }
 };
-// Q4_K and Q5_K share everything but the fifth-bit plane.
-template <int kFormat> constexpr bool kq_is_k45 = kFormat == 12 || kFormat == 13;
-
 template <int kFormat> __host__ __device__ constexpr uint32_t kq_row_stage_bytes() {
     uint32_t b = 0;
     for (int i = 0; i < KqFormat<kFormat>::kPlanes; ++i) b += KqFormat<kFormat>::seg_bytes(i);
@@ -125,9 +92,17 @@ __host__ __device__ inline size_t gemv_kq_smem_bytes(uint32_t nseg, int batch) {
     const size_t kpad = static_cast<size_t>(nseg) * kKqSegElems;
     return static_cast<size_t>(KqFormat<kFormat>::kStages) * kq_stage_bytes<kFormat>()
            + static_cast<size_t>(batch) * 2 * kpad                 // two digit planes, natural order
-           + static_cast<size_t>(batch) * (kpad / 32) * 8          // per-block scale (d/256) and code sum
+           + static_cast<size_t>(batch) * (kpad / 32) * 8          // per-block scale (d/256); half of it unused (the limit of columns x tokens counts it)
            + 2 * KqFormat<kFormat>::kStages * 8 + 16
            + kKqPartialFloats * sizeof(float);                      // batch 1: per-warp partial row sums
+}
+
+// The limit of columns x tokens that entry points and callers know of Q4_0, Q4_K and Q5_K: what their activations take as two digits
+// beside a ring of six (Q5_K: four) stages of eight rows.
+inline size_t gemv_kq_limit_bytes(int format, uint32_t nseg, int batch) {
+    const size_t kpad = static_cast<size_t>(nseg) * kKqSegElems, stages = format == 13 ? 4 : 6;
+    const size_t row = kKqSegElems / 2 + (format == 2 ? kKqSegElems / 32 * 2 : kKqSegElems / 16 + kKqSegElems / 256 * 4 + (format == 13 ? kKqSegElems / 8 : 0));
+    return stages * kTeamWarps * row + static_cast<size_t>(batch) * (2 * kpad + kpad / 32 * 8) + 2 * stages * 8 + 16 + kKqPartialFloats * sizeof(float);
 }
 
 struct KqWalk {  // GroupWalk over KqParams
@@ -157,44 +132,37 @@ __device__ __forceinline__ int dot16(const uint4& w, const uint4& x) {
 // from borrowing across bytes, flipping it back afterwards leaves the two's-complement difference.
 __device__ __forceinline__ uint32_t sub32_bytes(uint32_t q) { return ((q | 0x80808080u) - 0x20202020u) ^ 0x80808080u; }
 
-// Sum of `v` over the lanes of a warp for R rows at once.  Each exchange step halves the number of rows a lane still
-// carries, so R rows cost R - 1 + (5 - log2 R) shuffles instead of 5 R.  On return every lane holds the complete sum
+// Sum of `v` over the lanes of a warp for eight rows at once.  Each exchange step halves the number of rows a lane still
+// carries, so they cost 9 shuffles instead of 40.  On return every lane holds the complete sum
 // of row `row` (lanes that share the low bits hold the same row); the order of additions is fixed.
-template <int R>
-__device__ __forceinline__ float kq_reduce_rows(const float (&acc)[R], int lane, uint32_t& row) {
-    static_assert(R == 4 || R == 8, "four or eight rows per warp");
+__device__ __forceinline__ float kq_reduce_rows(const float (&acc)[8], int lane, uint32_t& row) {
     float a4[4];
-    if constexpr (R == 8) {
+    {
         const bool up = lane & 16;
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
             const float send = up ? acc[i] : acc[i + 4], keep = up ? acc[i + 4] : acc[i];
             a4[i] = keep + __shfl_xor_sync(0xffffffffu, send, 16);
         }
-    } else {
-#pragma unroll
-        for (int i = 0; i < 4; ++i) a4[i] = acc[i];
     }
-    constexpr int o2 = R == 8 ? 8 : 16, o1 = R == 8 ? 4 : 8;
     float a2[2];
     {
-        const bool up = lane & o2;
+        const bool up = lane & 8;
 #pragma unroll
         for (int i = 0; i < 2; ++i) {
             const float send = up ? a4[i] : a4[i + 2], keep = up ? a4[i + 2] : a4[i];
-            a2[i] = keep + __shfl_xor_sync(0xffffffffu, send, o2);
+            a2[i] = keep + __shfl_xor_sync(0xffffffffu, send, 8);
         }
     }
     float a1;
     {
-        const bool up = lane & o1;
+        const bool up = lane & 4;
         const float send = up ? a2[0] : a2[1], keep = up ? a2[1] : a2[0];
-        a1 = keep + __shfl_xor_sync(0xffffffffu, send, o1);
+        a1 = keep + __shfl_xor_sync(0xffffffffu, send, 4);
     }
 #pragma unroll
-    for (int o = o1 >> 1; o > 0; o >>= 1) a1 += __shfl_xor_sync(0xffffffffu, a1, o);
-    if constexpr (R == 8) row = ((lane >> 4) & 1) * 4 + ((lane >> 3) & 1) * 2 + ((lane >> 2) & 1);
-    else row = ((lane >> 4) & 1) * 2 + ((lane >> 3) & 1);
+    for (int o = 2; o > 0; o >>= 1) a1 += __shfl_xor_sync(0xffffffffu, a1, o);
+    row = ((lane >> 4) & 1) * 4 + ((lane >> 3) & 1) * 2 + ((lane >> 2) & 1);
     return a1;
 }
 
@@ -212,15 +180,13 @@ __global__ void __launch_bounds__(kGemvThreads, 1) gemv_kq_kernel(const __grid_c
     using F = KqFormat<kFormat>;
     constexpr int kStages = F::kStages;
     static_assert(kStages % kTeams == 0, "ring depth must be a multiple of the number of consumer teams");
-    static_assert(kBatch == 1 || kFormat == 14 || kFormat == kFormatQ6KCodes, "more rows: gemv_kq_mma.cuh");
     constexpr uint32_t kStageBytes = kq_stage_bytes<kFormat>();
     extern __shared__ __align__(128) uint8_t smem[];
     const uint32_t kpad = p.nseg * kKqSegElems;
     uint8_t* ring = smem;
     uint8_t* xd = ring + kStages * kStageBytes;                                  // [batch][2][kpad] int8, natural order
     float* xscale = reinterpret_cast<float*>(xd + static_cast<size_t>(kBatch) * 2 * kpad);   // [batch][kpad/32]  d/256
-    int* xsum = reinterpret_cast<int*>(xscale + static_cast<size_t>(kBatch) * (kpad / 32));  // [batch][kpad/32]  sum(256*q1+q2)
-    uint64_t* full = reinterpret_cast<uint64_t*>(xsum + static_cast<size_t>(kBatch) * (kpad / 32));
+    uint64_t* full = reinterpret_cast<uint64_t*>(xscale + static_cast<size_t>(kBatch) * 2 * (kpad / 32));
     uint64_t* empty = full + kStages;
     volatile int* abort_word = reinterpret_cast<volatile int*>(empty + kStages);
     float* partial = reinterpret_cast<float*>(empty + kStages + 2);   // batch 1: [team][unit parity][K slice][row]
@@ -370,19 +336,11 @@ __global__ void __launch_bounds__(kGemvThreads, 1) gemv_kq_kernel(const __grid_c
                 const float v[8] = {lo.x, lo.y, lo.z, lo.w, hi.x, hi.y, hi.z, hi.w};
                 uint2 c1, c2;
                 const float d = quantise_block_quad(v, c1, c2);
-                // sum of the eight two-digit codes of this lane, then of the block's four lanes
-                int sum = dp4a_ss(c1.x, 0x01010101u, 0) + dp4a_ss(c1.y, 0x01010101u, 0);
-                sum = sum * 256 + dp4a_ss(c2.x, 0x01010101u, 0) + dp4a_ss(c2.y, 0x01010101u, 0);
-                sum += __shfl_xor_sync(0xffffffffu, sum, 1);
-                sum += __shfl_xor_sync(0xffffffffu, sum, 2);
                 if (!live) continue;
                 uint8_t* base = xd + static_cast<size_t>(t) * 2 * kpad + b * 32 + part * 8;
                 *reinterpret_cast<uint2*>(base) = c1;
                 *reinterpret_cast<uint2*>(base + kpad) = c2;
-                if (part == 0) {
-                    xscale[static_cast<size_t>(t) * (kpad / 32) + b] = d * (1.0f / 256.0f);
-                    xsum[static_cast<size_t>(t) * (kpad / 32) + b] = sum;
-                }
+                if (part == 0) xscale[static_cast<size_t>(t) * (kpad / 32) + b] = d * (1.0f / 256.0f);
             }
         }
     }
@@ -394,57 +352,26 @@ __global__ void __launch_bounds__(kGemvThreads, 1) gemv_kq_kernel(const __grid_c
         // ---- batch 1: a warp owns a slice of K and walks every row of the unit with its activations in registers ----
         // Shared memory is then read for weights only (reading two activation digits per weight from it costs several
         // times the weight bytes in wavefronts and capped the kernel at a third of the HBM rate).
-        //   Q4_0: warp = (K slice of 32 blocks, half of the eight rows); a lane owns one 32-weight block
-        //   Q6_K: warp = K slice of two super-blocks, all eight rows;     a lane owns one 16-weight scale group
-        //   Q4_K / Q5_K: warp = (K slice of four super-blocks, half of the eight rows); a lane owns 16 nibble bytes, i.e. 16
-        //         weights of sub-block 2j (low nibbles) and the 16 of sub-block 2j+1 at the same positions (high nibbles)
-        constexpr bool kK45 = kq_is_k45<kFormat>;
+        // A warp has a K slice of two super-blocks and all eight rows; a lane owns one 16-weight scale group.
         constexpr bool kCodes = kFormat == kFormatQ6KCodes;   // a lane owns the 16 weights of group (lane & 15) of its super-block, in element order
-        constexpr int kR = (kFormat == 2 || kK45) ? 4 : 8;             // rows per warp
-        constexpr int kSlices = (kFormat == 2 || kK45) ? 4 : 8;        // K slices per segment
-        const uint32_t kslice = static_cast<uint32_t>(twarp) % kSlices;
-        const uint32_t rowbase = kR == 4 ? (static_cast<uint32_t>(twarp) / kSlices) * kR : 0u;
-        // Q4_K / Q5_K lane geometry (src/quant.cpp:133-141 and the kernels at kernels/avx2.cpp:329-378): element
-        // g*32 + l of a super-block is the nibble (g & 1) of byte (g >> 1)*32 + l, its fifth bit is bit g of qh[l]
-        const uint32_t k_sb = kslice * 4 + (static_cast<uint32_t>(lane) >> 3), k_j = (static_cast<uint32_t>(lane) >> 1) & 3, k_h = lane & 1;
-        float k_xs_hi = 0.0f, k_f_lo = 0.0f, k_f_hi = 0.0f;   // the high sub-block's activation scale; scale x code sum of both
+        constexpr int kR = kTeamWarps;             // rows per warp
+        constexpr int kSlices = 8;                 // K slices per segment
+        const uint32_t kslice = static_cast<uint32_t>(twarp);
         // Q6_K lane geometry (src/quant.cpp:500-517): element e = half*128 + group*32 + l lives in ql byte
         // half*64 + (group%2)*32 + l (low nibble for group < 2), qh byte half*32 + l bits 2*group.., scale half*8 + group*2 + l/16
         const uint32_t sg = lane & 15, qhalf = sg >> 3, group = (sg >> 1) & 3, six = sg & 1;
         const uint32_t shift4 = group >= 2 ? 4u : 0u, shift2 = group * 2;
         const uint32_t sbl = kslice * 2 + (static_cast<uint32_t>(lane) >> 4);   // super-block within the segment
 
-        uint4 xa = make_uint4(0, 0, 0, 0), xb = xa, xc = xa, xd4 = xa;   // Q4_0: digit 1 lo/hi halves, digit 2 lo/hi; Q6_K: digit 1, digit 2
-        float xs = 0.0f;     // activation scale of the lane's block, with the digit weight folded in
+        uint4 xa = make_uint4(0, 0, 0, 0), xc = xa;   // digit 1, digit 2
+        float xs = 0.0f;     // activation scale of the lane's block
         int bias = 0;        // minus (zero point x sum of the lane's activation codes), the dp4a chain's starting value
         // A lane whose block lies past the end of the row reads the segment's first block instead (valid bytes, so a
         // finite scale) with zero activations and a zero scale: its terms are exactly zero and need no select.
-        uint32_t wofs = 0;   // byte offset of the lane's weights within a row of plane 0 (Q4_0) / super-block index (Q6_K)
+        uint32_t wofs = 0;   // the lane's super-block
         auto load_x = [&](uint32_t seg) {
             const uint4 zero = make_uint4(0, 0, 0, 0);
-            if (kFormat == 2) {
-                const uint32_t b = seg * (kKqSegElems / 32) + kslice * 32 + lane;
-                const bool live = b * 32 < p.K;
-                const uint4* x1 = reinterpret_cast<const uint4*>(xd + b * 32);
-                const uint4* x2 = reinterpret_cast<const uint4*>(xd + kpad + b * 32);
-                xa = live ? x1[0] : zero; xb = live ? x1[1] : zero; xc = live ? x2[0] : zero; xd4 = live ? x2[1] : zero;
-                xs = live ? xscale[b] * (1.0f / 16.0f) : 0.0f;   // high nibbles enter sixteen-fold, so every sum is sixteen-fold
-                bias = live ? -128 * xsum[b] : 0;                 // -8 * sum, sixteen-fold
-                wofs = live ? kslice * 32 + lane : 0u;
-            } else if (kK45) {
-                const uint32_t e_lo = seg * kKqSegElems + k_sb * 256 + k_j * 64 + k_h * 16, e_hi = e_lo + 32;
-                const bool live = e_lo < p.K;   // K is a multiple of 256: the lane's two sub-blocks are both inside or both outside
-                xa = live ? *reinterpret_cast<const uint4*>(xd + e_lo) : zero;
-                xb = live ? *reinterpret_cast<const uint4*>(xd + e_hi) : zero;
-                xc = live ? *reinterpret_cast<const uint4*>(xd + kpad + e_lo) : zero;
-                xd4 = live ? *reinterpret_cast<const uint4*>(xd + kpad + e_hi) : zero;
-                xs = live ? xscale[e_lo / 32] : 0.0f;
-                k_xs_hi = live ? xscale[e_hi / 32] : 0.0f;
-                const uint4 ones = make_uint4(0x01010101u, 0x01010101u, 0x01010101u, 0x01010101u);
-                k_f_lo = xs * static_cast<float>(dot16(ones, xa) * 256 + dot16(ones, xc));        // for the minimum term
-                k_f_hi = k_xs_hi * static_cast<float>(dot16(ones, xb) * 256 + dot16(ones, xd4));
-                wofs = live ? k_sb : 0u;
-            } else if (kCodes) {
+            if (kCodes) {
                 const uint32_t e0 = seg * kKqSegElems + sbl * 256 + sg * 16;
                 const bool live = e0 < p.K;
                 xa = live ? *reinterpret_cast<const uint4*>(xd + e0) : zero;
@@ -491,16 +418,7 @@ __global__ void __launch_bounds__(kGemvThreads, 1) gemv_kq_kernel(const __grid_c
                 const uint8_t* w1;
                 const int8_t* sc = nullptr;
                 const __half* dd = nullptr;
-                if (kFormat == 2) {
-                    w0 = st + kq_plane_offset<kFormat>(0) + rowbase * F::seg_bytes(0) + wofs * 16;   // nibbles
-                    w1 = st + kq_plane_offset<kFormat>(1) + rowbase * F::seg_bytes(1) + wofs * 2;    // scale
-                } else if (kK45) {
-                    constexpr int kScm = F::kPlanes - 2, kDd = F::kPlanes - 1;
-                    w0 = st + kq_plane_offset<kFormat>(0) + rowbase * F::seg_bytes(0) + wofs * 128 + k_j * 32 + k_h * 16;   // nibbles
-                    w1 = st + kq_plane_offset<kFormat>(1) + rowbase * F::seg_bytes(1) + wofs * 32 + k_h * 16;             // Q5_K: fifth bits
-                    sc = reinterpret_cast<const int8_t*>(st + kq_plane_offset<kFormat>(kScm) + rowbase * F::seg_bytes(kScm)) + wofs * 16 + k_j * 2;
-                    dd = reinterpret_cast<const __half*>(st + kq_plane_offset<kFormat>(kDd) + rowbase * F::seg_bytes(kDd)) + wofs * 2;
-                } else if (kCodes) {
+                if (kCodes) {
                     w0 = st + kq_plane_offset<kFormat>(0) + wofs * 256 + sg * 16;   // codes
                     w1 = w0;
                     sc = reinterpret_cast<const int8_t*>(st + kq_plane_offset<kFormat>(1)) + wofs * 16 + sg;
@@ -512,40 +430,7 @@ __global__ void __launch_bounds__(kGemvThreads, 1) gemv_kq_kernel(const __grid_c
                     dd = reinterpret_cast<const __half*>(st + kq_plane_offset<kFormat>(3)) + wofs;
                 }
                 auto row_body = [&](int r) {
-                    if (kFormat == 2) {
-                        const uint4 w = *reinterpret_cast<const uint4*>(w0 + r * F::seg_bytes(0));
-                        const float dw = __half2float(*reinterpret_cast<const __half*>(w1 + r * F::seg_bytes(1)));
-                        // low nibbles are elements 0..15, high nibbles elements 16..31 (src/quant.cpp:391-397); the high
-                        // nibbles stay in place (value x 16, an unsigned byte), which saves the shifts
-                        const uint32_t m = 0x0F0F0F0Fu;
-                        int a = dp4a_us(w.x & m, xa.x, 0), b = dp4a_us(w.x & ~m, xb.x, 0), c = dp4a_us(w.x & m, xc.x, 0), d = dp4a_us(w.x & ~m, xd4.x, bias);
-                        a = dp4a_us(w.y & m, xa.y, a); b = dp4a_us(w.y & ~m, xb.y, b); c = dp4a_us(w.y & m, xc.y, c); d = dp4a_us(w.y & ~m, xd4.y, d);
-                        a = dp4a_us(w.z & m, xa.z, a); b = dp4a_us(w.z & ~m, xb.z, b); c = dp4a_us(w.z & m, xc.z, c); d = dp4a_us(w.z & ~m, xd4.z, d);
-                        a = dp4a_us(w.w & m, xa.w, a); b = dp4a_us(w.w & ~m, xb.w, b); c = dp4a_us(w.w & m, xc.w, c); d = dp4a_us(w.w & ~m, xd4.w, d);
-                        // 16 * (256 * (lo.q1 + hi.q1) + (lo.q2 + hi.q2) - 8 * sum) = 4096 a + 256 b + 16 c + d
-                        const int isum = ((a * 16 + b) * 16 + c) * 16 + d;
-                        acc[r] = fmaf(dw * xs, static_cast<float>(isum), acc[r]);
-                    } else if (kK45) {
-                        constexpr int kScm = F::kPlanes - 2, kDd = F::kPlanes - 1;
-                        const uint4 w = *reinterpret_cast<const uint4*>(w0 + r * F::seg_bytes(0));
-                        const uint32_t m = 0x0F0F0F0Fu;
-                        uint4 lo = make_uint4(w.x & m, w.y & m, w.z & m, w.w & m);
-                        uint4 hi = make_uint4((w.x >> 4) & m, (w.y >> 4) & m, (w.z >> 4) & m, (w.w >> 4) & m);
-                        if (kFormat == 13) {
-                            const uint4 q5 = *reinterpret_cast<const uint4*>(w1 + r * F::seg_bytes(1));
-                            const uint32_t s_lo = 2 * k_j, s_hi = 2 * k_j + 1, one = 0x01010101u;
-                            lo.x |= ((q5.x >> s_lo) & one) << 4; lo.y |= ((q5.y >> s_lo) & one) << 4; lo.z |= ((q5.z >> s_lo) & one) << 4; lo.w |= ((q5.w >> s_lo) & one) << 4;
-                            hi.x |= ((q5.x >> s_hi) & one) << 4; hi.y |= ((q5.y >> s_hi) & one) << 4; hi.z |= ((q5.z >> s_hi) & one) << 4; hi.w |= ((q5.w >> s_hi) & one) << 4;
-                        }
-                        const int i_lo = dot16(lo, xa) * 256 + dot16(lo, xc);     // codes are 0..31: signed and unsigned dp4a agree
-                        const int i_hi = dot16(hi, xb) * 256 + dot16(hi, xd4);
-                        const uint32_t sc2 = *reinterpret_cast<const uint16_t*>(sc + r * F::seg_bytes(kScm));        // scales of sub-blocks 2j, 2j+1
-                        const uint32_t mn2 = *reinterpret_cast<const uint16_t*>(sc + r * F::seg_bytes(kScm) + 8);    // their minimums
-                        const float2 dm = __half22float2(*reinterpret_cast<const __half2*>(dd + r * (F::seg_bytes(kDd) / 2)));
-                        const float pos = static_cast<float>(sc2 & 0xffu) * (xs * static_cast<float>(i_lo)) + static_cast<float>(sc2 >> 8) * (k_xs_hi * static_cast<float>(i_hi));
-                        const float neg = static_cast<float>(mn2 & 0xffu) * k_f_lo + static_cast<float>(mn2 >> 8) * k_f_hi;
-                        acc[r] = fmaf(dm.x, pos, fmaf(-dm.y, neg, acc[r]));
-                    } else if (kCodes) {
+                    if (kCodes) {
                         const uint4 q = *reinterpret_cast<const uint4*>(w0 + r * F::seg_bytes(0));
                         const int a = dot16(q, xa), c = dot16(q, xc);
                         const float dsc = __half2float(dd[r * (F::seg_bytes(2) / 2)]) * static_cast<float>(sc[r * F::seg_bytes(1)]);  // (d * scale), the reference's order
@@ -572,16 +457,16 @@ __global__ void __launch_bounds__(kGemvThreads, 1) gemv_kq_kernel(const __grid_c
                 } else {
 #pragma unroll
                     for (int r = 0; r < kR; ++r)
-                        if (rowbase + r < g.nrows) row_body(r);
+                        if (static_cast<uint32_t>(r) < g.nrows) row_body(r);
                 }
                 __syncwarp();
                 if (lane == 0) mbar_arrive(&empty[stage]);
             }
             // rows of the unit: sum over the warp's lanes, then over the K slices through shared memory
             uint32_t prow;
-            const float psum = kq_reduce_rows<kR>(acc, lane, prow);
+            const float psum = kq_reduce_rows(acc, lane, prow);
             float* part = partial + (team * 2 + (pair_index & 1)) * (kTeamWarps * kTeamWarps);
-            if ((lane & (kR == 8 ? 3 : 7)) == 0) part[kslice * kTeamWarps + rowbase + prow] = psum;
+            if ((lane & 3) == 0) part[kslice * kTeamWarps + prow] = psum;
             if (team_barrier_any(team, failed)) { ok = false; break; }
             if (twarp == 0 && static_cast<uint32_t>(lane) < g.nrows) {
                 float v = part[lane];

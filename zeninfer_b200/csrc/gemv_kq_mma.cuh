@@ -1,4 +1,4 @@
-// Decode-time matrix-vector products for Q4_0, Q6_K, Q4_K and Q5_K (batch 1..8).
+// Decode-time matrix-vector products for Q4_0, Q4_K, Q5_K and, below 4096 columns, Q6_K (batch 1..8).
 //
 // The reference evaluates these formats with fp32 activations: Q4_0 through its generic dequantise-then-dot route
 // (src/quant.cpp:1135-1162 over gemv_avx2, kernels/avx2.cpp:16-40), Q6_K through gemv_q6k_avx2 / gemm_q6k_kblk_avx2
@@ -11,7 +11,7 @@
 //   * weights: a code of up to ten bits IS an f16 number, the subnormal code * 2^-24, so a pair of weights costs one AND (high
 //     nibbles stay in place and count sixteenfold; their activations are divided by sixteen).  16 rows are the A operand;
 //   * activations: x * 2^e, one power of two per 256 columns, as the sum of two f16 numbers (22 bits), two columns of the B operand;
-//   * the scales differ per row and block, so a column may collect products of one block only.  One token: the four lanes that
+//   * the scales differ per row and block, so a column may collect products of one block only.  One token (not of Q6_K): the four lanes that
 //     share a row hold four different blocks, and B's eight columns are two digits of those four blocks, zero wherever column and
 //     lane belong to different blocks: a lane reads its weights as 16-byte words and ends up with the sums of its own block.  Two
 //     and more tokens: the four lanes hold four words of the same block and the columns are two digits of four tokens;
@@ -20,7 +20,8 @@
 //       Q4_0 : y += d_w * sum (n - 8) x                 per 32 weights
 //       Q6_K : y += d * sc_g * sum (q - 32) x           per 16 weights
 //       Q4_K / Q5_K : y += d * sc_g * sum q x  -  dmin * m_g * sum x        per 32 weights
-// What is dropped of an activation is below 2^-22 of it.  The instruction adds its sixteen products with the bits of fp32 below the
+// What is dropped of an activation is below 2^-22 of it, or below 2^-39 (high nibbles: 2^-35) of the largest of its 256 columns: next to
+// very much larger activations small ones lose bits that a scale per 32 columns would keep, and below that they vanish.  The instruction adds its sixteen products with the bits of fp32 below the
 // exponents' largest sum, and a code of a few bits has the exponent of 1024: a product loses what lies below 2^-14 of a code times the
 // largest activation of the sixteen, where gemv_kq.cuh's digits lose up to 2^-13.  Results are 4e-7 to 1.2e-6 from 64 bits at 4096
 // columns, those of the digits 2.2e-5.  The unpacking (a shift and four ANDs for eight weights, on a pipe that
@@ -41,7 +42,7 @@
 
 namespace zk {
 
-// kWide 0: one token; 1, 2: up to four or eight tokens.  Sixteen warps hide each other's chains of loads, unpacking and products; five
+// kWide 0: one token; 1, 2: up to four or eight tokens (and one of Q6_K).  Sixteen warps hide each other's chains of loads, unpacking and products; five
 // and more tokens have twice the products per weight and need more registers than that leaves.
 template <int kWide> __host__ __device__ constexpr int kqm_threads() { return kWide == 2 ? 256 : 512; }
 constexpr uint32_t kKqUnit = 256;      // columns of a unit: a super-block, or eight Q4_0 blocks
@@ -73,6 +74,7 @@ template <> struct KqmFormat<kFormatQ6KCodes> {      // codes [K] int8, sc, d
     static constexpr int kPlanes = 3, kSlots = 3, kSets = 4, kSums = 16;
     static constexpr uint32_t kHigh = 0, kSupers = 64;
 };
+template <int kFormat> constexpr bool kq_is_k45 = kFormat == 12 || kFormat == 13;      // alike but for the fifth bits
 template <int kFormat> constexpr bool kq_is_q6 = kFormat == 14 || kFormat == kFormatQ6KCodes;
 
 template <int kFormat> __host__ __device__ constexpr uint32_t kqm_words_bytes() { return KqmFormat<kFormat>::kSets * 1024; }
@@ -89,7 +91,7 @@ struct KqmParams {
     uint32_t ntasks, total_rows;
     const float* x;         // [batch][K] fp32; null with a gather: the vector gathered by the previous launch
     uint32_t K;             // columns, a multiple of the format's block size
-    uint32_t tokens, token_magic;   // token_magic: 2^32 / tokens, rounded up (two tokens and more)
+    uint32_t tokens, token_magic;   // token_magic: 2^32 / tokens, rounded up; 0 for one token
     uint32_t k_split;       // warps that share a tile: a power of two, at most the CTA's, and at most the units of a pass
     uint32_t pass_units;    // units whose activations are in shared memory at a time
     uint32_t pitch[kKqMaxPlanes];  // global row pitch of each plane, bytes
@@ -140,23 +142,25 @@ template <int kFormat> __device__ __forceinline__ uint32_t kq_high(uint32_t w, u
     return kFormat == 13 ? v | ((q5 << 7) & 0x01000100u) : v;
 }
 
-// Which launches come here (a B200; us of this kernel and of gemv_kq.cuh's).  One token: Q4_0 28672 x 4096 16.5 and 19.3, but 4096 x 14336
-// 14.7 and 14.9 and 6144 x 4096 7.4 and 6.4, where forming the operands in every CTA is most of it; Q4_K 17.0 and 24.9, 14.7 and 17.2, 7.7 and
-// 7.7; Q5_K 23.4 and 31.7, 18.7 and 21.2, 9.6 and 9.4; Q6_K, whose codes are bytes, 24.3 and 23.7, 17.9 and 16.5, 9.6 and 7.6.  Two tokens: Q4_0
-// 18.6 and 40.6, 18.4 and 24.6, 8.7 and 11.7; Q6_K 28.5 and 32.1, 24.3 and 21.6, 11.5 and 10.0.  Q6_K matrices of up to
-// a million weights, whose launches are all latency, stay with the digits whatever the tokens: a row's result then does not depend on the
-// rows that share its launch, as it did not before.
-inline bool kq_takes_mma(bool q4_0, bool q6, size_t tokens, uint64_t weights) {
-    if (q6 && weights <= (1u << 20)) return false;
-    if (tokens > 2) return true;
-    if (tokens == 2) return !q6 || weights >= (64u << 20);
-    return !q6 && weights >= (q4_0 ? 64u << 20 : 32u << 20);
-}
+// Which products come here: decided by format and columns alone, so that a row has the same arithmetic whatever tokens, tensors and rows
+// share its launch and whatever shard it is in (gemv_kq.cuh's digits are 2e-5 away).  A B200, us here and of the digits:
+//   one token      Q4_0         Q4_K         Q5_K          Q6_K          two tokens Q4_0  Q6_K         four tokens Q4_0  Q6_K
+//   256 x 1024      2.8   2.9    2.8   3.2    2.9    3.4    3.1    3.0    3.5   3.9    3.5   3.7     4.4   6.0     4.3   5.5
+//   1024 x 1024     3.1   2.8    3.2   3.1    3.3    3.3    3.5    3.0    3.9   3.9    3.9   3.7     4.6   6.0     4.6   5.5
+//   2048 x 2048     3.7   4.1    3.7   4.7    4.1    5.9    4.4    4.6    4.5   4.9    4.8   5.2     5.8   7.5     6.0   6.8
+//   8192 x 2048     5.7  10.2    5.8  12.5    7.2   16.8    8.2   12.2    6.7  11.1    8.6  12.6     7.9  16.0     9.7  14.0
+//   1536 x 4096     4.3   3.5    4.5   3.9    5.1    4.3    5.6    3.8    5.9   6.2    6.7   5.4     7.9  10.5     8.6   8.8
+//   6144 x 4096     6.8   6.3    7.1   7.5    8.9    9.0   10.2    7.4    8.4  11.5   11.2   9.7    10.4  20.1    13.0  15.7
+//   28672 x 4096   16.3  19.0   16.6  24.7   23.2   31.4   27.3   23.3   18.5  40.3   28.2  31.9    20.5  73.0    32.4  52.6
+//   4096 x 14336   14.3  14.7   14.5  17.0   18.5   21.0   20.4   16.3   18.2  24.5   24.0  21.6    21.8  34.5 (three tokens)
+// One token of Q6_K, whose codes are bytes here, costs up to half as much again from 4096 columns on, where the digits' rows arrive in whole
+// segments; there Q6_K stays with them for all tokens, at the price of the last column.
+inline bool kq_takes_mma(bool q6, uint32_t K) { return !q6 || K < static_cast<uint32_t>(kKqSegElems); }
 
 template <int kFormat, int kWide>
 __global__ void __launch_bounds__(kqm_threads<kWide>(), 1) gemv_kq_mma_kernel(const __grid_constant__ KqmParams p) {
     using F = KqmFormat<kFormat>;
-    static_assert(kWide || !kq_is_q6<kFormat>, "one token of Q6_K goes through gemv_kq.cuh");
+    static_assert(kWide || !kq_is_q6<kFormat>, "a column per block of a token is for blocks of 32 weights");
     constexpr int kThreads = kqm_threads<kWide>(), kWarps = kThreads / 32, kSlots = kqm_slots<kFormat, kWide>();
     constexpr bool kK45 = kq_is_k45<kFormat>, kQ6 = kq_is_q6<kFormat>, kCodes = kFormat == kFormatQ6KCodes;
     constexpr uint32_t kSlot = kqm_slot_bytes<kFormat>(), kHighAt = kqm_words_bytes<kFormat>(), kScalesAt = kqm_scales_at<kFormat>(), kSupersAt = kScalesAt + 256;
@@ -288,11 +292,12 @@ __global__ void __launch_bounds__(kqm_threads<kWide>(), 1) gemv_kq_mma_kernel(co
     auto prepare = [&](uint32_t pass) {
         const uint32_t first = pass * p.pass_units, jobs = pass_size(pass) * tokens;
         constexpr int kAtOnce = 4;
+        auto unit_of = [&](uint32_t j) { return kWide && p.token_magic ? __umulhi(j, p.token_magic) : j; };
         for (uint32_t j0 = warp; j0 < jobs; j0 += kWarps * kAtOnce) {
             float4 raw[kAtOnce][2];
 #pragma unroll
             for (int i = 0; i < kAtOnce; ++i) {
-                const uint32_t j = j0 + i * kWarps, unit = kWide ? __umulhi(j, p.token_magic) : j, token = kWide ? j - unit * tokens : 0, column = (first + unit) * kKqUnit + lane * 8;
+                const uint32_t j = j0 + i * kWarps, unit = unit_of(j), token = kWide ? j - unit * tokens : 0, column = (first + unit) * kKqUnit + lane * 8;
                 const bool live = j < jobs && column < p.K;
                 const float4* src = reinterpret_cast<const float4*>(x_src + (live ? static_cast<size_t>(token) * p.K + column : 0));
                 raw[i][0] = live ? __ldcg(src) : make_float4(0.f, 0.f, 0.f, 0.f);       // L2: coherent with peers' stores
@@ -300,7 +305,7 @@ __global__ void __launch_bounds__(kqm_threads<kWide>(), 1) gemv_kq_mma_kernel(co
             }
 #pragma unroll
             for (int i = 0; i < kAtOnce; ++i) {
-                const uint32_t j = j0 + i * kWarps, unit = kWide ? __umulhi(j, p.token_magic) : j, token = kWide ? j - unit * tokens : 0;
+                const uint32_t j = j0 + i * kWarps, unit = unit_of(j), token = kWide ? j - unit * tokens : 0;
                 if (j >= jobs) break;
                 float v[8] = {raw[i][0].x, raw[i][0].y, raw[i][0].z, raw[i][0].w, raw[i][1].x, raw[i][1].y, raw[i][1].z, raw[i][1].w};
                 float most = 0.0f;

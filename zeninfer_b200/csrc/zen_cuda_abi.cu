@@ -588,20 +588,17 @@ cudaError_t dispatch_kq_mma(State& s, zk::KqmParams& p, unsigned grid, bool stas
 
 template <int kFormat>
 cudaError_t dispatch_kq(size_t tokens, const zk::KqParams& p, unsigned grid, size_t smem, cudaStream_t st, bool pdl) {
-    if (tokens == 1) return launch_gemv_kq<kFormat, 1>(p, grid, smem, st, pdl);
-    if constexpr (zk::kq_is_q6<kFormat>) {
-        switch (tokens) {
-        case 2: return launch_gemv_kq<kFormat, 2>(p, grid, smem, st, pdl);
-        case 3: return launch_gemv_kq<kFormat, 3>(p, grid, smem, st, pdl);
-        case 4: return launch_gemv_kq<kFormat, 4>(p, grid, smem, st, pdl);
-        case 5: return launch_gemv_kq<kFormat, 5>(p, grid, smem, st, pdl);
-        case 6: return launch_gemv_kq<kFormat, 6>(p, grid, smem, st, pdl);
-        case 7: return launch_gemv_kq<kFormat, 7>(p, grid, smem, st, pdl);
-        case 8: return launch_gemv_kq<kFormat, 8>(p, grid, smem, st, pdl);
-        default: break;
-        }
+    switch (tokens) {
+    case 1: return launch_gemv_kq<kFormat, 1>(p, grid, smem, st, pdl);
+    case 2: return launch_gemv_kq<kFormat, 2>(p, grid, smem, st, pdl);
+    case 3: return launch_gemv_kq<kFormat, 3>(p, grid, smem, st, pdl);
+    case 4: return launch_gemv_kq<kFormat, 4>(p, grid, smem, st, pdl);
+    case 5: return launch_gemv_kq<kFormat, 5>(p, grid, smem, st, pdl);
+    case 6: return launch_gemv_kq<kFormat, 6>(p, grid, smem, st, pdl);
+    case 7: return launch_gemv_kq<kFormat, 7>(p, grid, smem, st, pdl);
+    case 8: return launch_gemv_kq<kFormat, 8>(p, grid, smem, st, pdl);
+    default: return cudaErrorInvalidValue;
     }
-    return cudaErrorInvalidValue;
 }
 
 size_t gemv_smem_bytes(int format, size_t cols, size_t tokens, int act_mode) {   // format: a kernel format (zen_cuda_weights::kernel_format)
@@ -610,11 +607,9 @@ size_t gemv_smem_bytes(int format, size_t cols, size_t tokens, int act_mode) {  
         return zk::gemv_q8_0_smem_bytes(nseg, static_cast<int>(tokens), act_mode == ZEN_CUDA_ACT_FP32 ? 2 : 1);
     }
     const uint32_t nseg = static_cast<uint32_t>((cols + zk::kKqSegElems - 1) / zk::kKqSegElems);
-    return format == ZEN_CUDA_Q4_0   ? zk::gemv_kq_smem_bytes<ZEN_CUDA_Q4_0>(nseg, static_cast<int>(tokens))
-           : format == ZEN_CUDA_Q4_K ? zk::gemv_kq_smem_bytes<ZEN_CUDA_Q4_K>(nseg, static_cast<int>(tokens))
-           : format == ZEN_CUDA_Q5_K ? zk::gemv_kq_smem_bytes<ZEN_CUDA_Q5_K>(nseg, static_cast<int>(tokens))
+    return format == ZEN_CUDA_Q6_K         ? zk::gemv_kq_smem_bytes<ZEN_CUDA_Q6_K>(nseg, static_cast<int>(tokens))
            : format == zk::kFormatQ6KCodes ? zk::gemv_kq_smem_bytes<zk::kFormatQ6KCodes>(nseg, static_cast<int>(tokens))
-                                     : zk::gemv_kq_smem_bytes<ZEN_CUDA_Q6_K>(nseg, static_cast<int>(tokens));
+                                           : zk::gemv_kq_limit_bytes(format, nseg, static_cast<int>(tokens));
 }
 
 // Largest number of activation rows (<= 8) one launch can keep in shared memory beside the weight ring; 0 if not even one.
@@ -661,17 +656,17 @@ bool enqueue_gemv_kq(State& s, const zen_cuda_weights* const* w, float* const* d
                                  : std::max(1u, std::min<unsigned>((total_rows + zk::kGemvWarps - 1) / zk::kGemvWarps, static_cast<unsigned>(s.sm_count)));
     const size_t smem = gemv_smem_bytes(fmt, w[0]->cols, tokens, ZEN_CUDA_ACT_FP32)
                         + (gather ? zk::gather_stash_bytes(total_rows, grid, static_cast<int>(tokens)) : 0);
-    // the limit of the entry points, which callers split their tokens by; the matrix instructions' kernel takes longer inputs in passes
+    // the limit of the entry points, which callers split their tokens by; the matrix instructions' kernel would take longer inputs in passes
     if (smem > s.smem_optin) return set_error(s, "gemv: activation rows do not fit shared memory (columns x tokens too large)");
     const bool q6 = fmt == ZEN_CUDA_Q6_K || fmt == zk::kFormatQ6KCodes;
     cudaError_t e;
-    if (zk::kq_takes_mma(fmt == ZEN_CUDA_Q4_0, q6, tokens, static_cast<uint64_t>(total_rows) * p.K)) {
+    if (zk::kq_takes_mma(q6, p.K)) {
         zk::KqmParams m{};
         std::copy(std::begin(p.task), std::end(p.task), std::begin(m.task));
         std::copy(std::begin(p.pitch), std::end(p.pitch), std::begin(m.pitch));
         m.ntasks = p.ntasks; m.total_rows = total_rows; m.x = d_x; m.K = p.K; m.error_word = s.d_error; m.gather = p.gather;
         m.tokens = static_cast<uint32_t>(tokens);
-        m.token_magic = static_cast<uint32_t>(((uint64_t(1) << 32) + tokens - 1) / tokens);
+        m.token_magic = tokens == 1 ? 0 : static_cast<uint32_t>(((uint64_t(1) << 32) + tokens - 1) / tokens);
         const unsigned g = gather ? grid : 0;
         e = fmt == ZEN_CUDA_Q4_0   ? dispatch_kq_mma<ZEN_CUDA_Q4_0>(s, m, g, gather != nullptr, st)
             : fmt == ZEN_CUDA_Q4_K ? dispatch_kq_mma<ZEN_CUDA_Q4_K>(s, m, g, gather != nullptr, st)
@@ -679,11 +674,8 @@ bool enqueue_gemv_kq(State& s, const zen_cuda_weights* const* w, float* const* d
             : fmt == zk::kFormatQ6KCodes ? dispatch_kq_mma<zk::kFormatQ6KCodes>(s, m, g, gather != nullptr, st)
                                          : dispatch_kq_mma<ZEN_CUDA_Q6_K>(s, m, g, gather != nullptr, st);
     } else {
-        e = fmt == ZEN_CUDA_Q4_0   ? dispatch_kq<ZEN_CUDA_Q4_0>(tokens, p, grid, smem, st, s.pdl)
-            : fmt == ZEN_CUDA_Q4_K ? dispatch_kq<ZEN_CUDA_Q4_K>(tokens, p, grid, smem, st, s.pdl)
-            : fmt == ZEN_CUDA_Q5_K ? dispatch_kq<ZEN_CUDA_Q5_K>(tokens, p, grid, smem, st, s.pdl)
-            : fmt == zk::kFormatQ6KCodes ? dispatch_kq<zk::kFormatQ6KCodes>(tokens, p, grid, smem, st, s.pdl)
-                                         : dispatch_kq<ZEN_CUDA_Q6_K>(tokens, p, grid, smem, st, s.pdl);
+        e = fmt == zk::kFormatQ6KCodes ? dispatch_kq<zk::kFormatQ6KCodes>(tokens, p, grid, smem, st, s.pdl)
+                                       : dispatch_kq<ZEN_CUDA_Q6_K>(tokens, p, grid, smem, st, s.pdl);
     }
     if (e != cudaSuccess) return set_error(s, std::string("gemv launch: ") + cudaGetErrorString(e));
     ++s.stats.dispatches;
@@ -946,7 +938,7 @@ bool make_tile_maps(State& s, zen_cuda_weights* w) {
     return true;
 }
 
-// The same for the planes of the Q4_0 / Q6_K / Q4_K / Q5_K kernel (zk::KqTileMaps): per plane the row pitch and the bytes
+// The same for the planes of gemv_kq.cuh's Q6_K (zk::KqTileMaps): per plane the row pitch and the bytes
 // of one 4096-column segment; planes wider than 256 bytes a segment need a pitch that is a multiple of 256.
 bool make_kq_tile_maps(State& s, zen_cuda_weights* w) {
     if (w->cols <= static_cast<size_t>(zk::kKqSegElems) || !s.encode_tiled) return true;
@@ -954,11 +946,8 @@ bool make_kq_tile_maps(State& s, zen_cuda_weights* w) {
     size_t pitch[4] = {0, 0, 0, 0}, seg[4] = {0, 0, 0, 0};
     int planes = 0;
     const size_t K = w->cols, E = zk::kKqSegElems;
-    if (kf == ZEN_CUDA_Q4_0) { planes = 2; pitch[0] = K / 2; seg[0] = E / 2; pitch[1] = size_t(w->nbp) * 2; seg[1] = E / 32 * 2; }
-    else if (kf == ZEN_CUDA_Q6_K) { planes = 4; pitch[0] = K / 2; seg[0] = E / 2; pitch[1] = K / 4; seg[1] = E / 4; pitch[2] = K / 16; seg[2] = E / 16; pitch[3] = size_t(w->nbp) * 2; seg[3] = E / 256 * 2; }
+    if (kf == ZEN_CUDA_Q6_K) { planes = 4; pitch[0] = K / 2; seg[0] = E / 2; pitch[1] = K / 4; seg[1] = E / 4; pitch[2] = K / 16; seg[2] = E / 16; pitch[3] = size_t(w->nbp) * 2; seg[3] = E / 256 * 2; }
     else if (kf == zk::kFormatQ6KCodes) { planes = 3; pitch[0] = K; seg[0] = E; pitch[1] = K / 16; seg[1] = E / 16; pitch[2] = size_t(w->nbp) * 2; seg[2] = E / 256 * 2; }
-    else if (kf == ZEN_CUDA_Q4_K) { planes = 3; pitch[0] = K / 2; seg[0] = E / 2; pitch[1] = K / 16; seg[1] = E / 16; pitch[2] = size_t(w->nbp) * 4; seg[2] = E / 256 * 4; }
-    else if (kf == ZEN_CUDA_Q5_K) { planes = 4; pitch[0] = K / 2; seg[0] = E / 2; pitch[1] = K / 8; seg[1] = E / 8; pitch[2] = K / 16; seg[2] = E / 16; pitch[3] = size_t(w->nbp) * 4; seg[3] = E / 256 * 4; }
     else return true;
     for (int pl = 0; pl < planes; ++pl)
         if (pitch[pl] % 16 || (seg[pl] > 256 && pitch[pl] % 256)) return true;   // no maps: the rows go one copy each
