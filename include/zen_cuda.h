@@ -198,8 +198,11 @@ void zen_cuda_dev_free(zen_cuda_weights* w);
 size_t zen_cuda_dev_weight_bytes(const zen_cuda_weights* w); /* device bytes held */
 
 /* y[i] = W[i] * x for up to ZEN_CUDA_MAX_BATCH tensors of the same format and column count
- * sharing x.  d_x: device fp32 [tokens][columns] (tokens <= 8); d_y[i]: device fp32
- * [tokens][rows_i].  Enqueued on `stream` (a cudaStream_t, or NULL for the backend's own
+ * sharing x.  d_x: device fp32 [tokens][columns], 16-byte aligned (tokens <= 8, and fewer where the activations of long rows
+ * would not fit shared memory: three of 14336 columns in Q4_0, Q4_K and Q5_K, two in Q6_K); d_y[i]: device fp32
+ * [tokens][rows_i].  The bits of a Q4_0, Q6_K, Q4_K or Q5_K row depend on its columns, its activations and the number of tokens, not on the
+ * tensors and rows that share the launch nor on the shard it is in; with other numbers of tokens they differ by the order of
+ * fp32 additions (about 1e-6).  Enqueued on `stream` (a cudaStream_t, or NULL for the backend's own
  * stream); returns without synchronising.  act_mode is ZEN_CUDA_ACT_*. */
 int zen_cuda_dev_gemv(const zen_cuda_weights* const* w, float* const* d_y, size_t count, const float* d_x,
                       size_t tokens, int act_mode, void* stream);

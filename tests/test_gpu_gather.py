@@ -54,6 +54,55 @@ def test_single_rank_gather_equals_plain_product(be, fmt, mode, tokens):
     be.dev_free(h)
 
 
+# The small formats' kernels: one token, two to four, five to eight; matrices of a million weights and more; inputs that are taken in passes; a
+# slice whose rows are taken in blocks.  slot: the gather's grid comes from it, a plain launch's from the rows.
+@pytest.mark.parametrize("fmt,name,rows,cols,tokens,slot", [
+    (blocks.Q4_0, "Q4_0", 1500, 4096, 1, 1), (blocks.Q4_0, "Q4_0", 700, 14336, 3, 2), (blocks.Q4_K, "Q4_K", 2048, 2048, 1, 4), (blocks.Q5_K, "Q5_K", 900, 4096, 6, 1),
+    (blocks.Q4_K, "Q4_K", 40000, 1024, 8, 1), (blocks.Q6_K, "Q6_K", 3000, 2048, 1, 1), (blocks.Q6_K, "Q6_K", 3000, 2048, 5, 3), (blocks.Q6_K, "Q6_K", 1000, 4096, 4, 2)])
+def test_single_rank_gather_of_the_small_formats(be, fmt, name, rows, cols, tokens, slot):
+    import torch
+    part = blocks.random_k_blocks(fmt, 50, cols, 7) if fmt in (blocks.Q4_K, blocks.Q5_K) else seeded_weights(fmt, 50, cols, 7)
+    h = be.dev_upload(name, np.ascontiguousarray(np.tile(part, (rows // 50 + 1, 1))[:rows]), rows, cols)
+    pg = shard.PeerGather(be, 1, 0, slot * tokens * rows)
+    x = torch.from_numpy(seeded_acts(tokens, cols, 8)).cuda()
+    want, got = torch.zeros((tokens, rows), device="cuda"), torch.zeros(slot * tokens * rows, device="cuda")
+    stream = torch.cuda.Stream()
+    stream.wait_stream(torch.cuda.current_stream())
+    be.dev_gemv([h], [want.data_ptr()], x.data_ptr(), tokens, ACT_FP32, stream.cuda_stream)
+    for _ in range(3):
+        pg.gemv([h], x.data_ptr(), tokens, ACT_FP32, stream.cuda_stream)
+    pg.fetch(got.data_ptr(), stream.cuda_stream)
+    stream.synchronize()
+    be.dev_check(stream.cuda_stream)
+    assert torch.equal(got[: tokens * rows].view(tokens, rows), want)
+    pg.close()
+    be.dev_free(h)
+
+
+@pytest.mark.parametrize("fmt,name,n", [(blocks.Q4_0, "Q4_0", 1024), (blocks.Q4_K, "Q4_K", 4096), (blocks.Q6_K, "Q6_K", 2048), (blocks.Q6_K, "Q6_K", 4096)])
+def test_single_rank_chain_of_the_small_formats(be, fmt, name, n):
+    import torch
+    w = blocks.random_k_blocks(fmt, n, n, 9) if fmt in (blocks.Q4_K, blocks.Q5_K) else seeded_weights(fmt, n, n, 9)
+    h = be.dev_upload(name, w, n, n)
+    pg = shard.PeerGather(be, 1, 0, n)
+    stream = torch.cuda.Stream()
+    a = torch.from_numpy(seeded_acts(1, n, 10)).cuda()
+    b, got = torch.zeros_like(a), torch.zeros(n, device="cuda")
+    stream.wait_stream(torch.cuda.current_stream())
+    for i in range(4):
+        pg.gemv([h], None if i else a.data_ptr(), 1, ACT_FP32, stream.cuda_stream)
+    pg.fetch(got.data_ptr(), stream.cuda_stream)
+    stream.synchronize()
+    for _ in range(4):
+        be.dev_gemv([h], [b.data_ptr()], a.data_ptr(), 1, ACT_FP32, stream.cuda_stream)
+        a, b = b, a
+    stream.synchronize()
+    be.dev_check(stream.cuda_stream)
+    assert torch.equal(got, a[0]) and bool(torch.isfinite(got).all())
+    pg.close()
+    be.dev_free(h)
+
+
 def test_single_rank_chain_reads_previous_gather(be):
     """x of launch n+1 is what launch n gathered (d_x = None): a chain y <- W y against the same chain made of plain
     launches through an ordinary buffer."""

@@ -189,6 +189,37 @@ def test_what_shares_a_launch_does_not_choose_a_rows_arithmetic(be, name, cols):
         assert apart(_rows_of(be, name, [large, w], x[:tokens], cols)[1]) < 5e-6
 
 
+# A row's bits depend on its columns and tokens only: alone, in shards, beside other tensors, in slices that are taken in blocks and passes.
+@pytest.mark.parametrize("name", list(ALL))
+@pytest.mark.parametrize("cols,tokens", [(256, 1), (1024, 2), (2048, 5), (3840, 1), (3840, 4), (4096, 1), (4096, 4), (4096, 8), (11008, 2), (14336, 1)])
+def test_a_rows_bits_are_the_same_in_any_launch(be, name, cols, tokens):
+    fmt, rows = ALL[name], 300
+    w, x = _weights(fmt, rows, cols, cols), seeded_acts(tokens, cols, cols + 1)
+    whole, = _rows_of(be, name, [w], x, cols)
+    for cut in (1, 100, 284):
+        assert np.array_equal(np.concatenate([_rows_of(be, name, [part], x, cols)[0] for part in (w[:cut], w[cut:])], axis=1), whole)
+    for more in (2_000, 24_000, 130_000):
+        if more * cols > 140 << 20:
+            break
+        other = np.ascontiguousarray(np.tile(w[:100], (more // 100, 1)))
+        first, got, last = _rows_of(be, name, [other, w, w[:77]], x, cols)
+        assert np.array_equal(got, whole) and np.array_equal(last, whole[:, :77])
+        assert np.array_equal(first, np.tile(whole[:, :100], (1, more // 100)))
+
+
+@pytest.mark.parametrize("rows,cols,tokens", [(14336, 4096, 4), (28672, 2048, 4), (70000, 2048, 4), (70000, 1024, 8), (9000, 3840, 1)])
+def test_q6_k_layouts_give_the_same_bits_for_many_rows(be, rows, cols, tokens):
+    w, x = np.ascontiguousarray(np.tile(_weights(blocks.Q6_K, 40, cols, 1), (rows // 40 + 1, 1))[:rows]), seeded_acts(tokens, cols, 2)
+    before, got = be.set_q6k_codes(True), []
+    try:
+        for codes in (True, False):
+            be.set_q6k_codes(codes)
+            got.append(_products(be, "Q6_K", w, x, rows, cols))
+    finally:
+        be.set_q6k_codes(before)
+    assert np.array_equal(got[0], got[1])
+
+
 # edges of tiles (16 rows), of units (256 columns; Q4_0 ends inside one), of warps' shares; one or more groups of four tokens;
 # 16384 columns by three tokens and 14336 by two or three go over the row in several passes
 @pytest.mark.parametrize("name", list(ALL))

@@ -92,14 +92,26 @@ struct KqmParams {
     const float* x;         // [batch][K] fp32; null with a gather: the vector gathered by the previous launch
     uint32_t K;             // columns, a multiple of the format's block size
     uint32_t tokens, token_magic;   // token_magic: 2^32 / tokens, rounded up; 0 for one token
-    uint32_t k_split;       // warps that share a tile: a power of two, at most the CTA's, and at most the units of a pass
+    uint32_t partials;      // sums that a row is added up from (kqm_partials)
+    uint32_t k_split;       // warps that share a tile: a power of two, at most `partials`
     uint32_t pass_units;    // units whose activations are in shared memory at a time
+    uint32_t block_rows;    // rows of a slice whose sums are in shared memory at a time: all of it, or whole tiles
+    uint32_t sums_ld;       // floats between the sums of two tokens
     uint32_t pitch[kKqMaxPlanes];  // global row pitch of each plane, bytes
     int* error_word;
     PeerGather gather;      // world == 0: outputs go to task[].y only
 };
 
 __host__ __device__ inline uint32_t kqm_units(uint32_t K) { return (K + kKqUnit - 1) / kKqUnit; }
+// A row is added up from so many sums, of every kqm_partials-th unit each.  The number comes from the columns and the kernel's width
+// alone, not from how many warps share a tile: a row's bits then depend neither on the tensors and rows of its launch nor on the
+// shard it is in.  As many as warps may share a tile; long rows of several tokens, whose activations take the shared memory, do with eight.
+template <int kWide> inline uint32_t kqm_partials(uint32_t units) {
+    const uint32_t most = kWide == 2 || (kWide == 1 && units >= 48) ? 8 : 16;
+    uint32_t n = 1;
+    while (2 * n <= most && 2 * n <= units) n *= 2;
+    return n;
+}
 
 // 16 or 4 bytes global -> shared, or 16 zero bytes.
 __device__ __forceinline__ void kq_copy16(uint32_t dst, const void* src) {
@@ -171,36 +183,36 @@ __global__ void __launch_bounds__(kqm_threads<kWide>(), 1) gemv_kq_mma_kernel(co
     uint8_t* const xop = smem + kqm_ring_bytes<kFormat, kWide>();                // [unit of the pass][1024 * tokens]
     float* const xscale = reinterpret_cast<float*>(xop + static_cast<size_t>(p.pass_units) * tokens * 1024);     // [unit][token]
     float* const xsum = xscale + ((p.pass_units * tokens + 3) & ~3u);                                            // [unit][token][kSums]
-    float* const sums = xsum + p.pass_units * tokens * F::kSums;                                  // [k_split][token][row of the slice]
+    const uint32_t span = p.block_rows, ld = p.sums_ld;
+    float* const sums = xsum + p.pass_units * tokens * F::kSums;                                  // [partial][token][row of the block]
+    float* const stash = sums + static_cast<size_t>(p.partials) * tokens * ld;                  // gather only: [token][row of the slice]
     uint32_t r_first, r_last;
     cta_row_slice(p.total_rows, blockIdx.x, gridDim.x, r_first, r_last);
     const uint32_t n_mine = r_last - r_first, units = kqm_units(p.K), ks = p.k_split;
-    float* const stash = ks == 1 ? sums : sums + static_cast<size_t>(n_mine) * ks * tokens;                      // gather only: [token][row of the slice]
     const uint32_t team = warp / ks, part = warp % ks, teams = kWarps / ks;
     pdl_launch_dependents();
 
-    // A warp's steps are (pass, unit, task, tile), in this order: a unit's activations stay in its registers while it goes over the
-    // rows.  (Read anew for every tile they took 32 of the 117 wavefronts of shared memory a step, where HBM allows 90 clocks.)
-    // Rows past the slice's end ask for its last row once more; their sums are not used.
+    // A warp's steps are (block of rows, pass, unit, task, tile), in this order: a unit's activations stay in its registers while it goes
+    // over the rows.  (Read anew for every tile they took 32 of the 117 wavefronts of shared memory a step, where HBM allows 90 clocks.)
+    // Rows past the block's end ask for its last row once more; their sums are not used.
     struct Walk {                                                // what is asked for next
         const uint8_t *words, *scales, *supers, *high;           // the lane's place in row 0 of the task, at the unit
-        uint32_t ti, r, r_end, u, pass;                          // r: the tile's first row in its task; u: the unit in its pass
-        bool over;
+        uint32_t ti, r, r_end, u, pass, first;                   // r: the tile's first row in its task; u: the unit in its pass; first: the block's first row, the slice's end behind the last step
     };
     const uint32_t stride = teams * kKqTile;
     auto pass_size = [&](uint32_t pass) { return min(p.pass_units, units - pass * p.pass_units); };
-    auto rows_of = [&](uint32_t ti, uint32_t& r, uint32_t& r_end) {      // the team's first tile of a task; false where it has none
+    auto rows_of = [&](uint32_t first, uint32_t ti, uint32_t& r, uint32_t& r_end) {      // the team's first tile of a task in a block; false where it has none
         const KqTask& k = p.task[ti];
-        const uint32_t a = max(r_first, k.first_row) + team * kKqTile, b = min(r_last, k.first_row + k.rows);
+        const uint32_t a = max(first, k.first_row) + team * kKqTile, b = min(min(first + span, r_last), k.first_row + k.rows);
         r = a - k.first_row;
         r_end = b - k.first_row;
         return a < b;
     };
     auto enter = [&](Walk& w) {      // from task ti of unit u on
-        while (w.pass * p.pass_units < units) {
+        while (w.first < r_last) {
             if (w.u < pass_size(w.pass)) {
                 for (; w.ti < p.ntasks; ++w.ti) {
-                    if (!rows_of(w.ti, w.r, w.r_end)) continue;
+                    if (!rows_of(w.first, w.ti, w.r, w.r_end)) continue;
                     const KqTask& k = p.task[w.ti];
                     const uint32_t unit = w.pass * p.pass_units + w.u;
                     w.words = k.plane[0] + unit * kUnitBytes + t * 16;
@@ -212,12 +224,14 @@ __global__ void __launch_bounds__(kqm_threads<kWide>(), 1) gemv_kq_mma_kernel(co
                 }
                 w.u += ks;
             } else {
-                ++w.pass;
                 w.u = part;
+                if (++w.pass * p.pass_units >= units) {
+                    w.pass = 0;
+                    w.first += min(span, r_last - w.first);
+                }
             }
             w.ti = 0;
         }
-        w.over = true;
     };
     auto advance = [&](Walk& w) {
         w.r += stride;
@@ -260,10 +274,11 @@ __global__ void __launch_bounds__(kqm_threads<kWide>(), 1) gemv_kq_mma_kernel(co
     };
     Walk in{};
     in.u = part;
+    in.first = r_first;
     enter(in);
 #pragma unroll
     for (int s = 0; s < kSlots; ++s) {
-        if (!in.over) { ask(in, s); advance(in); }
+        if (in.first < r_last) { ask(in, s); advance(in); }
         asm volatile("cp.async.commit_group;" ::: "memory");
     }
 
@@ -560,61 +575,63 @@ __global__ void __launch_bounds__(kqm_threads<kWide>(), 1) gemv_kq_mma_kernel(co
     };
 
     int slot = 0;
-    for (uint32_t pass = 0; pass * p.pass_units < units && !failed; ++pass) {
-        if (pass) __syncthreads();
-        prepare(pass);
-        __syncthreads();
-        const uint32_t count = pass_size(pass);
-        for (uint32_t u = part; u < count; u += ks) {
-            take(u);
-            const bool add = pass || u >= ks;
-            const uint32_t unit = pass * p.pass_units + u;
-            for (uint32_t ti = 0; ti < p.ntasks; ++ti) {
-                uint32_t r, r_end;
-                if (!rows_of(ti, r, r_end)) continue;
-                const uint32_t token = kWide ? t : 0;
-                float* to = sums + (part * tokens + token) * n_mine + (p.task[ti].first_row + r + g - r_first);      // [part][token][row]
-                for (; r < r_end; r += stride, to += stride) {
-                    asm volatile("cp.async.wait_group %0;" ::"n"(kSlots - 1) : "memory");
-                    __syncwarp();
-                    float v[kN][2];
-                    const uint8_t* st = ring + slot * kSlot;
-                    if constexpr (kWide == 0) consume_one(st, v[0]);
-                    else consume_several(st, unit, v);
-                    __syncwarp();                 // every lane has read the slot
-                    if (!in.over) { ask(in, slot); advance(in); }
-                    asm volatile("cp.async.commit_group;" ::: "memory");
-                    if (++slot == kSlots) slot = 0;
-                    if (kWide == 0 && t) continue;
-                    const uint32_t rows = r_end - r;
+    for (uint32_t first = r_first; first < r_last && !failed; first += span) {
+        for (uint32_t pass = 0; pass * p.pass_units < units; ++pass) {
+            if (pass || first != r_first) __syncthreads();                     // the operands and sums of before have been read
+            if (first == r_first || p.pass_units < units) prepare(pass);       // operands of all units stay
+            __syncthreads();
+            const uint32_t count = pass_size(pass);
+            for (uint32_t u = part; u < count; u += ks) {
+                take(u);
+                const uint32_t unit = pass * p.pass_units + u;
+                const bool add = unit >= p.partials;
+                for (uint32_t ti = 0; ti < p.ntasks; ++ti) {
+                    uint32_t r, r_end;
+                    if (!rows_of(first, ti, r, r_end)) continue;
+                    const uint32_t token = kWide ? t : 0;
+                    float* to = sums + ((unit & (p.partials - 1)) * tokens + token) * ld + (p.task[ti].first_row + r + g - first);
+                    for (; r < r_end; r += stride, to += stride) {
+                        asm volatile("cp.async.wait_group %0;" ::"n"(kSlots - 1) : "memory");
+                        __syncwarp();
+                        float v[kN][2];
+                        const uint8_t* st = ring + slot * kSlot;
+                        if constexpr (kWide == 0) consume_one(st, v[0]);
+                        else consume_several(st, unit, v);
+                        __syncwarp();                 // every lane has read the slot
+                        if (in.first < r_last) { ask(in, slot); advance(in); }
+                        asm volatile("cp.async.commit_group;" ::: "memory");
+                        if (++slot == kSlots) slot = 0;
+                        if (kWide == 0 && t) continue;
+                        const uint32_t rows = r_end - r;
 #pragma unroll
-                    for (int n = 0; n < kN; ++n) {
-                        if (kWide && token + 4 * n >= tokens) break;
-                        float* sum = to + 4 * n * n_mine;
-                        if (g < rows) *sum = add ? *sum + v[n][0] : v[n][0];
-                        if (g + 8 < rows) sum[8] = add ? sum[8] + v[n][1] : v[n][1];
+                        for (int n = 0; n < kN; ++n) {
+                            if (kWide && token + 4 * n >= tokens) break;
+                            float* sum = to + 4 * n * ld;
+                            if (g < rows) *sum = add ? *sum + v[n][0] : v[n][0];
+                            if (g + 8 < rows) sum[8] = add ? sum[8] + v[n][1] : v[n][1];
+                        }
                     }
                 }
             }
         }
-    }
-    asm volatile("cp.async.wait_all;" ::: "memory");
-    __syncthreads();
-    const uint32_t parts = min(ks, pass_size(0));
-    for (uint32_t token = 0; token < tokens && !failed; ++token) {
-        for (uint32_t i = threadIdx.x; i < n_mine; i += kThreads) {
-            const uint32_t row = r_first + i;
-            uint32_t ti = 0;
-            while (row >= p.task[ti].first_row + p.task[ti].rows) ++ti;
-            const KqTask& k = p.task[ti];
-            float v = 0.0f;
+        __syncthreads();
+        const uint32_t count = min(span, r_last - first);
+        for (uint32_t token = 0; token < tokens; ++token) {
+            for (uint32_t i = threadIdx.x; i < count; i += kThreads) {
+                const uint32_t row = first + i;
+                uint32_t ti = 0;
+                while (row >= p.task[ti].first_row + p.task[ti].rows) ++ti;
+                const KqTask& k = p.task[ti];
+                float v = 0.0f;
 #pragma unroll 4
-            for (uint32_t s = 0; s < parts; ++s) v += sums[(s * tokens + token) * n_mine + i];
-            v *= 4096.0f;                     // 2^24 of the weights, 2^12 of which are in the activations' scales
-            if (k.y) k.y[static_cast<size_t>(token) * k.rows + (row - k.first_row)] = v;
-            if (p.gather.world) stash[token * n_mine + i] = v;
+                for (uint32_t s = 0; s < p.partials; ++s) v += sums[(s * tokens + token) * ld + i];
+                v *= 4096.0f;                     // 2^24 of the weights, 2^12 of which are in the activations' scales
+                if (k.y) k.y[static_cast<size_t>(token) * k.rows + (row - k.first_row)] = v;
+                if (p.gather.world) stash[token * n_mine + (row - r_first)] = v;
+            }
         }
     }
+    asm volatile("cp.async.wait_all;" ::: "memory");
     if (p.gather.world) {
         __syncthreads();
         // With an input of its own the launch needs the other ranks only now: they must have finished the previous

@@ -533,31 +533,43 @@ cudaError_t launch_gemv_kq_mma(State& s, zk::KqmParams& p, unsigned grid, bool s
     constexpr uint32_t kWarps = zk::kqm_threads<kWide>() / 32;
     const uint32_t units = zk::kqm_units(p.K);
     const size_t unit = static_cast<size_t>(p.tokens) * zk::kqm_unit_bytes<kFormat>(), most = s.smem_optin;
-    const bool choose = grid == 0;      // otherwise the gather's, whose outputs are collected in shared memory (stash)
-    if (choose) grid = std::max(1u, std::min<unsigned>((p.total_rows + 7) / 8, static_cast<unsigned>(s.sm_count)));
-    // The warps of a CTA share tiles and units so that the busiest has the fewest steps; with equal counts a tile goes to fewer
-    // warps, whose partial sums take less shared memory.  Sums and activations have to leave room for the ring.
-    size_t fixed = 0;
-    auto split = [&] {
-        const uint32_t slice = (p.total_rows + grid - 1) / grid, tiles = (slice + zk::kKqTile - 1) / zk::kKqTile;
-        uint32_t best = 0;
-        for (uint32_t k = 1; k <= kWarps && k <= units; k *= 2) {
-            const size_t sums = static_cast<size_t>(slice) * p.tokens * (k + (stash && k > 1 ? 1 : 0)) * sizeof(float);
-            const size_t bytes = zk::kqm_ring_bytes<kFormat, kWide>() + 16 + sums;
-            if (bytes + k * unit > most) break;
-            const uint32_t teams = kWarps / k, steps = (tiles + teams - 1) / teams * ((units + k - 1) / k);
-            if (!best || steps < best) { best = steps; p.k_split = k; fixed = bytes; }
+    if (!grid)      // otherwise the gather's, whose outputs are collected in shared memory (stash)
+        grid = std::max(1u, std::min<unsigned>((p.total_rows + 7) / 8, static_cast<unsigned>(s.sm_count)));
+    const uint32_t slice = (p.total_rows + grid - 1) / grid;
+    p.partials = zk::kqm_partials<kWide>(units);
+    const size_t fixed = zk::kqm_ring_bytes<kFormat, kWide>() + 16 + (stash ? slice * p.tokens * sizeof(float) : 0);
+    // Beside the ring, shared memory has the sums of a block of rows and the activations of the units of a pass; rows and units that do
+    // not fit are taken after one another.  The warps share tiles and units so that the busiest has the fewest steps; a block counts as
+    // four of them (6144 x 4096 times eight tokens in three blocks instead of two passes: 26.3 us and 18.7), a pass's barriers as
+    // two, four units' operands that a warp forms as one.
+    const size_t row_sums = p.partials * p.tokens * sizeof(float);
+    uint64_t best = 0;
+    for (uint32_t n = 1; n <= units && (n <= 8 || !best); ++n) {
+        for (uint32_t k = 1; k <= p.partials; k *= 2) {
+            const uint32_t pass = std::min(units, ((units + n - 1) / n + k - 1) / k * k), passes = (units + pass - 1) / pass;
+            if (fixed + pass * unit + zk::kKqTile * row_sums > most) continue;
+            const uint32_t room = static_cast<uint32_t>(std::min<size_t>(slice, (most - fixed - pass * unit) / row_sums));
+            uint32_t rows = slice, tiles = (slice + zk::kKqTile - 1) / zk::kKqTile, blocks = 1;
+            if (room < slice) {
+                blocks = (tiles + room / zk::kKqTile - 1) / (room / zk::kKqTile);
+                tiles = (tiles + blocks - 1) / blocks;
+                rows = tiles * zk::kKqTile;
+            }
+            const uint32_t teams = kWarps / k, formed = passes == 1 ? 1 : blocks;      // formed: times that all units' operands are
+            const uint64_t steps = uint64_t(blocks) * ((tiles + teams - 1) / teams) * ((passes - 1) * (pass / k) + (units - (passes - 1) * pass + k - 1) / k);
+            const uint64_t cost = steps + 4 * blocks + 2 * passes * formed + formed * (units * p.tokens / (4 * kWarps));
+            if (!best || cost < best) {
+                best = cost;
+                p.k_split = k; p.pass_units = pass; p.block_rows = rows;
+                // several tokens' sums lie in different banks where their pitch is 8 modulo 16
+                const uint32_t apart = (rows + 7) / 16 * 16 + 8;
+                p.sums_ld = p.tokens > 1 && apart * row_sums <= most - fixed - pass * unit ? apart : rows;
+            }
         }
-        return best != 0;
-    };
-    while (!split()) {           // so many rows that their sums do not fit: several CTAs after one another
-        if (!choose || grid >= p.total_rows) return cudaErrorInvalidValue;
-        grid = std::min(2 * grid, p.total_rows);
     }
-    p.pass_units = static_cast<uint32_t>(std::min<size_t>(units, (most - fixed) / unit));
-    if (p.pass_units < units) p.pass_units -= p.pass_units % p.k_split;
+    if (!best) return cudaErrorInvalidValue;
     // more than half of an SM's shared memory in any case: one CTA per SM (gemv_bf16.cuh)
-    const size_t smem = std::max(fixed + p.pass_units * unit, most / 2 + 1024);
+    const size_t smem = std::max(fixed + p.pass_units * unit + p.sums_ld * row_sums, most / 2 + 1024);
     auto* fn = &zk::gemv_kq_mma_kernel<kFormat, kWide>;
     static size_t configured = 0;
     if (smem > configured) {
