@@ -460,9 +460,10 @@ __global__ void __launch_bounds__(kGemvThreads, (kBatch * kDigits == 1 ? ZK_GEMV
                 for (int w = 0; w < kGemvWarps; ++w) total += norm_part[t * kGemvWarps + w];
                 inv_norm = 1.0f / sqrtf(static_cast<float>(total / p.K) + p.norm_eps);
             }
-            // One token's long rows ask for three passes' values at a time: 14336 columns take four passes, and with an L2 latency
-            // each the product of 4096 rows took 13.9 us instead of 13.1 (7168 columns times 3000 rows 7.0 and 6.6).  Rows of up to
-            // 2048 columns are one pass (1024 x 1024 with the empty fetches 2.77 us, 2.64 without).
+            // One token's rows of more than a pass (4096 columns) ask for three passes' values at a time: 14336 columns take four passes, and
+            // with an L2 latency each the product of 4096 rows took 13.8 us instead of 12.8 (7168 columns times 3000 rows 6.6 and
+            // 6.5).  Rows of one pass ask for no more than it: the empty fetches cost 0.1 us (300 x 1056 2.75 and 2.66, 1024 x 4096
+            // 3.04 and 2.98).
             constexpr bool kAhead = kBatch == 1 && kPack == 1;
             const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
             constexpr uint32_t kPass = kGemvWarps * 8;
@@ -474,8 +475,9 @@ __global__ void __launch_bounds__(kGemvThreads, (kBatch * kDigits == 1 ? ZK_GEMV
                 hi = b < nb ? __ldcg(src + 1) : zero;
             };
             float4 lo, hi, lo1, hi1, lo2, hi2;
-            if constexpr (kAhead) {
-                fetch(warp * 8, lo, hi);
+            const bool ahead = kAhead && nb > kPass;
+            if (kAhead) fetch(warp * 8, lo, hi);
+            if (ahead) {
                 fetch(warp * 8 + kPass, lo1, hi1);
                 fetch(warp * 8 + 2 * kPass, lo2, hi2);
             }
@@ -484,7 +486,7 @@ __global__ void __launch_bounds__(kGemvThreads, (kBatch * kDigits == 1 ? ZK_GEMV
                 const bool live = b < nb;
                 if constexpr (!kAhead) fetch(b0, lo, hi);
                 float v[8] = {lo.x, lo.y, lo.z, lo.w, hi.x, hi.y, hi.z, hi.w};
-                if constexpr (kAhead) {
+                if (ahead) {
                     lo = lo1; hi = hi1;
                     lo1 = lo2; hi1 = hi2;
                     fetch(b0 + 3 * kPass, lo2, hi2);
