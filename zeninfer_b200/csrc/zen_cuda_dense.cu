@@ -7,6 +7,7 @@
 #include <algorithm>
 #include <string>
 #include <type_traits>
+#include <unordered_map>
 
 #include "attention.cuh"
 #include "attention_tc.cuh"
@@ -27,8 +28,13 @@ using zk_host::Entry;
 template <typename... KArgs, typename... Args>
 cudaError_t launch(const Entry& e, void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, Args... args) {
     if (smem > 48 * 1024) {
-        const cudaError_t r = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
-        if (r != cudaSuccess) return r;
+        static std::unordered_map<const void*, size_t> allowed;      // what the kernels of this signature may use so far; under the Entry's lock
+        size_t& most = allowed[reinterpret_cast<const void*>(kernel)];
+        if (smem > most) {
+            const cudaError_t r = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
+            if (r != cudaSuccess) return r;
+            most = smem;
+        }
     }
     cudaLaunchConfig_t cfg{};
     cfg.gridDim = grid;
