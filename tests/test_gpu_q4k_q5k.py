@@ -261,6 +261,26 @@ def test_more_rows_than_their_sums_fit(be):
     _close_to_f64(_products(be, "Q4_0", w, x, rows, 32), blocks.Q4_0, w, x, some, 32, True)
 
 
+# Two blocks of one unit far apart: an activation is held to 2^-35 of the largest of its 256 columns (2^-39 in low nibbles), seen where
+# the large ones meet weights that are zero.
+@pytest.mark.parametrize("tokens", [1, 3, 8])
+@pytest.mark.parametrize("log2", [8, 16, 30])
+def test_small_activations_beside_large_ones(be, tokens, log2):
+    rows, cols = 100, 1024
+    w, x = _weights(blocks.Q4_0, rows, cols, 11), seeded_acts(tokens, cols, 12)
+    w.reshape(rows, cols // 32, 18)[:, ::8, :2] = 0           # the scale of every unit's first block
+    x.reshape(tokens, cols // 32, 32)[:, ::8] *= np.float32(2.0 ** log2)
+    got = _products(be, "Q4_0", w, x, rows, cols)
+    decoded = blocks.dequantize(blocks.Q4_0, w, rows, cols).astype(np.float64)
+    small = np.abs(x).astype(np.float64) * (np.arange(cols) % 256 >= 32)
+    largest = np.abs(x).reshape(tokens, -1, 256).max(axis=2).astype(np.float64)
+    step = w.reshape(rows, cols // 32, 18)[:, :, :2].copy().view(np.float16).astype(np.float64)[..., 0]
+    in_block = small.reshape(tokens, -1, 32).max(axis=2)
+    bound = small @ np.abs(decoded).T * (2.0 ** -22 + 64 * 2.0 ** -24) + largest @ np.abs(decoded).reshape(rows, -1, 256).sum(axis=2).T * 2.0 ** -35 + 32 * 2.0 ** -14 * in_block @ np.abs(step).T
+    bound += largest @ np.abs(step).reshape(rows, -1, 8).sum(axis=2).T * 256 * 2.0 ** -35      # nibbles are up to 8 steps from the weight they stand for
+    assert np.all(np.abs(got - x.astype(np.float64) @ decoded.T) <= bound)
+
+
 @pytest.mark.parametrize("name", list(ALL))
 def test_activations_of_any_size(be, name):
     """The operands are scaled by a power of two per 256 columns: vectors of very large, very small and no values, and both in one."""

@@ -84,10 +84,6 @@ __device__ __forceinline__ void dense_fma8_pairs(const uint4& w, const unsigned 
     for (int i = 0; i < 4; ++i)
         asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(acc) : "l"(dense_pair(__uint_as_float(u[i] << 16), __uint_as_float(u[i] & 0xffff0000u))), "l"(x[i]));
 }
-// 16 bytes global -> shared, or 16 zero bytes.
-__device__ __forceinline__ void dense_copy(uint32_t dst, const void* src, bool real) {
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(real ? 16u : 0u) : "memory");
-}
 
 // The prologue of rows of up to 4096 values (a multiple of 32, in 1, 2, 4 or 8 parts, every array 16-byte aligned), formed as
 // sublayer_row and sublayer_view form it: a warp holds an eighth of the row in registers and all arrays are asked for at once.
@@ -206,9 +202,9 @@ __global__ void __launch_bounds__(kDenseThreads, 2) gemv_bf16_kernel(const __gri
     pdl_launch_dependents();
 
     // A warp's steps: (task, row group, K unit), walked in that order, once to ask for the weights and once to use them; what a step
-    // needs of its task stays in registers.  Where the warps that share a row group do not divide its units evenly, the ones with
-    // a unit more are others in the next group: with the same warps every time, rows of 18432 columns (72 units on 16 warps) kept
-    // half of the warps waiting for a tenth of the launch.
+    // needs of its task stays in registers.  Where the warps that share a row group do not divide its units evenly (9, 17 or 20 units
+    // on eight warps), the ones with a unit more are others in the next group: the same warps every time would keep the rest waiting,
+    // half of them for a tenth of the launch where sixteen warps shared 72 units.
     struct Walk {
         const __nv_bfloat16* w;       // the lane's word of row r
         uint32_t ti, r, r_end, u, units, ld, x;
@@ -253,7 +249,7 @@ __global__ void __launch_bounds__(kDenseThreads, 2) gemv_bf16_kernel(const __gri
         const __nv_bfloat16* src = real ? w.w : w.w - lane * 8;
 #pragma unroll
         for (int i = 0; i < kDenseRows; ++i)
-            if (w.r + i < w.r_end) dense_copy(dst + i * 512, src + static_cast<size_t>(i) * w.ld, real);
+            if (w.r + i < w.r_end) copy16_or_zero(dst + i * 512, src + static_cast<size_t>(i) * w.ld, real);
     };
     Walk in{}, at;
     enter(in);

@@ -113,15 +113,12 @@ template <int kWide> inline uint32_t kqm_partials(uint32_t units) {
     return n;
 }
 
-// 16 or 4 bytes global -> shared, or 16 zero bytes.
+// 16 or 4 bytes global -> shared.
 __device__ __forceinline__ void kq_copy16(uint32_t dst, const void* src) {
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory");
 }
 __device__ __forceinline__ void kq_copy4(uint32_t dst, const void* src) {
     asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(dst), "l"(src) : "memory");
-}
-__device__ __forceinline__ void kq_copy16_or_zero(uint32_t dst, const void* src, bool real) {
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(real ? 16u : 0u) : "memory");
 }
 // 16 rows x 16 columns of A (f16) times 16 x 8 of B, fp32 sums.
 __device__ __forceinline__ void kq_mma(float (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
@@ -254,8 +251,8 @@ __global__ void __launch_bounds__(kqm_threads<kWide>(), 1) gemv_kq_mma_kernel(co
             const uint32_t to = dst + i * 1024 + place16;
             if (kFormat == 2 && ragged) {      // behind the row's last block: zeros, and no address to read at
                 const bool real = unit * kKqUnit + i * 128 + t * 32 < p.K;
-                kq_copy16_or_zero(to, real ? a + i * 64 : p.task[w.ti].plane[0], real);
-                kq_copy16_or_zero(to + 512, real ? b + i * 64 : p.task[w.ti].plane[0], real);
+                copy16_or_zero(to, real ? a + i * 64 : p.task[w.ti].plane[0], real);
+                copy16_or_zero(to + 512, real ? b + i * 64 : p.task[w.ti].plane[0], real);
             } else {
                 kq_copy16(to, a + i * 64);
                 kq_copy16(to + 512, b + i * 64);

@@ -166,6 +166,11 @@ __host__ __device__ constexpr uint32_t umma_idesc_bf16(uint32_t m, uint32_t n) {
     return (1u << 4) | (1u << 7) | (1u << 10) | ((n >> 3) << 17) | ((m >> 4) << 24);
 }
 
+// 16 bytes global -> shared, or 16 zero bytes.
+__device__ __forceinline__ void copy16_or_zero(uint32_t dst, const void* src, bool real) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(real ? 16u : 0u) : "memory");
+}
+
 // Programmatic dependent launch: wait for the producing grid's memory, and let
 // the dependent grid start its own prologue early.
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
