@@ -462,8 +462,8 @@ __global__ void __launch_bounds__(kGemvThreads, (kBatch * kDigits == 1 ? ZK_GEMV
             }
             // One token's rows of more than a pass (4096 columns) ask for three passes' values at a time: 14336 columns take four passes, and
             // with an L2 latency each the product of 4096 rows took 13.8 us instead of 12.8 (7168 columns times 3000 rows 6.6 and
-            // 6.5).  Rows of one pass ask for no more than it: the empty fetches cost 0.1 us (300 x 1056 2.75 and 2.66, 1024 x 4096
-            // 3.04 and 2.98).
+            // 6.5).  Rows of one pass ask for no more than it: the empty fetches cost 0.1 us (300 x 1056 2.75 and 2.67, 1024 x 4096
+            // 3.04 and 2.96).  Not so where the launch forms its input itself: requests of width 4096 took 5713 us without them, 5670 with.
             constexpr bool kAhead = kBatch == 1 && kPack == 1;
             const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
             constexpr uint32_t kPass = kGemvWarps * 8;
@@ -474,23 +474,10 @@ __global__ void __launch_bounds__(kGemvThreads, (kBatch * kDigits == 1 ? ZK_GEMV
                 lo = b < nb ? __ldcg(src) : zero;
                 hi = b < nb ? __ldcg(src + 1) : zero;
             };
-            float4 lo, hi, lo1, hi1, lo2, hi2;
-            const bool ahead = kAhead && nb > kPass;
-            if (kAhead) fetch(warp * 8, lo, hi);
-            if (ahead) {
-                fetch(warp * 8 + kPass, lo1, hi1);
-                fetch(warp * 8 + 2 * kPass, lo2, hi2);
-            }
-            for (uint32_t b0 = warp * 8; b0 < nb; b0 += kPass) {  // warp-uniform trip count: the quantiser shuffles
+            auto quantise = [&](uint32_t b0, const float4& lo, const float4& hi) {
                 const uint32_t b = b0 + quad;
                 const bool live = b < nb;
-                if constexpr (!kAhead) fetch(b0, lo, hi);
                 float v[8] = {lo.x, lo.y, lo.z, lo.w, hi.x, hi.y, hi.z, hi.w};
-                if (ahead) {
-                    lo = lo1; hi = hi1;
-                    lo1 = lo2; hi1 = hi2;
-                    fetch(b0 + 3 * kPass, lo2, hi2);
-                }
                 if (kFuse && (flags & kGemvFlagNorm)) {
                     const float4* wsrc = reinterpret_cast<const float4*>(p.norm_weight + b * 32 + part * 8);
                     const float4 wlo = live ? __ldg(wsrc) : zero, whi = live ? __ldg(wsrc + 1) : zero;
@@ -509,7 +496,7 @@ __global__ void __launch_bounds__(kGemvThreads, (kBatch * kDigits == 1 ? ZK_GEMV
                 }
                 uint2 c1, c2;
                 const float d = quantise_block_quad(v, c1, c2);
-                if (!live) continue;
+                if (!live) return;
                 const uint32_t l = b & 31, grp = b >> 5;
                 const uint32_t hh = (part >> 1) ^ ((l >> 2) & 1);
                 const size_t slot = (static_cast<size_t>(grp) * 2 + hh) * 32 + l;  // uint4 index
@@ -517,6 +504,25 @@ __global__ void __launch_bounds__(kGemvThreads, (kBatch * kDigits == 1 ? ZK_GEMV
                 *dst = c1;
                 if (kDigits == 2) dst[static_cast<size_t>(kpad_blocks) * 4] = c2;
                 if (part == 0) xscale[static_cast<size_t>(t) * kpad_blocks + b] = kDigits == 2 ? d * (1.0f / 256.0f) : d;
+            };
+            float4 lo, hi;
+            if (kAhead && (kFuse || nb > kPass)) {
+                float4 lo1, hi1, lo2, hi2;
+                fetch(warp * 8, lo, hi);
+                fetch(warp * 8 + kPass, lo1, hi1);
+                fetch(warp * 8 + 2 * kPass, lo2, hi2);
+                for (uint32_t b0 = warp * 8; b0 < nb; b0 += kPass) {  // warp-uniform trip count: the quantiser shuffles
+                    const float4 l = lo, h = hi;
+                    lo = lo1; hi = hi1;
+                    lo1 = lo2; hi1 = hi2;
+                    fetch(b0 + 3 * kPass, lo2, hi2);
+                    quantise(b0, l, h);
+                }
+            } else {
+                for (uint32_t b0 = warp * 8; b0 < nb; b0 += kPass) {
+                    fetch(b0, lo, hi);
+                    quantise(b0, lo, hi);
+                }
             }
         }
     }
