@@ -21,14 +21,14 @@
 //       Q6_K : y += d * sc_g * sum (q - 32) x           per 16 weights
 //       Q4_K / Q5_K : y += d * sc_g * sum q x  -  dmin * m_g * sum x        per 32 weights
 // What is dropped of an activation is below 2^-22 of it, or below 2^-39 (high nibbles: 2^-35) of the largest of its 256 columns: next to
-// very much larger activations small ones lose bits that a scale per 32 columns would keep, and below that they vanish.  The instruction adds its sixteen products with the bits of fp32 below the
-// exponents' largest sum, and a code of a few bits has the exponent of 1024: a product loses what lies below 2^-14 of a code times the
-// largest activation of the sixteen, where gemv_kq.cuh's digits lose up to 2^-13.  Results are 4e-7 to 1.2e-6 from 64 bits at 4096
-// columns, those of the digits 2.2e-5.  The unpacking (a shift and four ANDs for eight weights, on a pipe that
-// takes one every other clock) and the steps' own instructions bound one token, the products from five tokens on.  A layer of
-// 4096 / 14336 columns: Q4_0 45.9 -> 44.2 us, Q4_K 55.5 -> 45.9, Q5_K 69.4 -> 58.9; two tokens Q4_0 87.7 -> 54.3; with 4096 columns
-// everywhere and four tokens Q4_0 77.7 -> 39, Q6_K 62.1 -> 50, eight Q4_0 142 -> 72, Q6_K 106 -> 83.  Tried and slower: the shift on the
-// multiplier pipe, steps of two units by eight warps.
+// very much larger activations small ones lose bits that a scale per 32 columns would keep, and below that they vanish.  The
+// instruction adds its sixteen products with the bits of fp32 below the exponents' largest sum, and a code of a few bits has the exponent
+// of 1024: a product loses what lies below 2^-14 of a code times the largest activation of the sixteen, where int8 digits lose
+// up to 2^-13.  Results are 4e-7 to 1.2e-6 from 64 bits at 4096 columns, those of the digits 2.2e-5.
+//
+// The unpacking (a shift and four ANDs for eight weights, on a pipe that takes one every other clock) and the steps' own instructions
+// bound one token, the products from five tokens on, and the operands that every CTA forms first bound small launches; times and
+// those of the digits: kq_takes_mma.  Tried and slower: the shift on the multiplier pipe, steps of two units by eight warps.
 //
 // Weights stream as in gemv_bf16.cuh: one CTA per SM owns a contiguous row slice (the cut of ComputePool::parallel_for,
 // src/compute_pool.cpp:104-106), its warps split it by 16-row tiles and 256-column units, and each warp's share arrives by
@@ -153,15 +153,15 @@ template <int kFormat> __device__ __forceinline__ uint32_t kq_high(uint32_t w, u
 
 // Which products come here: decided by format and columns alone, so that a row has the same arithmetic whatever tokens, tensors and rows
 // share its launch and whatever shard it is in (gemv_kq.cuh's digits are 2e-5 away).  A B200, us here and of the digits:
-//   one token      Q4_0         Q4_K         Q5_K          Q6_K          two tokens Q4_0  Q6_K         four tokens Q4_0  Q6_K
-//   256 x 1024      2.8   2.9    2.8   3.2    2.9    3.4    3.1    3.0    3.5   3.9    3.5   3.7     4.4   6.0     4.3   5.5
-//   1024 x 1024     3.1   2.8    3.2   3.1    3.3    3.3    3.5    3.0    3.9   3.9    3.9   3.7     4.6   6.0     4.6   5.5
-//   2048 x 2048     3.7   4.1    3.7   4.7    4.1    5.9    4.4    4.6    4.5   4.9    4.8   5.2     5.8   7.5     6.0   6.8
-//   8192 x 2048     5.7  10.2    5.8  12.5    7.2   16.8    8.2   12.2    6.7  11.1    8.6  12.6     7.9  16.0     9.7  14.0
-//   1536 x 4096     4.3   3.5    4.5   3.9    5.1    4.3    5.6    3.8    5.9   6.2    6.7   5.4     7.9  10.5     8.6   8.8
-//   6144 x 4096     6.8   6.3    7.1   7.5    8.9    9.0   10.2    7.4    8.4  11.5   11.2   9.7    10.4  20.1    13.0  15.7
-//   28672 x 4096   16.3  19.0   16.6  24.7   23.2   31.4   27.3   23.3   18.5  40.3   28.2  31.9    20.5  73.0    32.4  52.6
-//   4096 x 14336   14.3  14.7   14.5  17.0   18.5   21.0   20.4   16.3   18.2  24.5   24.0  21.6    21.8  34.5 (three tokens)
+//   one token      Q4_0         Q4_K         Q5_K         Q6_K      two tokens Q4_0   Q6_K       four tokens Q4_0   Q6_K
+//   256 x 1024      2.9   2.9    2.9   3.1    3.1   3.4    3.3   3.0    3.5   3.9    3.7   3.7     4.4   6.0    4.5   5.5
+//   1024 x 1024     3.3   2.8    3.2   3.1    3.3   3.3    3.6   3.0    3.9   3.9    4.0   3.7     4.6   6.0    4.7   5.6
+//   2048 x 2048     3.8   4.1    3.8   4.7    4.1   5.9    4.5   4.6    4.5   4.9    4.9   5.2     5.7   7.4    6.1   6.7
+//   8192 x 2048     5.8  10.2    5.9  12.5    7.3  16.8    8.3  12.2    6.8  11.1    8.8  12.6     7.9  16.0    9.8  14.0
+//   1536 x 4096     4.4   3.5    4.5   3.9    5.2   4.3    5.6   3.7    5.9   6.2    6.6   5.3     7.8  10.7    8.6   8.7
+//   6144 x 4096     7.0   6.3    7.2   7.5    9.2   9.0   10.1   7.3    8.4  11.4   11.2   9.6    10.3  20.0   13.1  15.4
+//   28672 x 4096   16.5  19.1   16.6  24.6   23.6  31.4   27.2  23.1   18.7  40.3   28.2  31.9    20.6  73.0   32.3  52.4
+//   4096 x 14336   14.8  14.7   14.6  17.0   18.9  21.0   20.4  15.3   18.3  24.3   24.0  20.6
 // One token of Q6_K, whose codes are bytes here, costs up to half as much again from 4096 columns on, where the digits' rows arrive in whole
 // segments; there Q6_K stays with them for all tokens, at the price of the last column.
 inline bool kq_takes_mma(bool q6, uint32_t K) { return !q6 || K < static_cast<uint32_t>(kKqSegElems); }

@@ -1258,7 +1258,8 @@ bool enqueue_gemm_q8_0(State& s, const zen_cuda_weights* const* w, float* const*
 // Narrow tiles (32 columns = 16 tokens) up to kQ6kNarrowMaxTokens rows, the prefill GEMM's 128 columns (64 tokens) beyond.
 constexpr size_t kQ6kNarrowMaxTokens = 16;
 // From this many activation rows on the host-pointer call takes the tensor-core product: the narrow-tile kernel takes the
-// same ~270 us for the 128256 x 4096 lm_head whatever the row count, the decode kernel 43 + 41 us per row.
+// same ~270 us for the 128256 x 4096 lm_head whatever the row count, the decode kernel 92, 124, 207 and 370 us for one, two, four and
+// eight.  (The group-scale kernel, which runs where its digits are kept, takes 169 us: no threshold has been measured for it.)
 constexpr size_t kQ6kTensorMinTokens = 7;
 size_t gemm_q6k_ws_bytes(size_t tokens, size_t cols) { return std::max(gemm_ws_bytes(2 * tokens, cols, 2), gemm_groups_ws_bytes(tokens, cols)); }
 
@@ -1319,7 +1320,7 @@ bool enqueue_gemm_q6k(State& s, const zen_cuda_weights* w, float* d_out, const f
 // f16 block scales that is a Q8_0 tensor), then the Q8_0 GEMM with two activation digits, the fp32-activation arithmetic
 // the reference uses for this format (generic route, src/quant.cpp:1135-1162).  The workspace holds the codes
 // (rows x cols bytes, padded to 256) followed by the GEMM's own workspace.
-constexpr size_t kQ4TensorMinTokens = 9;    // 14336 x 4096: 37 us up to 128 rows through the group-scale kernel (96 us with nibbles widened per call), 75 us per chunk of eight through the decode kernel
+constexpr size_t kQ4TensorMinTokens = 9;    // 14336 x 4096: 27 us for 16 rows through the group-scale kernel (96 us with nibbles widened per call), 26 us per chunk of eight through the decode kernel
 size_t gemm_q4_0_ws_bytes(size_t tokens, size_t rows, size_t cols) {
     return std::max(((rows * cols + 255) & ~size_t(255)) + gemm_ws_bytes(tokens, cols, 2), gemm_groups_ws_bytes(tokens, cols));
 }
@@ -1350,7 +1351,7 @@ bool enqueue_gemm_q4_0(State& s, const zen_cuda_weights* w, float* d_out, const 
 // of every 32-weight sub-block (w = scale * q - offset), then the tensor-core GEMM with two activation digits whose
 // epilogue also subtracts offset x (activation sum of the block).  Workspace: codes | scales | offsets | GEMM workspace |
 // block-major activation sums.
-constexpr size_t kK45TensorMinTokens = 9;
+constexpr size_t kK45TensorMinTokens = 9;    // 14336 x 4096: 27 us for 16 rows through the group-scale kernel, 27 (Q4_K) and 29 us (Q5_K) per chunk of eight through the decode kernel
 size_t align256(size_t n) { return (n + 255) & ~size_t(255); }
 size_t gemm_k45_ws_bytes(size_t tokens, size_t rows, size_t cols) {
     const size_t t_ld = (tokens + 3) & ~size_t(3);
