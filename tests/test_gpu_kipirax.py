@@ -105,6 +105,23 @@ def test_dense_gemm_tile_widths(be, rows, tokens):
     test_dense_gemm(be, rows, 72, tokens, False)
 
 
+# A number that names no activation is none, in all three products, whatever cap says.
+@pytest.mark.parametrize("act", [3, 7, -1])
+def test_an_unknown_activation_is_none(be, act):
+    import torch
+    h, w = bf16_matrix(be, 130, 64, 5)
+    x = dev(np.random.default_rng(6).standard_normal((40, 64))).to(torch.bfloat16)
+    want = host(x).astype(np.float64) @ w.T
+    for rows, exact in ((x, False), (x.float(), True)):
+        out = zeros(40, 130)
+        be.dev_dense_gemm(h, rows.data_ptr(), 64, 40, out.data_ptr(), 130, exact=exact, act=act, cap=0.5)
+        close(host(out), want)
+    y, one = zeros(130), x[0].float()
+    be.dev_dense_gemv([(h, one.data_ptr(), y.data_ptr())], act=act, cap=0.5)
+    close(host(y), want[0])
+    be.dev_free(h)
+
+
 def test_products_refuse_bad_arguments(be):
     h, _ = bf16_matrix(be, 16, 24, 0)
     y = zeros(64)

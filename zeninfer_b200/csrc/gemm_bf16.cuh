@@ -70,9 +70,9 @@ __device__ __forceinline__ void gemm_bf16_store(const GemmBf16Params& p, const u
             if (p.out) gemm_bf16_column(p.out + at, p.out_ld, v, count, f);
             else gemm_bf16_column(p.out_bf16 + at, p.out_ld, v, count, [&](float y) { return __float2bfloat16_rn(f(y)); });
         };
-        if (p.act == kActNone) with([&](float y) { return y + bias; });
+        if (p.act == kActSoftcap) with([&](float y) { return dense_activation(y + bias, kActSoftcap, p.cap); });
         else if (p.act == kActSquaredRelu) with([&](float y) { return dense_activation(y + bias, kActSquaredRelu, 0.0f); });
-        else with([&](float y) { return dense_activation(y + bias, kActSoftcap, p.cap); });
+        else with([&](float y) { return y + bias; });      // and any other number, as dense_activation has it
     }
 }
 
